@@ -135,3 +135,18 @@ def test_gemm_mx_refuses_bad_arguments():
     with pytest.raises(native.NativeError):
         native.call("tf_gemm_mx", a, 128, a, 128, 256, 0, sf, 1, sfb, sfb.shape[1], c, 256, 0, 128, 256, 128, None, None,
                     st.t)                                                  # too few scale units for the rows
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,K,off", [(1, 128, 0), (127, 4096, 0), (129, 4224, 0), (640, 8320, 0), (130, 256, 1)])
+def test_scale_units_transpose(rows, K, off):
+    """Tiles of 128 rows x 4096 inputs with ragged edges, and a source off the 4-byte boundary: bytes move unchanged."""
+    from titanic_flash_41_b200.ops import mx, native
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    flat = torch.randint(0, 256, (rows * (K // 32) + off,), generator=g, device="cuda", dtype=torch.uint8)
+    s = flat[off:].view(rows, K // 32)
+    out = torch.full((K // 128, mx.sf_units(rows, 256), 128), 7, dtype=torch.uint8, device="cuda")
+    native.call("tf_mx_sf_to_units", s, out, rows, K, out.shape[1])
+    assert torch.equal(mx.units_to_rowmajor(out, rows), s)
+    pad = out.view(K // 128, -1, 4)[:, rows:]
+    assert int((pad != 7).sum()) == 0                      # rows beyond the matrix are left alone

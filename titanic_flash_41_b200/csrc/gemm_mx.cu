@@ -386,15 +386,42 @@ __global__ void __launch_bounds__(128) swiglu_rows_mx_units_kernel(const __nv_bf
   sf[((long)(b >> 2) * sf_units + (r >> 5)) * 128 + (r & 31) * 4 + (b & 3)] = (uint8_t)(ex + 127);
 }
 
-// row-major UE8M0 scales [rows, K/32] -> unit layout [K/128][units][128]
+// row-major UE8M0 scales [rows, K/32] -> unit layout [K/128][units][128].  Seen as 4-byte words (the four
+// scales of a 128-deep k block) this is the transpose of a [rows][K/128] matrix: word (kb, row) lands at
+// kb * units * 32 + row.  Bound by HBM, so a CTA moves 128 rows x 32 words through shared memory and
+// both sides are whole 128-byte lines (a 33-word pitch keeps the column reads free of bank conflicts).
+// One thread per byte scattered over 512-byte strides took 272 us for 524,288 rows of K = 4096 (134 MB
+// moved, 0.5 TB/s); a 197-row prefill of four layers (twelve of these) went from 9.44 to 6.95 ms.  `s` or `out` off a 4-byte boundary: byte by byte.
+constexpr int kTrRows = 128, kTrWords = 32;
 __global__ void __launch_bounds__(256) sf_to_units_kernel(const uint8_t* __restrict__ s, uint8_t* __restrict__ out,
-                                                          long rows, int ks, int units) {
+                                                          long rows, int kb_n, int units, int words) {
   tf_pdl_sync();
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * ks) return;
-  const long r = i / ks;
-  const int b = (int)(i % ks);
-  out[((long)(b >> 2) * units + (r >> 5)) * 128 + (r & 31) * 4 + (b & 3)] = s[i];
+  __shared__ uint32_t tile[kTrRows][kTrWords + 1];
+  const long r0 = (long)blockIdx.x * kTrRows;
+  const int k0 = blockIdx.y * kTrWords, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k = k0 + lane;
+#pragma unroll
+  for (int i = 0; i < kTrRows / 8; ++i) {
+    const long r = r0 + warp + 8 * i;
+    uint32_t v = 0;
+    if (r < rows && k < kb_n) {
+      const uint8_t* src = s + (r * kb_n + k) * 4;
+      if (words) v = *reinterpret_cast<const uint32_t*>(src);
+      else v = src[0] | (src[1] << 8) | (src[2] << 16) | ((uint32_t)src[3] << 24);
+    }
+    tile[warp + 8 * i][lane] = v;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kTrWords * kTrRows / 256; ++i) {
+    const int j = i * 256 + threadIdx.x, kk = j / kTrRows, rr = j % kTrRows;
+    if (k0 + kk >= kb_n || r0 + rr >= rows) continue;
+    uint8_t* dst = out + ((long)(k0 + kk) * units * 32 + r0 + rr) * 4;
+    const uint32_t v = tile[rr][kk];
+    if (words) *reinterpret_cast<uint32_t*>(dst) = v;
+    else
+      for (int b = 0; b < 4; ++b) dst[b] = (uint8_t)(v >> (8 * b));
+  }
 }
 
 // fp32 power-of-two scales per 128 x 128 block [rows/128, K/128] -> unit layout (every 32 x 32
@@ -520,9 +547,10 @@ TF_API int tf_swiglu_rows_mx_units(const void* y, int ldy, void* q, void* sf, in
 // row-major UE8M0 scales [rows, K / 32] -> unit layout (`out` holds K / 128 * units * 128 bytes, zeroed by the caller)
 TF_API int tf_mx_sf_to_units(const void* s, void* out, long rows, int K, int units, cudaStream_t st) {
   if (rows <= 0 || K % 128 || units * 32L < rows) return -1;
-  const long n = rows * (K / 32);
-  tf_launch(sf_to_units_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st,
-            reinterpret_cast<const uint8_t*>(s), reinterpret_cast<uint8_t*>(out), rows, K / 32, units);
+  const int words = !((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(out)) & 3);
+  tf_launch(sf_to_units_kernel, dim3((unsigned)((rows + kTrRows - 1) / kTrRows), (K / 128 + kTrWords - 1) / kTrWords),
+            dim3(256), 0, st, reinterpret_cast<const uint8_t*>(s), reinterpret_cast<uint8_t*>(out), rows, K / 128,
+            units, words);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
