@@ -30,3 +30,51 @@ def test_prepare_and_post_match_oracle(T, H, d):
     y = hb.finish(x.to(dev), a.to(dev)).float().cpu()
     want_y = oracle.hc_post(x.float(), a, post, comb)
     assert (y - want_y).abs().max() < 0.03 * want_y.abs().max() + 1e-2
+
+
+@pytest.mark.parametrize("T,H,d", [(1, 4, 5120), (37, 3, 136), (38, 4, 5120), (100, 4, 1000), (65, 2, 72), (50, 1, 64), (40, 4, 100)])
+def test_prepare_post_and_head_over_both_forms(T, H, d):
+    """One row and sixteen rows per cluster (the line is at 37 rows), ragged last clusters, widths that do not
+    divide into eight slices, and a width off the vector grain (general kernel; no head form).
+
+    fp32 sums of n = H d products in two orders differ by at most about 2 n 2^-24 of the sum of magnitudes, and
+    in practice by its square root: far below 1e-4 of a mix here; stored rows carry bf16 rounding, 2^-9 relative."""
+    from titanic_flash_41_b200.ops import native
+    from titanic_flash_41_b200.ops.mhc import HcBoundary
+    dev = "cuda"
+    g = torch.Generator().manual_seed(T * d)
+    x = torch.randn(T, H, d, generator=g).bfloat16()
+    fn = torch.randn(H * (2 + H), H * d, generator=g) * 0.05
+    base = torch.randn(H * (2 + H), generator=g) * 0.3
+    scale = torch.tensor([0.7, 1.3, 0.9])
+    nw = (1 + 0.1 * torch.randn(d, generator=g)).bfloat16()
+    hb = HcBoundary(fn.to(dev), base.to(dev), scale.to(dev), H, d, iters=20, eps=1e-6, rms_eps=1e-6)
+    v, h16 = hb.prepare(x.to(dev), nw.to(dev))
+    pre, post, comb = (t.double() for t in oracle.hc_coefficients(x.float(), fn, base, scale, 20, 1e-6, 1e-6))
+    for got, want in zip(hb.coefficients(T), (pre, post, comb)):
+        assert (got.double().cpu() - want).abs().max() < 2e-4
+
+    def bf16_close(got, want):                  # one bf16 rounding, plus the coefficients' 2e-4
+        return ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3).all()
+    want_v = (x.double() * pre[:, :, None]).sum(1)
+    assert bf16_close(v, want_v)
+    vb = v.double().cpu()
+    want_h = vb * torch.rsqrt(vb.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    assert ((h16.double().cpu() - want_h).abs() <= 2.0 ** -10 * want_h.abs() + 1e-4).all()
+    a = torch.randn(T, d, generator=g)
+    y = hb.finish(x.to(dev), a.to(dev))
+    want_y = post[:, :, None] * a.double()[:, None] + torch.einsum("thc,thd->tcd", comb, x.double())
+    assert bf16_close(y, want_y)
+    if d % 8:
+        return
+    hfn, hbase, hscale = fn[:H].contiguous().to(dev), base[:H].contiguous().to(dev), scale[:1].to(dev)
+    hv, hm = (torch.empty(T, d, dtype=torch.bfloat16, device=dev) for _ in range(2))
+    hh, hbf = torch.empty(T, d, dtype=torch.float16, device=dev), torch.empty(T, d, dtype=torch.bfloat16, device=dev)
+    native.call("tf_hc_head", x.to(dev), hfn, hbase, hscale, hv, hm, nw.to(dev), hh, hbf, T, H, d, 1e-6, 1e-6)
+    flat = x.double().reshape(T, -1)
+    mixes = (flat @ fn[:H].double().t()) * torch.rsqrt(flat.pow(2).mean(-1, keepdim=True) + 1e-6)
+    hp = torch.sigmoid(mixes * 0.7 + base[:H].double()) + 1e-6
+    assert bf16_close(hv, (x.double() * hp[:, :, None]).sum(1)) and bf16_close(hm, x.double().mean(1))
+    hvb = hv.double().cpu()
+    want = hvb * torch.rsqrt(hvb.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    assert bf16_close(hbf, want) and torch.equal(hh, hbf.half())

@@ -1318,15 +1318,11 @@ class Engine:
             # final collapse of the residual copies with the head's own pre-mix weights
             # (reference: src/model_io.rs final hc combine)
             fn, base, scale = self.draft_extra["hc_head"]
-            xh = b["x"][:T].view(T, cfg.hc_mult, d).float()
-            flat = xh.reshape(T, -1)
-            inv = torch.rsqrt(flat.pow(2).mean(-1, keepdim=True) + cfg.rms_eps)
-            pre = torch.sigmoid((flat @ fn.t()) * inv * scale[0] + base) + cfg.hc_eps
-            b["v"][:T].copy_((xh * pre[:, :, None]).sum(1))
-            native.call("tf_add_norm", b["v"], None, 0, d, self.final_norm, b["h16"] if draft else None, b["hb"], None,
-                        None, T, d, cfg.rms_eps)
+            b["hmean"] = torch.empty(T, d, dtype=torch.bfloat16, device=self.dev)     # mean of the copies
+            native.call("tf_hc_head", b["x"], fn, base, scale, b["v"], b["hmean"], self.final_norm,
+                        b["h16"] if draft else None, b["hb"], T, cfg.hc_mult, d, cfg.hc_eps, cfg.rms_eps)
             if not draft:
-                self.last_hidden = xh.mean(1).to(torch.bfloat16)
+                self.last_hidden = b["hmean"]
         else:
             if not b.pop("normed", False):
                 native.call("tf_add_norm", b["x"], b["delta"] if b.get("pending") else None, 0, d, self.final_norm,

@@ -230,7 +230,7 @@ class SpecDecoder:
             if cfg.hc_mult > 1:
                 # the next pass is conditioned on the mean of the residual copies (as the target's
                 # hidden state is: Engine._head)
-                hid.copy_(self.bd["x"].view(S, cfg.hc_mult, cfg.hidden).float().mean(1))
+                hid.copy_(self.bd["hmean"])
             else:
                 hid.copy_(self.bd["x"])
             # sample proposal j from the modified draft law
