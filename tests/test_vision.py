@@ -102,3 +102,32 @@ def test_prefill_with_image_span_embeddings():
     assert torch.equal(base, same)
     other = run_prefill(eng, 1, p, 64, embeds=(offs, own.flip(0)))
     assert not torch.equal(base, other) and torch.isfinite(other).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,heads,spread", [(1, 1, 1.0), (127, 2, 1.0), (128, 1, 1.0), (129, 3, 4.0), (300, 2, 30.0), (1521, 16, 2.0)])
+def test_dense_attention_kernel(n, heads, spread):
+    """One key, a last tile of 1 / 127 / 128 keys, several tiles, and scores that grow along the keys so that the
+    reference maximum moves (spread 30: by far more than the 2^8 it tolerates).
+
+    Probabilities are rounded to bf16 (eight significant bits: at most 2^-8 relative) before PV and the output once
+    more: |error| is at most 2^-8 (sum_k p_k |v_k| + |o|); the rest of the bound covers fp32 sums and the exponential."""
+    from titanic_flash_41_b200.ops import native
+    dev, n_pad = "cuda", -(-n // 128) * 128
+    g = torch.Generator(device=dev).manual_seed(n)
+    q, k, v = (torch.zeros(heads, n_pad, 64, dtype=torch.bfloat16, device=dev) for _ in range(3))
+    ramp = torch.linspace(0.2, spread, n, device=dev)[None, :, None]
+    q[:, :n] = torch.randn(heads, n, 64, generator=g, device=dev).bfloat16()
+    k[:, :n] = (torch.randn(heads, n, 64, generator=g, device=dev) * ramp).bfloat16()
+    v[:, :n] = torch.randn(heads, n, 64, generator=g, device=dev).bfloat16()
+    out = torch.full((n + 1, heads * 64), 5.0, dtype=torch.bfloat16, device=dev)
+    status = native.StatusWord(torch.device(dev))
+    native.call("tf_vis_attention", q, k, v, out, n, n_pad, heads, heads * 64, 0.125, status.t)
+    status.check()
+    s = torch.einsum("hnd,hmd->hnm", q[:, :n].double(), k[:, :n].double()) * 0.125
+    p = torch.softmax(s, -1)
+    want = torch.einsum("hnm,hmd->nhd", p, v[:, :n].double())
+    mag = torch.einsum("hnm,hmd->nhd", p, v[:, :n].double().abs())
+    err = (out[:n].view(n, heads, 64).double() - want).abs()
+    assert (err <= 2.0 ** -8 * 1.01 * (mag + want.abs()) + 1e-5).all(), float((err / (mag + want.abs())).max())
+    assert (out[n] == 5.0).all()

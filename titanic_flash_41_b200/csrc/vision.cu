@@ -5,12 +5,10 @@
 //   tf_vis_rope_split      qkv [n, 3*width] -> per-head q, k, v with 2-D rotary embedding: of each head's
 //                          32 rotation pairs the first 16 turn with the patch row, the last 16
 //                          with the patch column, frequency 10000^(-(c mod 16)/16)
-//   tf_vis_softmax         row softmax of attention scores, scaled, over the first n columns
 //   tf_vis_swiglu          silu(gate) rounded to bf16, times up
 //   tf_vis_unfold          3x3 neighbourhoods (channel, dy, dx order; zero beyond the bottom/right edge)
 //   tf_vis_gelu            exact (erf) GELU
 //   tf_vis_span            start | feature rows each followed by a newline embedding | end
-//   tf_vis_transpose_pad   V [n, 64] of one head -> [128, n_pad] (rows 64.. zero) for the P*V GEMM
 // (reference: kernels/vision.cu:7-177, 12 kernels; encoder dataflow src/vision.rs:481 encode).
 #include "common.cuh"
 
@@ -69,36 +67,6 @@ __global__ void vis_rope_split_kernel(const B* qkv, B* q, B* k, B* v, int n, int
   v[dst] = qkv[src + 2 * width + half];
 }
 
-// scores [rows, ld] f32 -> probs [rows, ld] bf16 over the first n columns (the rest zero)
-__global__ void __launch_bounds__(256) vis_softmax_kernel(const float* s, B* p, int n, int ld, float scale) {
-  tf_pdl_sync();
-  __shared__ float red[8];
-  const long row = blockIdx.x;
-  const float* sr = s + row * ld;
-  float mx = -1e30f;
-  for (int c = threadIdx.x; c < n; c += 256) mx = fmaxf(mx, sr[c] * scale);
-#pragma unroll
-  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  mx = red[0];
-#pragma unroll
-  for (int q = 1; q < 8; ++q) mx = fmaxf(mx, red[q]);
-  __syncthreads();
-  float sum = 0.f;
-  for (int c = threadIdx.x; c < n; c += 256) sum += expf(sr[c] * scale - mx);
-#pragma unroll
-  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
-  __syncthreads();
-  float tot = 0.f;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) tot += red[q];
-  const float inv = 1.f / tot;
-  for (int c = threadIdx.x; c < ld; c += 256)
-    p[row * ld + c] = __float2bfloat16_rn(c < n ? expf(sr[c] * scale - mx) * inv : 0.f);
-}
-
 __global__ void vis_swiglu_kernel(const B* gu, B* y, long count, int inter) {
   tf_pdl_sync();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -142,15 +110,6 @@ __global__ void vis_span_kernel(const B* f, const B* start, const B* newline, co
   }
 }
 
-// v [n_pad, 64] -> vt [128, n_pad]: vt[c][r] = v[r][c] for c < 64 and r < n, zero elsewhere
-__global__ void vis_transpose_pad_kernel(const B* v, B* vt, int n, int n_pad) {
-  tf_pdl_sync();
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 128L * n_pad) return;
-  const int c = (int)(i / n_pad), r = (int)(i % n_pad);
-  vt[i] = (c < 64 && r < n) ? v[(long)r * 64 + c] : __float2bfloat16_rn(0.f);
-}
-
 inline unsigned blocks(long n) { return (unsigned)((n + 255) / 256); }
 }  // namespace
 
@@ -167,10 +126,6 @@ TF_API int tf_vis_rope_split(const void* qkv, void* q, void* k, void* v, int n, 
                              cudaStream_t st) {
   tf_launch(vis_rope_split_kernel, dim3(blocks((long)n * heads * 64)), dim3(256), 0, st, (const B*)qkv, (B*)q, (B*)k, (B*)v, n, n_pad,
                                                                       grid_w, heads);
-  return (int)cudaGetLastError();
-}
-TF_API int tf_vis_softmax(const float* s, void* p, int rows, int n, int ld, float scale, cudaStream_t st) {
-  tf_launch(vis_softmax_kernel, dim3(rows), dim3(256), 0, st, s, (B*)p, n, ld, scale);
   return (int)cudaGetLastError();
 }
 TF_API int tf_vis_swiglu(const void* gu, void* y, long rows, int inter, cudaStream_t st) {
@@ -190,9 +145,5 @@ TF_API int tf_vis_span(const void* f, const void* start, const void* newline, co
                        int tokens, int d, cudaStream_t st) {
   tf_launch(vis_span_kernel, dim3(blocks((long)tokens * d)), dim3(256), 0, st, (const B*)f, (const B*)start, (const B*)newline,
                                                             (const B*)end, (B*)out, width, tokens, d);
-  return (int)cudaGetLastError();
-}
-TF_API int tf_vis_transpose_pad(const void* v, void* vt, int n, int n_pad, cudaStream_t st) {
-  tf_launch(vis_transpose_pad_kernel, dim3(blocks(128L * n_pad)), dim3(256), 0, st, (const B*)v, (B*)vt, n, n_pad);
   return (int)cudaGetLastError();
 }

@@ -1,8 +1,8 @@
 """Vision tower: ViT over 14x14 patches -> 3x3 unfold -> two-layer aligner -> image token span.
 
 ``VisionOracle`` is the fp32 PyTorch definition; ``VisionTower`` runs the same network on the
-device with the tcgen05 bf16 GEMM for every projection and for both attention products
-(QK^T and PV per head) and the glue kernels of ``csrc/vision.cu`` in between
+device with the tcgen05 bf16 GEMM for every projection, the fused tcgen05 attention of
+``csrc/vision_attn.cu`` and the glue kernels of ``csrc/vision.cu`` in between
 (reference: src/vision.rs:139 Vision, :481 encode, :386 encode_split; kernels/vision.cu).
 """
 from __future__ import annotations
@@ -138,10 +138,6 @@ class VisionTower:
         x = self._linear(pp, "patch")
         h = torch.empty(n, width, **bf)
         q, k, v = (torch.zeros(heads, n_pad, HEAD, **bf) for _ in range(3))
-        vt = torch.empty(128, n_pad, **bf)
-        scores = torch.empty(n, n_pad, dtype=torch.float32, device=dev)
-        probs = torch.empty(n, n_pad, **bf)
-        o128 = torch.empty(n, 128, **bf)
         att = torch.empty(n, width, **bf)
         delta = None
         for l in range(vc.layers):
@@ -149,12 +145,7 @@ class VisionTower:
             nat.call("tf_vis_norm", x, delta, self.W[p + "norm1.weight"], h, n, width, self.eps)
             qkv = self._linear(h, p + "qkv")
             nat.call("tf_vis_rope_split", qkv, q, k, v, n, n_pad, gw, heads)
-            for hd in range(heads):
-                self._gemm(q[hd, :n], k[hd], scores)
-                nat.call("tf_vis_softmax", scores, probs, n, n, n_pad, 1.0 / math.sqrt(HEAD))
-                nat.call("tf_vis_transpose_pad", v[hd], vt, n, n_pad)
-                self._gemm(probs, vt, o128)
-                att[:, hd * HEAD:(hd + 1) * HEAD].copy_(o128[:, :HEAD])
+            nat.call("tf_vis_attention", q, k, v, att, n, n_pad, heads, width, 1.0 / math.sqrt(HEAD), self.status.t)
             d1 = self._linear(att, p + "proj")
             nat.call("tf_vis_norm", x, d1, self.W[p + "norm2.weight"], h, n, width, self.eps)
             gu = self._linear(h, p + "gate_up", bias=False)
