@@ -118,13 +118,10 @@ class VisionTower:
                     2 if out.dtype == torch.bfloat16 else 0, None, None, 0, self.status.t)
         return out
 
-    def _linear(self, a, name, bias=True):
+    def _linear(self, a, name):
         w = self.W[name + ".weight"]
         out = torch.empty(a.shape[0], w.shape[0], dtype=torch.bfloat16, device=self.dev)
-        self._gemm(a, w, out)
-        if bias:
-            self.n.call("tf_vis_bias", out, self.W[name + ".bias"], out, out.numel(), w.shape[0])
-        return out
+        return self._gemm(a, w, out)
 
     def encode(self, patches: torch.Tensor, gh: int, gw: int) -> torch.Tensor:
         """patches [gh*gw, 588] bf16 -> span [tokens, d_model] bf16."""
@@ -135,33 +132,35 @@ class VisionTower:
         bf = dict(dtype=torch.bfloat16, device=dev)
         pp = torch.zeros(n, self.pk_pad, **bf)
         pp[:, :self.pk] = patches.to(dev, torch.bfloat16)
+        W = self.W
         x = self._linear(pp, "patch")
+        nat.call("tf_vis_bias", x, W["patch.bias"], x, x.numel(), width)
         h = torch.empty(n, width, **bf)
-        q, k, v = (torch.zeros(heads, n_pad, HEAD, **bf) for _ in range(3))
+        q, k, v = (torch.empty(heads, n_pad, HEAD, **bf) for _ in range(3))
         att = torch.empty(n, width, **bf)
         delta = None
         for l in range(vc.layers):
             p = f"blocks.{l}."
-            nat.call("tf_vis_norm", x, delta, self.W[p + "norm1.weight"], h, n, width, self.eps)
+            nat.call("tf_vis_norm", x, delta, None, W[p + "norm1.weight"], h, n, width, self.eps)
             qkv = self._linear(h, p + "qkv")
-            nat.call("tf_vis_rope_split", qkv, q, k, v, n, n_pad, gw, heads)
+            nat.call("tf_vis_rope_split", qkv, W[p + "qkv.bias"], q, k, v, n, n_pad, gw, heads)
             nat.call("tf_vis_attention", q, k, v, att, n, n_pad, heads, width, 1.0 / math.sqrt(HEAD), self.status.t)
             d1 = self._linear(att, p + "proj")
-            nat.call("tf_vis_norm", x, d1, self.W[p + "norm2.weight"], h, n, width, self.eps)
-            gu = self._linear(h, p + "gate_up", bias=False)
+            nat.call("tf_vis_norm", x, d1, W[p + "proj.bias"], W[p + "norm2.weight"], h, n, width, self.eps)
+            gu = self._linear(h, p + "gate_up")
             act = torch.empty(n, vc.intermediate, **bf)
             nat.call("tf_vis_swiglu", gu, act, n, vc.intermediate)
-            delta = self._linear(act, p + "down", bias=False)
-        nat.call("tf_vis_norm", x, delta, self.W["norm.weight"], h, n, width, self.eps)
+            delta = self._linear(act, p + "down")
+        nat.call("tf_vis_norm", x, delta, None, W["norm.weight"], h, n, width, self.eps)
         ds = vc.downsample
         oh, ow = -(-gh // ds), -(-gw // ds)
         u = torch.empty(oh * ow, width * ds * ds, **bf)
         nat.call("tf_vis_unfold", h, u, gh, gw, width)
         f1 = self._linear(u, "align1")
-        nat.call("tf_vis_gelu", f1, f1, f1.numel())
+        nat.call("tf_vis_gelu", f1, W["align1.bias"], f1, f1.numel(), self.d)
         f2 = self._linear(f1, "align2")
         tokens = oh * (ow + 1) + 2
         span = torch.empty(tokens, self.d, **bf)
-        nat.call("tf_vis_span", f2, self.W["start"], self.W["newline"], self.W["end"], span, ow, tokens, self.d)
+        nat.call("tf_vis_span", f2, W["align2.bias"], W["start"], W["newline"], W["end"], span, ow, tokens, self.d)
         self.status.check()
         return span
