@@ -376,6 +376,53 @@ def test_block_verification_preserves_target_law():
     assert 0.2 < float((nacc > 0).double().mean()) < 1.0
 
 
+@pytest.mark.parametrize("Hl,drift", [(64, 0.0), (33, 0.0), (1, 0.0), (64, 12.0)])
+def test_wide_sparse_attention_of_prefill_rows_on_tcgen05(Hl, drift):
+    """Head dim 512, 64 rows or more of one split: 64-key chunks, the second contraction transposed.  Rows of one
+    key, of exactly 64 and 65, of several chunks; ``drift`` makes later keys' scores grow, so that the reference
+    maximum moves in some heads and their columns are rescaled.
+
+    P and V are f16 (at most 2^-11 relative each, V exact), the output f16: within 1e-3 of the fp32 reference."""
+    torch.manual_seed(18 + Hl)
+    T, Dh, window, ring, C, k = 200, 512, 128, 512, 400, 320
+    win_row, comp_row = Dh + Dh // 32, Dh // 2 + Dh // 16
+    u = torch.randn(Dh) / Dh ** 0.5
+    ramp = drift * torch.arange(C)[:, None] / C
+    win = codecs.kv_v41_encode(torch.randn(2, ring, Dh) * 1.5)
+    comp = codecs.kv_v41fp4_encode(torch.randn(2, C, Dh) + ramp * u * 8)
+    kvd, ckd = codecs.kv_v41_decode(win, Dh), codecs.kv_v41fp4_decode(comp, Dh)
+    pos = torch.cat([torch.arange(0, 100), torch.arange(300, 400)]).int()
+    region = torch.cat([torch.zeros(100), torch.ones(100)]).int()
+    sel = torch.full((T, k), -1, dtype=torch.int32)
+    cnt = torch.zeros(T, dtype=torch.int32)
+    for r in range(T):
+        n = [0, 1, 37, 64, 129, 255, 320][r % 7]
+        sel[r, :n] = torch.sort(torch.randperm(C)[:n]).values.int()
+        cnt[r] = n
+    q = (torch.randn(T, Hl, Dh) * 0.5 + (drift > 0) * 40 * u * (torch.arange(Hl) % 2)[None, :, None]).bfloat16()
+    sink = torch.randn(Hl) * 0.5
+    freqs = torch.tensor([10000.0 ** (-2.0 * j / 64) for j in range(32)])
+    dev = lambda t: t.to(DEV).contiguous()
+    st = native.StatusWord(DEV)
+    from titanic_flash_41_b200.models.oracle import apply_rope
+    for counts in (None, dev(cnt)):
+        part_o, part_lse = torch.zeros(1, device=DEV), torch.zeros(1, device=DEV)      # (not read or written by this form)
+        out = torch.zeros(T, Hl * Dh, device=DEV, dtype=torch.float16)
+        outb = torch.zeros(T, Hl * Dh, device=DEV, dtype=torch.bfloat16)
+        native.call("tf_sparse_attention", dev(q), T, Hl, Dh, dev(pos), dev(region), None, dev(win), ring * win_row,
+                    win_row, ring, window, dev(comp), C * comp_row, comp_row, dev(sel), k, counts, C,
+                    1 / math.sqrt(Dh), 1, part_o, part_lse, dev(sink), dev(freqs), 64, out, outb, Hl * Dh, st.t)
+        st.check()
+        got, gotb = out.cpu().view(T, Hl, Dh).double(), outb.cpu().view(T, Hl, Dh).double()
+        for r in range(T):
+            p, rg = int(pos[r]), int(region[r])
+            nw = min(p + 1, window)
+            Kmat = torch.cat([kvd[rg, [(p - nw + 1 + i) % ring for i in range(nw)]], ckd[rg, sel[r, :int(cnt[r])].long()]]).double()
+            lg = torch.cat([q[r].double() @ Kmat.t() / math.sqrt(Dh), sink[:, None].double()], 1)
+            o = apply_rope((torch.softmax(lg, -1)[:, :-1] @ Kmat)[None].float(), torch.tensor([p]), freqs, inverse=True)[0]
+            assert _rel(got[r], o) < 1e-3 and _rel(gotb[r], o) < 4e-3, (r, _rel(got[r], o))
+
+
 @pytest.mark.parametrize("world", [2, 4, 8])
 def test_key_sharded_selection_equals_unsharded(world):
     """Scoring split over `world` key shards (run one after the other here) + gather + merge gives

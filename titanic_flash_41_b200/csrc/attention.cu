@@ -57,6 +57,7 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
 }
 
 #include "attention_tc.cuh"     // sparse_attn_tc_kernel: prefill rows on tcgen05 (inside this namespace)
+#include "attention_tcw.cuh"    // sparse_attn_tcw_kernel: the same for 512-wide heads
 
 int g_attn_tc = 1;               // tf_sparse_attention_set_tc
 int g_attn_sms = 0;
@@ -586,7 +587,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
 
 }  // namespace
 
-// 1 (default): prefill rows (one split, head dim 128, 64 rows or more) run on the tcgen05 kernel;
+// 1 (default): prefill rows (one split, head dim 128 or 512, 64 rows or more) run on the tcgen05 kernels;
 // 0: always the mma.sync kernels.  Returns the previous setting.
 TF_API int tf_sparse_attention_set_tc(int on) {
   const int old = g_attn_tc;
@@ -614,17 +615,21 @@ TF_API int tf_sparse_attention(const void* q, int T, int Hl, int Dh, const int* 
   const int warps = 4;
   dim3 grid(T, nsplit);
   p.sink = sink; p.freqs = freqs; p.rope_dim = rope_dim; p.out16 = (__half*)out16; p.outb = (__nv_bfloat16*)outb; p.ldo = ldo;
-  if (g_attn_tc && Dh == 128 && nsplit == 1 && T >= 64 && Hl <= 64 && !(reinterpret_cast<uintptr_t>(q) & 15) &&
-      rope_dim <= 64 && rope_dim % 2 == 0 && ldo % 8 == 0 && !(reinterpret_cast<uintptr_t>(out16) & 15) &&
-      !(reinterpret_cast<uintptr_t>(outb) & 15)) {
+  auto aligned16 = [](const void* a) { return !(reinterpret_cast<uintptr_t>(a) & 15); };
+  if (g_attn_tc && (Dh == 128 || Dh == 512) && nsplit == 1 && T >= 64 && Hl <= 64 && aligned16(q) && aligned16(win) &&
+      win_region_stride % 16 == 0 && aligned16(comp) && comp_region_stride % 16 == 0 && rope_dim <= 64 &&
+      rope_dim % 2 == 0 && ldo % 8 == 0 && aligned16(out16) && aligned16(outb)) {
     // prefill rows: persistent CTAs on the tcgen05 tensor cores, one query row at a time
     if (!g_attn_sms) {
       int dev = 0;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&g_attn_sms, cudaDevAttrMultiProcessorCount, dev);
       cudaFuncSetAttribute(sparse_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+      cudaFuncSetAttribute(sparse_attn_tcw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTwSmem);
     }
-    tf_launch(sparse_attn_tc_kernel, dim3(T < g_attn_sms ? T : g_attn_sms), dim3(kTcThreads), kTcSmem, st, p);
+    const dim3 g(T < g_attn_sms ? T : g_attn_sms);
+    if (Dh == 128) tf_launch(sparse_attn_tc_kernel, g, dim3(kTcThreads), kTcSmem, st, p);
+    else tf_launch(sparse_attn_tcw_kernel, g, dim3(kTcThreads), kTwSmem, st, p);
     return (int)cudaGetLastError();      // (sink, inverse rotation and the output rows are part of that kernel)
   } else if (Dh == 512 || Dh == 256) {
     const int smem = (kChunk * (Dh + 8) + Dh * (kChunk + 8)) * 2 + 4 * 16 * (kChunk + 4) * 4;
