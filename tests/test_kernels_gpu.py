@@ -62,6 +62,36 @@ def test_smallm_fp8_dual_swiglu_and_kslice():
     assert _rel(out, g * torch.sigmoid(g) * u) < 3e-3
 
 
+@pytest.mark.parametrize("M,N,K,kind", [(1, 128, 128, "fp8"), (8, 384, 1152, "fp8"), (17, 384, 1280, "fp8"), (24, 12800, 384, "fp8"),
+                                        (32, 256, 2176, "fp8"), (9, 12800, 256, "dual"), (25, 256, 1152, "dual"), (3, 128, 128, "dual"),
+                                        (4, 12800, 128, "bf16"), (24, 256, 640, "bf16"), (32, 128, 1152, "bf16")])
+def test_smallm_dense_stream(M, N, K, kind):
+    """One to four 8-row tiles with ragged last ones; fewer K blocks than warps, one or two blocks more than a
+    multiple of eight, and more feature tiles than resident CTAs (the copies then run across tiles).
+
+    Against fp64 of the same stored values: products are exact in fp32, sums of K terms in fp32."""
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device=DEV).to(torch.bfloat16 if kind == "bf16" else torch.float16)
+    out = torch.full((M + 1, N), 9.0, device=DEV)
+    if kind == "bf16":
+        w = (torch.randn(N, K, device=DEV) * 0.05).bfloat16()
+        native.call("tf_smallm_gemm", 2, w, None, None, None, 0, 0, K * 2, 0, x, K, out, N, 0, N, K, M,
+                    None, None, None, None, None, 1, 0, M, 0.0)
+        want = x.double() @ w.double().t()
+    else:
+        ws = [E.quant_fp8_device(torch.randn(N, K, device=DEV) * 0.05 * (1 + torch.arange(N, device=DEV)[:, None] // 128))
+              for _ in range(2 if kind == "dual" else 1)]
+        w3 = ws[1] if kind == "dual" else None
+        native.call("tf_smallm_gemm", 0, ws[0].q, w3.q if w3 else None, ws[0].s, w3.s if w3 else None, 0, 0, K, K // 128,
+                    x, K, out, N, 0, N, K, M, None, None, None, None, None, 1, 0, M, 4.0)
+        want = x.double() @ E.dequant_fp8(ws[0]).double().t()
+        if w3 is not None:
+            want = want.clamp(max=4.0)
+            want = want * torch.sigmoid(want) * (x.double() @ E.dequant_fp8(w3).double().t()).clamp(-4.0, 4.0)
+    assert float((out[:M].double() - want).norm() / want.norm()) < 2e-6 * K ** 0.5
+    assert (out[M] == 9.0).all()
+
+
 def test_smallm_bf16_head():
     torch.manual_seed(1)
     N, K, M = 2048, 512, 9

@@ -404,6 +404,8 @@ cudaError_t launch(const SmallMParams& p, int slots, cudaStream_t st, int warps 
   return cudaGetLastError();
 }
 
+#include "smallm_dense.cuh"      // dense FP8 / bf16 matrices (inside this namespace)
+
 }  // namespace
 
 // kind: 0 = FP8 block-128, 1 = MXFP4, 2 = bf16 weights (X is then bf16, not f16).
@@ -417,6 +419,15 @@ TF_API int tf_smallm_gemm(int kind, const void* W, const void* W3, const void* S
                           int max_rows, float swiglu_limit, cudaStream_t stream) {
   (void)max_rows;
   if (N % kTileN != 0 || K % 128 != 0 || (ldx % 8) != 0 || (ldw % 16) != 0) return -1;
+  const bool dual = W3 != nullptr;
+  if (!group_expert && (kind == 0 || (kind == 2 && !dual)) && M >= 1 && M <= 32) {
+    DenseParams q;
+    q.W = (const uint8_t*)W; q.W3 = (const uint8_t*)W3; q.S = (const float*)S; q.S3 = (const float*)S3;
+    q.ldw = ldw; q.lds = lds; q.X = (const __half*)X; q.ldx = ldx; q.Y = Y; q.ldy = ldy; q.out_kind = out_kind;
+    q.N = N; q.K = K; q.M = M; q.tiles = 0; q.swiglu_limit = swiglu_limit;
+    if (kind == 2) return (int)launch_dense<2, false>(q, stream);
+    return (int)(dual ? launch_dense<0, true>(q, stream) : launch_dense<0, false>(q, stream));
+  }
   SmallMParams p;
   p.W = (const uint8_t*)W; p.W3 = (const uint8_t*)W3; p.S = S; p.S3 = S3;
   p.w_group_stride = w_group_stride; p.s_group_stride = s_group_stride;
@@ -427,7 +438,6 @@ TF_API int tf_smallm_gemm(int kind, const void* W, const void* W3, const void* S
   p.swiglu_limit = swiglu_limit;
   p.k_per_warp = ((K + kWarps - 1) / kWarps + 127) / 128 * 128;
   p.use_comm = 0;
-  const bool dual = W3 != nullptr;
   cudaError_t e;
   // dense FP8 with so few tiles that an SM gets two CTAs or fewer: eight K-splitting warps per CTA
   int warps = kWarps;
