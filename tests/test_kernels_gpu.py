@@ -784,3 +784,34 @@ def test_two_level_candidates_match_dense_selection():
         if a != b:
             cut = min(float(scores[r, i]) for i in b)
             assert all(abs(float(scores[r, i]) - cut) <= 1e-3 * abs(cut) + 1e-5 for i in a ^ b), r
+
+
+@pytest.mark.parametrize("T,d,kind", [(1, 128, None), (3, 4096, "f32"), (5, 5120, "bf16"), (2, 8192, "f32"), (2, 8320, "f32"), (70, 384, "bf16")])
+def test_add_norm_vector_form(T, d, kind):
+    """One and two 16-byte pieces a thread (the second ragged at 5120), a width beyond the vector form, and both kinds of delta.
+
+    The residual is one bf16 rounding of an fp32 sum (exact match); the normalised row one bf16 rounding (2^-8) of
+    values whose fp32 mean square has an error far below that."""
+    torch.manual_seed(d + T)
+    x = torch.randn(T, d, device=DEV).bfloat16()
+    delta = None if kind is None else torch.randn(T, d, device=DEV).to(torch.float32 if kind == "f32" else torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(d, device=DEV)).bfloat16()
+    h16, hb = torch.zeros(T, d, device=DEV, dtype=torch.float16), torch.zeros(T, d, device=DEV, dtype=torch.bfloat16)
+    res = x.clone() if delta is None else (x.float() + delta.float()).bfloat16()
+    native.call("tf_add_norm", x, delta, 1 if kind == "bf16" else 0, d, w, h16, hb, None, None, T, d, 1e-6)
+    assert torch.equal(x, res)
+    want = res.double() * torch.rsqrt(res.double().pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert ((hb.double() - want).abs() <= 2.0 ** -8 * 1.01 * want.abs() + 1e-30).all() and torch.equal(h16, hb.half())
+
+
+@pytest.mark.parametrize("T", [1, 4, 5, 8, 9, 17, 32])
+@pytest.mark.parametrize("E_,d", [(256, 4096), (33, 8), (384, 5120)])
+def test_router_logits_row_forms(T, E_, d):
+    """The three row forms and several passes, an odd number of experts, fewer 16-byte steps than warps: fp32 sums
+    of exact products, against fp64."""
+    torch.manual_seed(T + E_)
+    x, gate = torch.randn(T, d, device=DEV).bfloat16(), torch.randn(E_, d, device=DEV).bfloat16()
+    out = torch.full((T, E_ + 1), 3.0, device=DEV)
+    native.call("tf_router_logits_small", x, d, gate, out, E_ + 1, T, E_, d)
+    want = x.double() @ gate.double().t()
+    assert float((out[:, :E_].double() - want).abs().max()) < 1e-5 * d ** 0.5 + 1e-6 and (out[:, E_] == 3.0).all()
