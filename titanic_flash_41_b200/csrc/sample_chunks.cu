@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
   float* tbuf = reinterpret_cast<float*>(smem);
   float* dbuf = tbuf + p.chunk;
   unsigned long long* whist = reinterpret_cast<unsigned long long*>(dbuf + p.chunk);   // [32][256]
-  __shared__ unsigned long long gbins[256], gpart[4][256];
+  __shared__ unsigned long long gpart[4][256], wtot[8];
   __shared__ double wm[32], cm[(kMaxG + 1) * kMaxP], Rrow[kMaxG + 1], wrow[kMaxG + 1], ptq[2 * kMaxG];
   __shared__ float redf[32];
   __shared__ int redi[32];
@@ -210,14 +210,10 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
     redi[warp] = bad;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float mm = -INFINITY;
-    int b2 = 0;
-    for (int w = 0; w < 32; ++w) {
-      b2 |= redi[w];
-      if (!redi[w]) mm = fmaxf(mm, redf[w]);
-    }
-    push2(p, A.maxw + (((long)par * P + part) * p.max_rows + row) * 2, mm > -INFINITY ? fkey(mm) : 0u, (uint32_t)b2, tag0);
+  if (warp == 0) {
+    const int b2 = __any_sync(0xffffffffu, redi[lane]);
+    const float mm = warp_max(redi[lane] ? -INFINITY : redf[lane]);
+    if (lane == 0) push2(p, A.maxw + (((long)par * P + part) * p.max_rows + row) * 2, mm > -INFINITY ? fkey(mm) : 0u, (uint32_t)b2, tag0);
   }
   if (threadIdx.x < P) {
     const ulonglong2 v = W.wait(mine + A.maxw + (((long)par * P + threadIdx.x) * p.max_rows + row) * 2, tag0, 0, row);
@@ -248,6 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
     for (int k = threadIdx.x; k < 32 * 256; k += kThreads) whist[k] = 0;
     __syncthreads();
     const uint32_t prefix = s_prefix, mask = s_mask;
+    const unsigned long long above = s_above, target_prev = s_target;
     {
       // a thread's consecutive elements mostly fall into the same few bins (the top key bits are the
       // sign and the exponent): add up a run privately and touch shared memory once per run
@@ -295,28 +292,45 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
     }
     __syncthreads();
     if (s_fail) return;
-    if (threadIdx.x < 256)
-      gbins[threadIdx.x] = gpart[0][threadIdx.x] + gpart[1][threadIdx.x] + gpart[2][threadIdx.x] + gpart[3][threadIdx.x];
+    // The bin that holds the target, counted from the top: thread t owns bin 255 - t and the running mass from
+    // the top down to it is a prefix sum over the first eight warps (integers: the same bin and the
+    // same masses as a walk).  One thread walking the bins through shared memory spent 1 - 3 us a level.
+    unsigned long long mine_b = 0, incl = 0;
+    if (threadIdx.x < 256) {
+      const int b = 255 - threadIdx.x;
+      mine_b = gpart[0][b] + gpart[1][b] + gpart[2][b] + gpart[3][b];
+      incl = mine_b;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      if (lane == 31) wtot[warp] = incl;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 256) {
+      unsigned long long pre = 0, tot = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        if (w < warp) pre += wtot[w];
+        tot += wtot[w];
+      }
+      unsigned long long target = target_prev;
       if (level == 0) {
-        unsigned long long tot = 0;
-        for (int b = 0; b < 256; ++b) tot += gbins[b];
-        s_total = tot;
         const unsigned long long tg = top_p < 1.f ? (unsigned long long)((double)top_p * (double)tot) : 0ull;
-        s_target = tg ? tg : 1ull;
+        target = tg ? tg : 1ull;
+        if (threadIdx.x == 0) {
+          s_total = tot;
+          s_target = target;
+        }
       }
-      const unsigned long long target = s_target;
-      unsigned long long cum = s_above;
-      int b = 255;
-      for (; b > 0; --b) {
-        if (cum + gbins[b] >= target) break;
-        cum += gbins[b];
+      const unsigned long long upto = above + pre + incl, over = upto - mine_b;    // with / without this bin
+      if (over < target && (upto >= target || threadIdx.x == 255)) {
+        s_above = over;
+        s_inbin = mine_b;
+        s_prefix = prefix | ((uint32_t)(255 - threadIdx.x) << shift);
+        s_mask = mask | (255u << shift);
       }
-      s_above = cum;
-      s_inbin = gbins[b];
-      s_prefix |= (uint32_t)b << shift;
-      s_mask |= 255u << shift;
     }
     __syncthreads();
   }
