@@ -40,6 +40,7 @@ namespace {
 
 constexpr int BM = 128, BN = 256, BK = 128;
 constexpr int kStages = 4;
+constexpr int kGroupM = 16;                                    // M tiles of a dense matrix walked together
 constexpr int kSfaBytes = BM / 32 * 128;                       // 512
 constexpr int kSfbBytes = BN / 32 * 128;                       // 1024
 constexpr int kStageBytes = BM * 128 + BN * 128 + 2048;        // tiles, scale pieces, pad to 1 KB multiple
@@ -132,6 +133,20 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   const int mt = p.tile_expert ? *p.num_m_tiles : (p.M + BM - 1) / BM;
   const int tiles = mt * nt;
   const int stride = gridDim.x;
+  // Order of the tiles.  The CTAs running at one time should share their operands: experts take all N tiles
+  // of an M tile before the next M tile (with the M tiles first, the rows of all experts were fetched again
+  // for every N tile: 256 experts of one 128-row tile, N 2048, K 4096, moved twice the weights' bytes,
+  // 381 us; now 284), dense matrices sixteen M tiles by as many N tiles as there are CTAs.
+  auto coord = [&](int tile, int& mi, int& ni) {
+    if (p.tile_expert) {
+      mi = tile / nt;
+      ni = tile - mi * nt;
+    } else {
+      const int g = tile / (kGroupM * nt), r = tile - g * kGroupM * nt, gm = min(kGroupM, mt - g * kGroupM);
+      mi = g * kGroupM + r % gm;
+      ni = r / gm;
+    }
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -142,8 +157,10 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       int it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += stride) {
-        const int m0 = (tile % mt) * BM, n0 = (tile / mt) * BN;
-        const int nb0 = n0 + (p.tile_expert ? p.tile_expert[tile % mt] * p.N : 0);
+        int mi, ni;
+        coord(tile, mi, ni);
+        const int m0 = mi * BM, n0 = ni * BN;
+        const int nb0 = n0 + (p.tile_expert ? p.tile_expert[mi] * p.N : 0);
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % kStages;
           if (!(ok = tc::mbar_wait(empty(s), ((it / kStages) & 1) ^ 1, abort_flag))) break;
@@ -220,7 +237,9 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     int n_tile = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < tiles && ok; tile += stride, ++n_tile) {
-      const int m0 = (tile % mt) * BM, n0 = (tile / mt) * BN;
+      int mi, ni;
+      coord(tile, mi, ni);
+      const int m0 = mi * BM, n0 = ni * BN;
       const int row = m0 + quad * 32 + lane;
       const int col0 = n0 + half * 128;
       if (!(ok = tc::mbar_wait(tfull, n_tile & 1, abort_flag))) break;
