@@ -138,9 +138,11 @@ def test_gemm_mx_refuses_bad_arguments():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,K,off", [(1, 128, 0), (127, 4096, 0), (129, 4224, 0), (640, 8320, 0), (130, 256, 1)])
+@pytest.mark.parametrize("rows,K,off", [(1, 128, 0), (127, 4096, 0), (129, 4224, 0), (640, 8320, 0), (130, 256, 1), (131, 4096, 4),
+                                        (261, 8192, 0), (258, 2048, 0), (1025, 5120, 0)])
 def test_scale_units_transpose(rows, K, off):
-    """Tiles of 128 rows x 4096 inputs with ragged edges, and a source off the 4-byte boundary: bytes move unchanged."""
+    """Both forms (16-byte pieces for 32, 16 or 8 words a row piece; words) with ragged edges, and sources off the 16-byte
+    and the 4-byte boundary: bytes move unchanged."""
     from titanic_flash_41_b200.ops import mx, native
     g = torch.Generator(device="cuda").manual_seed(rows)
     flat = torch.randint(0, 256, (rows * (K // 32) + off,), generator=g, device="cuda", dtype=torch.uint8)
@@ -150,3 +152,29 @@ def test_scale_units_transpose(rows, K, off):
     assert torch.equal(mx.units_to_rowmajor(out, rows), s)
     pad = out.view(K // 128, -1, 4)[:, rows:]
     assert int((pad != 7).sum()) == 0                      # rows beyond the matrix are left alone
+
+
+@pytest.mark.parametrize("El,e_lo,pairs", [(1, 0, 5), (33, 7, 700), (512, 0, 3000), (700, 64, 20000)])
+def test_moe_plan_tables(El, e_lo, pairs):
+    """Experts below, at and beyond one pass of the offset scan, experts without rows and pairs of other ranks: padded offsets,
+    tile table, placement; and the counters are ready for the next call."""
+    g = torch.Generator().manual_seed(El)
+    ids = torch.randint(0, e_lo + El + 40, (pairs,), generator=g, dtype=torch.int32)
+    ids[ids % 5 == 1] = e_lo                                   # one expert over several tiles, others empty
+    i32 = lambda n: torch.full((n,), -5, dtype=torch.int32, device=DEV)
+    counts = torch.zeros(El, dtype=torch.int32, device=DEV)
+    cap = pairs // 128 + El + 1
+    for _ in range(2):
+        offs, cur, tile_e, nt, pad, dst = i32(El + 1), i32(El), i32(cap), i32(1), i32(1), i32(pairs)
+        native.call("tf_moe_plan", ids.to(DEV), pairs, e_lo, El, counts, offs, cur, tile_e, cap, nt, pad, dst)
+        local = ids.long() - e_lo
+        mine = (local >= 0) & (local < El)
+        cnt = torch.bincount(local[mine], minlength=El)
+        tiles = (cnt + 127) // 128
+        want = torch.cat([torch.zeros(1, dtype=torch.long), torch.cumsum(tiles * 128, 0)])
+        assert torch.equal(offs.cpu().long(), want) and int(nt) == int(tiles.sum()) and int(pad) == int(want[-1])
+        assert torch.equal(tile_e[:int(nt)].cpu().long(), torch.arange(El).repeat_interleave(tiles))
+        d = dst.cpu().long()
+        assert bool((d[~mine] == -1).all()) and d[mine].unique().numel() == int(mine.sum())
+        assert bool(((d[mine] >= want[local[mine]]) & (d[mine] < want[local[mine]] + cnt[local[mine]])).all())
+        assert int(counts.abs().sum()) == 0

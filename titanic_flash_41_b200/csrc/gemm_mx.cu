@@ -443,6 +443,50 @@ __global__ void __launch_bounds__(256) sf_to_units_kernel(const uint8_t* __restr
   }
 }
 
+// The same transpose in 16-byte pieces on both sides (rows of a multiple of W words, 16-byte aligned): a CTA
+// moves 4096 / W rows x W words.  Word (w, r) sits at w * rows + (r ^ (w / 4) * (128 / W)): the four
+// scattered stores of a piece and the 16-byte reads are free of bank conflicts.
+template <int W>
+__global__ void __launch_bounds__(256) sf_to_units_vec_kernel(const uint8_t* __restrict__ s, uint8_t* __restrict__ out,
+                                                              long rows, int kb_n, int units) {
+  tf_pdl_sync();
+  constexpr int ROWS = 4096 / W;
+  __shared__ __align__(16) uint32_t tile[4096];
+  const long r0 = (long)blockIdx.x * ROWS;
+  const int k0 = blockIdx.y * W;
+  uint4 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int p = threadIdx.x + 256 * i, r = p / (W / 4), q = p % (W / 4);
+    v[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (r0 + r < rows) v[i] = __ldg(reinterpret_cast<const uint4*>(s + ((r0 + r) * kb_n + k0) * 4) + q);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int p = threadIdx.x + 256 * i, q = p % (W / 4);
+    uint32_t* d = tile + 4 * q * ROWS + ((p / (W / 4)) ^ (q * (128 / W)));
+    d[0] = v[i].x;
+    d[ROWS] = v[i].y;
+    d[2 * ROWS] = v[i].z;
+    d[3 * ROWS] = v[i].w;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int p = threadIdx.x + 256 * i, w = p / (ROWS / 4), r = p % (ROWS / 4) * 4;
+    const uint4 o = *reinterpret_cast<const uint4*>(tile + w * ROWS + (r ^ ((w >> 2) * (128 / W))));
+    uint8_t* dst = out + ((long)(k0 + w) * units * 32 + r0 + r) * 4;
+    if (r0 + r + 3 < rows) {
+      *reinterpret_cast<uint4*>(dst) = o;
+    } else {
+      const uint32_t e[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (r0 + r + j < rows) reinterpret_cast<uint32_t*>(dst)[j] = e[j];
+    }
+  }
+}
+
 // fp32 power-of-two scales per 128 x 128 block [rows/128, K/128] -> unit layout (every 32 x 32
 // sub-block of a block carries the block's exponent).  `bad` counts scales that are not powers of two
 // in the UE8M0 range.
@@ -566,7 +610,16 @@ TF_API int tf_swiglu_rows_mx_units(const void* y, int ldy, void* q, void* sf, in
 // row-major UE8M0 scales [rows, K / 32] -> unit layout (`out` holds K / 128 * units * 128 bytes, zeroed by the caller)
 TF_API int tf_mx_sf_to_units(const void* s, void* out, long rows, int K, int units, cudaStream_t st) {
   if (rows <= 0 || K % 128 || units * 32L < rows) return -1;
-  const int words = !((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(out)) & 3);
+  const uintptr_t both = reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(out);
+  const int W = K / 128 % 32 == 0 ? 32 : K / 128 % 16 == 0 ? 16 : K / 128 % 8 == 0 ? 8 : 0;
+  if (W && !(both & 15)) {
+    auto kernel = W == 32 ? sf_to_units_vec_kernel<32> : W == 16 ? sf_to_units_vec_kernel<16> : sf_to_units_vec_kernel<8>;
+    const int tr = 4096 / W;
+    tf_launch(kernel, dim3((unsigned)((rows + tr - 1) / tr), K / 128 / W), dim3(256), 0, st,
+              reinterpret_cast<const uint8_t*>(s), reinterpret_cast<uint8_t*>(out), rows, K / 128, units);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  const int words = !(both & 3);
   tf_launch(sf_to_units_kernel, dim3((unsigned)((rows + kTrRows - 1) / kTrRows), (K / 128 + kTrWords - 1) / kTrWords),
             dim3(256), 0, st, reinterpret_cast<const uint8_t*>(s), reinterpret_cast<uint8_t*>(out), rows, K / 128,
             units, words);
