@@ -815,3 +815,51 @@ def test_router_logits_row_forms(T, E_, d):
     native.call("tf_router_logits_small", x, d, gate, out, E_ + 1, T, E_, d)
     want = x.double() @ gate.double().t()
     assert float((out[:, :E_].double() - want).abs().max()) < 1e-5 * d ** 0.5 + 1e-6 and (out[:, E_] == 3.0).all()
+
+
+@pytest.mark.parametrize("T,Hi,C,lo,hi", [(33, 8, 300, 0, 300), (70, 8, 2600, 0, 2600), (64, 16, 1000, 128, 900), (45, 32, 700, 0, 700),
+                                          (40, 64, 129, 0, 129), (320, 8, 9000, 0, 9000)])
+def test_index_scores_of_prefill_rows_on_tcgen05(T, Hi, C, lo, hi):
+    """Row tiles of 32, 16, 8 and 4 rows with a ragged last one, key tiles that end inside, at and one past 128 keys, a
+    shard of the keys, causal counts (rows without a valid key included): scores against fp64, -inf from a row's
+    count to the end of the shard, nothing written outside it.
+
+    Operands are exact in f16; a score is a sum over heads of fp32 sums of 128 products: 1e-5 of its magnitude."""
+    torch.manual_seed(T + Hi)
+    Di, lds = 128, C + 40
+    enc = codecs.index_key_encode(torch.randn(1, C, Di))
+    kd = codecs.index_key_decode(enc, Di)[0].to(DEV).double()
+    keys = enc.to(DEV).contiguous()
+    krow = enc.shape[-1]
+    q, w = torch.randn(T, Hi, Di, device=DEV).bfloat16(), torch.randn(T, Hi, device=DEV)
+    region = torch.zeros(T, dtype=torch.int32, device=DEV)
+    nvalid = torch.linspace(0, C, T, device=DEV).int()
+    scores = torch.full((T, lds), 7.0, device=DEV)
+    st = native.StatusWord(DEV)
+    native.call("tf_index_scores_rows", q, w, region, nvalid, keys, C * krow, krow, T, Hi, Di, 32, scores, lds, lo, hi, st.t)
+    st.check()
+    s = torch.einsum("thd,cd->thc", q.double(), kd).relu()
+    want, mag = (s * w.double()[:, :, None]).sum(1), (s * w.double().abs()[:, :, None]).sum(1)
+    col = torch.arange(C, device=DEV)[None, :]
+    live = (col < nvalid[:, None]) & (col >= lo) & (col < hi)
+    err = (scores[:, :C].double() - want).abs()
+    assert bool((err[live] <= 1e-5 * mag[live] + 1e-5).all()), float((err / (mag + 1))[live].max())
+    dead = (col >= nvalid[:, None]) & (col >= lo) & (col < hi)
+    assert bool((scores[:, :C][dead] == -float("inf")).all())
+    assert bool((scores[:, hi:] == 7.0).all()) and bool((scores[:, :lo] == 7.0).all())
+
+
+@pytest.mark.parametrize("T,n,lds,k", [(33, 5000, 5000, 512), (33, 4097, 4099, 2048), (40, 49152, 49152, 2048), (34, 50000, 50000, 33), (2, 3000, 4096, 1)])
+def test_topk_select_rows_edges(T, n, lds, k):
+    """Rows in shared memory up to its limit, one past it, strides off the vector grain, k of one, all three digits
+    deciding: negative, equal and nearly equal scores."""
+    torch.manual_seed(n)
+    scores = torch.randn(T, lds, device=DEV)
+    scores[0] = -scores[0].abs() - 1
+    scores[1] = 1.0 + torch.randint(0, 3, (lds,), device=DEV) * 2.0 ** -23
+    nvalid = torch.full((T,), n, dtype=torch.int32, device=DEV)
+    sel, cnt = torch.zeros(T, k, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+    native.call("tf_topk_select", scores, lds, nvalid, k, sel, cnt, None, 0, T)
+    for r in range(T):
+        order = torch.sort(scores[r, :n].cpu(), descending=True, stable=True).indices[:k].sort().values
+        assert torch.equal(sel[r].cpu().long(), order) and int(cnt[r]) == k

@@ -236,6 +236,8 @@ __global__ void __launch_bounds__(128, 3) index_score_kernel(ScoreParams p) {
   }
 }
 
+#include "indexer_tc.cuh"       // index_score_tc_kernel: prefill rows (inside this namespace)
+
 // ---------------------------------------------------------------------------------------------
 // exact top-k per row by radix select on the order-preserving integer image of the float
 // ---------------------------------------------------------------------------------------------
@@ -246,120 +248,137 @@ __device__ __forceinline__ uint32_t float_key(float f) {
 
 // scores [T, lds]; n[r] valid entries; out ids [T, k] ascending, -1 padded; count[r] = min(n, k).
 // `base` is added to every id (key-sharded scoring passes the shard offset).
-__global__ void __launch_bounds__(1024) topk_select_kernel(const float* __restrict__ scores, int lds,
-                                                           const int* __restrict__ nvalid, int k,
-                                                           int* __restrict__ out, int* __restrict__ count,
-                                                           float* __restrict__ out_scores, int base) {
+//
+// One CTA per row.  The row is read once into shared memory (STAGE; up to kSelStage scores, two CTAs an
+// SM up to half of that) and passed over five times there: histograms of 12, 10 and 10 key bits (a first digit
+// this fine spreads scores that share two or three octaves over enough bins for plain shared atomics), a
+// count per warp and the ordered compaction, in which every warp owns a contiguous stretch and finds its place
+// from ballots.  The bin of the k-th largest comes from a prefix sum over the bins.  Byte digits, a walk over
+// 256 bins by one thread, five reads from global memory and a block-wide scan with three barriers per
+// 1,024 scores took 3.45 ms for 16,384 rows of 16,384 scores on average.
+constexpr int kSelRowThreads = 1024;
+constexpr int kSelStage = 48 * 1024;                 // scores a CTA can hold
+constexpr int kSelBins = 4096;
+
+// thread t owns bins [top, top - per) counted from the largest; finds the bin where the running count from the
+// top reaches `need` and how many of that bin are still needed
+template <int BINS>
+__device__ __forceinline__ void select_bin(const int* hist, int need, int* wsum, int* s_bin, int* s_need) {
+  constexpr int PER = BINS / kSelRowThreads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int c[PER], sum = 0;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    c[j] = hist[BINS - 1 - (tid * PER + j)];
+    sum += c[j];
+  }
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) wsum[warp] = inc;
+  __syncthreads();
+  const int w = wsum[lane];
+  const int pre = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
+  int before = pre + inc - sum;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    if (before < need && before + c[j] >= need) {    // exactly one bin of the block
+      *s_bin = BINS - 1 - (tid * PER + j);
+      *s_need = need - before;
+    }
+    before += c[j];
+  }
+  __syncthreads();
+}
+
+template <bool STAGE>
+__global__ void __launch_bounds__(kSelRowThreads) topk_select_kernel(const float* __restrict__ scores, int lds,
+                                                                     const int* __restrict__ nvalid, int k,
+                                                                     int* __restrict__ out, int* __restrict__ count,
+                                                                     float* __restrict__ out_scores, int base, int vec) {
   tf_pdl_sync();
-  __shared__ int hist[256];
-  __shared__ uint32_t s_prefix;
-  __shared__ int s_need, s_run, s_tie_run;
-  __shared__ int warp_tot[32][2];
-  const int r = blockIdx.x, tid = threadIdx.x;
+  extern __shared__ __align__(16) float row_s[];
+  __shared__ int hist[kSelBins];
+  __shared__ int wsum[32], weq[32];
+  __shared__ int s_bin, s_need;
+  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = min(nvalid[r], lds);
   const float* s = scores + (long)r * lds;
   int* o = out + (long)r * k;
   if (n <= k) {
-    for (int i = tid; i < k; i += blockDim.x) {
+    for (int i = tid; i < k; i += kSelRowThreads) {
       o[i] = i < n ? base + i : -1;
       if (out_scores) out_scores[(long)r * k + i] = i < n ? s[i] : -INFINITY;
     }
     if (tid == 0 && count) count[r] = n;
     return;
   }
-  // find the k-th largest key: MSB-first radix over 4 bytes
-  if (tid == 0) {
-    s_prefix = 0;
-    s_need = k;
-  }
-  uint32_t mask = 0;
-  for (int pass = 0; pass < 4; ++pass) {
-    const int shift = 24 - 8 * pass;
-    for (int i = tid; i < 256; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    const uint32_t prefix = s_prefix;
-    if (pass == 0) {
-      // index scores crowd into a few exponent bytes: one shared atomic per warp and distinct bin
-      for (int i0 = 0; i0 < n; i0 += blockDim.x) {
-        const int i = i0 + tid;
-        const bool in = i < n;
-        const int bin = in ? (int)(float_key(s[i]) >> 24) : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, bin);
-        if (in && (tid & 31) == __ffs(peers) - 1) atomicAdd(&hist[bin], __popc(peers));
-      }
+  const float* src = STAGE ? row_s : s;
+  for (int i = tid; i < kSelBins; i += kSelRowThreads) hist[i] = 0;
+  if (STAGE) {
+    if (vec) {
+      for (int i = tid * 4; i < n; i += kSelRowThreads * 4)      // (lds is a multiple of 4: the last piece stays in the row)
+        *reinterpret_cast<float4*>(row_s + i) = *reinterpret_cast<const float4*>(s + i);
     } else {
-      for (int i = tid; i < n; i += blockDim.x) {
-        const uint32_t key = float_key(s[i]);
-        if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 0xff], 1);
-      }
+      for (int i = tid; i < n; i += kSelRowThreads) row_s[i] = s[i];
     }
-    __syncthreads();
-    if (tid == 0) {
-      int need = s_need, b = 255;
-      for (; b > 0; --b) {
-        if (hist[b] >= need) break;
-        need -= hist[b];
-      }
-      s_need = need;                     // how many to take from bin b (at deeper levels)
-      s_prefix = prefix | ((uint32_t)b << shift);
-    }
-    __syncthreads();
-    mask |= 0xffu << shift;
-  }
-  const uint32_t thr = s_prefix;         // key of the k-th largest
-  const int need_ties = s_need;          // elements equal to thr to keep (lowest positions first)
-  if (tid == 0) {
-    s_run = 0;
-    s_tie_run = 0;
   }
   __syncthreads();
-  // ordered compaction in position order
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int base_i = 0; base_i < n; base_i += blockDim.x) {
-    const int i = base_i + tid;
-    uint32_t key = i < n ? float_key(s[i]) : 0;
-    const int gt = (i < n && key > thr) ? 1 : 0;
-    const int eq = (i < n && key == thr) ? 1 : 0;
-    // inclusive scans of gt and eq within the block
-    int sg = gt, se = eq;
+  for (int i = tid; i < n; i += kSelRowThreads) atomicAdd(&hist[float_key(src[i]) >> 20], 1);
+  __syncthreads();
+  select_bin<kSelBins>(hist, k, wsum, &s_bin, &s_need);
+  uint32_t prefix = (uint32_t)s_bin << 20;
+  int need = s_need;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      int a = __shfl_up_sync(0xffffffffu, sg, d), b = __shfl_up_sync(0xffffffffu, se, d);
-      if (lane >= d) {
-        sg += a;
-        se += b;
-      }
-    }
-    if (lane == 31) {
-      warp_tot[warp][0] = sg;
-      warp_tot[warp][1] = se;
+  for (int shift = 10; shift >= 0; shift -= 10) {
+    hist[tid] = 0;
+    __syncthreads();
+    for (int i = tid; i < n; i += kSelRowThreads) {
+      const uint32_t d = float_key(src[i]) ^ prefix;             // zero above the digits still open: same prefix
+      if (d >> (shift + 10) == 0) atomicAdd(&hist[(d >> shift) & 1023], 1);
     }
     __syncthreads();
-    int og = 0, oe = 0;
-    for (int w2 = 0; w2 < warp; ++w2) {
-      og += warp_tot[w2][0];
-      oe += warp_tot[w2][1];
-    }
-    const int run = s_run, tie_run = s_tie_run;
-    const int eq_rank = tie_run + oe + se - eq;           // ties before this element
-    const int take_eq = eq && (eq_rank < need_ties);
-    // position among kept elements = kept gt before + kept eq before
-    const int gt_before = run + og + sg - gt;
-    const int eq_before = min(eq_rank, need_ties);
-    if (gt || take_eq) {
-      const int dst = gt_before + eq_before - 0;
-      // run counts only gt; ties tracked separately: final index = gt_before + eq_before
+    select_bin<1024>(hist, need, wsum, &s_bin, &s_need);
+    prefix |= (uint32_t)s_bin << shift;
+    need = s_need;
+  }
+  const uint32_t thr = prefix;           // key of the k-th largest; `need` of its equals are kept, lowest positions first
+  // ordered compaction: warp w owns positions [w * per, w * per + per)
+  const int per = ((n + 31) / 32 + 31) / 32 * 32, lo = warp * per, hi = min(n, lo + per);
+  int gt = 0, eq = 0;
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int i = i0 + lane;
+    const uint32_t key = i < hi ? float_key(src[i]) : 0u;
+    gt += __popc(__ballot_sync(0xffffffffu, i < hi && key > thr));
+    eq += __popc(__ballot_sync(0xffffffffu, i < hi && key == thr));
+  }
+  __syncthreads();                       // (wsum has been read)
+  if (lane == 0) {
+    wsum[warp] = gt;
+    weq[warp] = eq;
+  }
+  __syncthreads();
+  gt = __reduce_add_sync(0xffffffffu, lane < warp ? wsum[lane] : 0);
+  eq = __reduce_add_sync(0xffffffffu, lane < warp ? weq[lane] : 0);
+  const unsigned below = (1u << lane) - 1u;
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int i = i0 + lane;
+    const float v = i < hi ? src[i] : 0.f;
+    const uint32_t key = float_key(v);
+    const unsigned mg = __ballot_sync(0xffffffffu, i < hi && key > thr), me = __ballot_sync(0xffffffffu, i < hi && key == thr);
+    const int eq_rank = eq + __popc(me & below);
+    if ((mg >> lane & 1) || ((me >> lane & 1) && eq_rank < need)) {
+      const int dst = gt + __popc(mg & below) + min(eq_rank, need);
       if (dst < k) {
         o[dst] = base + i;
-        if (out_scores) out_scores[(long)r * k + dst] = s[i];
+        if (out_scores) out_scores[(long)r * k + dst] = v;
       }
     }
-    __syncthreads();
-    if (tid == blockDim.x - 1) {
-      s_run = run + og + sg;
-      s_tie_run = tie_run + oe + se;
-    }
-    __syncthreads();
+    gt += __popc(mg);
+    eq += __popc(me);
   }
   if (tid == 0 && count) count[r] = k;
 }
@@ -369,8 +388,6 @@ __global__ void __launch_bounds__(1024) topk_select_kernel(const float* __restri
 // atomics (scores crowd into a few exponent bytes, which serialises plain atomics) and read by all
 // eight CTAs over distributed shared memory; the compaction needs only the totals of the CTAs
 // before this one.  Output identical to topk_select_kernel.
-// (Measured for the many rows of a prefill chunk too, as 2 CTAs x 32 keys per thread: 1,058 us for
-// 2,048 rows x 32,768 scores against 816 us of the one-CTA kernel above, which therefore keeps them.)
 constexpr int kSelThreads = 512;
 
 template <int kSelCluster, int kSelKeysPerThread>
@@ -608,14 +625,65 @@ TF_API int tf_index_scores(const void* q, const float* w, const int* region, con
   return (int)cudaGetLastError();
 }
 
+// The same scores for the rows of a prefill: more than 32 rows of 128-dim heads whose count divides 256 (8, 16, 32 or
+// 64), groups of whole row tiles and 16-byte aligned queries run on the tcgen05 kernel, everything else as above.  The line lies at the
+// decode kernel's 32 rows: two row tiles of 32,768 keys are already 64 or more work items.
+TF_API int tf_index_scores_rows(const void* q, const float* w, const int* region, const int* nvalid, const void* keys,
+                                long key_region_stride, int key_row, int T, int Hi, int Di, int rows_per_group,
+                                float* scores, int lds, int key_lo, int key_hi, void* status, cudaStream_t st) {
+  const bool heads = Hi == 8 || Hi == 16 || Hi == 32 || Hi == 64;
+  if (T <= 32 || Di != 128 || !heads || rows_per_group < 1 || rows_per_group % (kItCols / Hi) || key_row % 4 ||
+      key_row < 68 || (reinterpret_cast<uintptr_t>(q) & 15) || (reinterpret_cast<uintptr_t>(keys) & 3) ||
+      key_region_stride % 4 || key_hi <= key_lo)
+    return tf_index_scores(q, w, region, nvalid, keys, key_region_stride, key_row, T, Hi, Di, rows_per_group, scores, lds,
+                           key_lo, key_hi, st);
+  ScoreParams p;
+  p.q = (const __nv_bfloat16*)q; p.w = w; p.region = region; p.nvalid = nvalid;
+  p.keys = (const uint8_t*)keys; p.key_region_stride = key_region_stride; p.key_row = key_row;
+  p.T = T; p.Hi = Hi; p.Di = Di; p.rows_per_group = rows_per_group; p.scores = scores; p.lds = lds;
+  p.key_lo = key_lo; p.key_hi = key_hi;
+  auto kernel = Hi == 8 ? index_score_tc_kernel<8> : Hi == 16 ? index_score_tc_kernel<16>
+              : Hi == 32 ? index_score_tc_kernel<32> : index_score_tc_kernel<64>;
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kItSmem);
+  if (e != cudaSuccess) return (int)e;
+  // key tiles per item: many, so that Q is converted seldom, while there are two items for every SM
+  const int rt = kItCols / Hi, row_tiles = (T + rt - 1) / rt, key_tiles = (key_hi - key_lo + kItKeys - 1) / kItKeys;
+  int per = 16;
+  while (per > 2 && (long)row_tiles * ((key_tiles + per - 1) / per) < 2L * sms) per /= 2;
+  const long items = (long)row_tiles * ((key_tiles + per - 1) / per);
+  if (items > 0x7fffffff) return -1;
+  tf_launch(kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(kItThreads), kItSmem, st, p, per, (int)items,
+            (TfStatusWord*)status);
+  return (int)cudaGetLastError();
+}
+
 TF_API int tf_topk_select(const float* scores, int lds, const int* nvalid, int k, int* out, int* count,
                           float* out_scores, int base, int T, cudaStream_t st) {
   // a few long rows (decode): one cluster of CTAs per row; many rows: one CTA per row fills the GPU
   if (T <= 32 && lds > 4096 && lds <= 8 * kSelThreads * 16)
     tf_launch(topk_select_cluster_kernel<8, 16>, dim3(8, T), dim3(kSelThreads), 0, st, scores, lds, nvalid, k, out,
               count, out_scores, base);
-  else
-    tf_launch(topk_select_kernel, dim3(T), dim3(1024), 0, st, scores, lds, nvalid, k, out, count, out_scores, base);
+  else if (lds <= kSelStage) {
+    static bool attr = false;
+    if (!attr) {
+      const cudaError_t e = cudaFuncSetAttribute(topk_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 kSelStage * 4);
+      if (e != cudaSuccess) return (int)e;
+      attr = true;
+    }
+    const int vec = lds % 4 == 0 && !(reinterpret_cast<uintptr_t>(scores) & 15);
+    tf_launch(topk_select_kernel<true>, dim3(T), dim3(kSelRowThreads), (size_t)(lds + 3) / 4 * 16, st, scores, lds, nvalid, k,
+              out, count, out_scores, base, vec);
+  } else {
+    tf_launch(topk_select_kernel<false>, dim3(T), dim3(kSelRowThreads), 0, st, scores, lds, nvalid, k, out, count, out_scores,
+              base, 0);
+  }
   return (int)cudaGetLastError();
 }
 

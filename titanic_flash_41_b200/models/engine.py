@@ -1006,15 +1006,15 @@ class Engine:
             Hi, Di = cfg.index_heads, cfg.index_dim
             for r0 in range(0, T, rows_t):
                 n = min(rows_t, T - r0)
-                native.call("tf_index_scores", b["iq"][r0:], b["iw"][r0:], region[r0:], nvalid[r0:], self.keys[sslot],
+                native.call("tf_index_scores_rows", b["iq"][r0:], b["iw"][r0:], region[r0:], nvalid[r0:], self.keys[sslot],
                             self.keys[sslot].stride(0), self.key_row, n, Hi, Di,
-                            rows_per_group, scores, scores.stride(0), 0, nmax)
+                            rows_per_group, scores, scores.stride(0), 0, nmax, self.status.t)
                 native.call("tf_topk_select", scores, scores.stride(0), nvalid[r0:], cfg.index_topk, sel[r0:], selcnt[r0:],
                             None, 0, n)
             return
-        native.call("tf_index_scores", b["iq"], b["iw"], region, nvalid, self.keys[sslot],
+        native.call("tf_index_scores_rows", b["iq"], b["iw"], region, nvalid, self.keys[sslot],
                     self.keys[sslot].stride(0), self.key_row, T, cfg.index_heads, cfg.index_dim,
-                    rows_per_group, scores, scores.stride(0), 0, nmax)
+                    rows_per_group, scores, scores.stride(0), 0, nmax, self.status.t)
         native.call("tf_topk_select", scores, scores.stride(0), nvalid, cfg.index_topk, sel, selcnt,
                     None, 0, T)
         if two_level and li == pub:
