@@ -6,8 +6,8 @@
 // A CTA takes 128 query rows of one head and walks the keys in tiles of 128; scores and probabilities
 // never leave the SM.  Four softmax warps (one accumulator lane = one query row per thread) turn S
 // into bf16 probabilities that go back to tensor memory as the A operand of PV; the reference maximum is the
-// first tile's and moves (O rescaled) only when a score exceeds it by 2^8, so the common path reads
-// S once.  One thread issues TMA (K and V rings of two tiles), one the MMAs: QK of tile j + 1 before
+// first tile's and moves (O rescaled) only when a score exceeds it by 2^8.  A row of S is read into
+// registers at once, so QK of tile j + 1 runs under the exponentials of tile j.  One thread issues TMA (K and V rings of two tiles), one the MMAs: QK of tile j + 1 before
 // PV of tile j.  256 tensor-memory columns (S 128, P 64, O 64) and 81 KB of shared memory: two CTAs share an SM,
 // and one's exponentials run while the other waits for its MMAs.
 //
@@ -26,7 +26,7 @@ constexpr int kTile = 128;                          // query rows of a CTA and k
 constexpr int kTileBytes = kTile * 128;             // 128 rows of 64 bf16
 constexpr int kRing = 2;
 constexpr int kVaThreads = 6 * 32;                  // 4 softmax warps, MMA warp, TMA warp
-constexpr int kVaSmem = kTileBytes * (1 + 2 * kRing) + 1024 + 128;
+constexpr int kVaSmem = kTileBytes * (1 + 2 * kRing) + 1024 + 256;
 constexpr int kVaCols = 256;
 constexpr float kVaNeg = -1e30f;
 
@@ -47,6 +47,17 @@ __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t v[32]
       "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
       "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t v[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t v[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
 }
 __device__ __forceinline__ void tmem_st_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -77,7 +88,7 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   uint8_t* tail = smem_raw + (base - raw) + kTileBytes * (1 + 2 * kRing);
   const uint32_t q_s = base, k_s = base + kTileBytes, v_s = k_s + kRing * kTileBytes;
   const uint32_t bar0 = v_s + kRing * kTileBytes;
-  const uint32_t q_full = bar0, s_ready = bar0 + 8, p_ready = bar0 + 16, o_done = bar0 + 24;
+  const uint32_t q_full = bar0, s_ready = bar0 + 8, p_ready = bar0 + 16, o_done = bar0 + 24, s_free = bar0 + 112;
   auto k_full = [&](int s) { return bar0 + 32u + 8u * s; };
   auto k_empty = [&](int s) { return bar0 + 48u + 8u * s; };
   auto v_full = [&](int s) { return bar0 + 64u + 8u * s; };
@@ -90,6 +101,7 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     tc::mbar_init(q_full, 1);
     tc::mbar_init(s_ready, 1);
     tc::mbar_init(p_ready, 4);
+    tc::mbar_init(s_free, 4);
     tc::mbar_init(o_done, 1);
     for (int s = 0; s < kRing; ++s) {
       tc::mbar_init(k_full(s), 1);
@@ -149,10 +161,9 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       bool ok = tc::mbar_wait(q_full, 0, abort_flag) && qk(0);
       for (int j = 0; j < tiles && ok; ++j) {
         const int s = j % kRing;
-        // P of tile j is in tensor memory: S has been read as well
+        // S of tile j has been read: QK of the next tile; then PV once P of tile j is in tensor memory
+        if (j + 1 < tiles && !(ok = tc::mbar_wait(s_free, j & 1, abort_flag) && qk(j + 1))) break;
         if (!(ok = tc::mbar_wait(p_ready, j & 1, abort_flag))) break;
-        tc::tc_fence_after();
-        if (j + 1 < tiles && !(ok = qk(j + 1))) break;
         if (!(ok = tc::mbar_wait(v_full(s), (j / kRing) & 1, abort_flag))) break;
         tc::tc_fence_after();
         const uint64_t dv = v_desc(v_s + s * kTileBytes);
@@ -176,71 +187,65 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
       const int valid = p.n - j * kTile;
       wait(s_ready, j & 1);
       tc::tc_fence_after();
-      if (j == 0) {
-        float cm = kVaNeg;
-#pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-          uint32_t v[32];
-          tc::tmem_ld32(tS + lane_off + q * 32, v);
-          tc::tmem_ld_wait();
+      // The whole row of S comes into registers at once, so QK of the next tile can overwrite it while this
+      // one is exponentiated.
+      uint32_t v[128];
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (q * 32 + i < valid) cm = fmaxf(cm, __uint_as_float(v[i]));
-        }
-        m = cm * p.scale_log2;
+      for (int q = 0; q < 4; ++q) tc::tmem_ld32(tS + lane_off + q * 32, v + q * 32);
+      tc::tmem_ld_wait();
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(s_free);
+      if (valid < kTile) {
+#pragma unroll
+        for (int i = 0; i < 128; ++i)
+          if (i >= valid) v[i] = __float_as_uint(-INFINITY);
       }
-      bool again = false;
-      do {
-        float cm0 = kVaNeg, cm1 = kVaNeg, ls[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-        for (int q = 0; q < 2; ++q) {
-          uint32_t v[64];
-          tc::tmem_ld32(tS + lane_off + q * 64, v);
-          tc::tmem_ld32(tS + lane_off + q * 64 + 32, v + 32);
+      float c0 = kVaNeg, c1 = kVaNeg, c2 = kVaNeg, c3 = kVaNeg;
+#pragma unroll
+      for (int i = 0; i < 128; i += 4) {
+        c0 = fmaxf(c0, __uint_as_float(v[i]));
+        c1 = fmaxf(c1, __uint_as_float(v[i + 1]));
+        c2 = fmaxf(c2, __uint_as_float(v[i + 2]));
+        c3 = fmaxf(c3, __uint_as_float(v[i + 3]));
+      }
+      const float cm = fmaxf(fmaxf(c0, c1), fmaxf(c2, c3)) * p.scale_log2;
+      if (j == 0) {
+        m = cm;
+      } else if (__any_sync(0xffffffffu, cm > m + 8.f)) {
+        // rare: the maximum moves; O and l are rescaled once the PV before is done
+        const float nm = fmaxf(m, cm), f = exp2f(m - nm);
+        m = nm;
+        l *= f;
+        wait(o_done, (j & 1) ^ 1);
+        tc::tc_fence_after();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          uint32_t o[8];
+          tmem_ld8(tO + lane_off + q * 8, o);
           tc::tmem_ld_wait();
-          uint32_t pk[32];
-          if (valid < kTile) {
 #pragma unroll
-            for (int i = 0; i < 64; ++i)
-              if (q * 64 + i >= valid) v[i] = __float_as_uint(-INFINITY);
-          }
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float x0 = __uint_as_float(v[2 * i]), x1 = __uint_as_float(v[2 * i + 1]);
-            cm0 = fmaxf(cm0, x0);
-            cm1 = fmaxf(cm1, x1);
-            const float a = exp2f(fmaf(x0, p.scale_log2, -m)), b = exp2f(fmaf(x1, p.scale_log2, -m));
-            ls[(2 * i) & 3] += a;
-            ls[(2 * i + 1) & 3] += b;
-            pk[i] = pack_bf16(a, b);
-          }
-          // P may be overwritten once the PV before has read it
-          if (q == 0 && j > 0) wait(o_done, (j & 1) ^ 1);
-          tmem_st_x32(tP + lane_off + q * 32, pk);
+          for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+          tmem_st8(tO + lane_off + q * 8, o);
         }
-        const float cm = fmaxf(cm0, cm1) * p.scale_log2;
-        again = __any_sync(0xffffffffu, cm > m + 8.f);
-        if (!again) {
-          l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
-        } else {
-          // rare: move the maximum, rescale O and l, exponentiate the tile again (PV before is done)
-          const float nm = fmaxf(m, cm), f = exp2f(m - nm);
-          m = nm;
-          l *= f;
-          if (j > 0) {
-            tc::tc_fence_after();
-#pragma unroll 1
-            for (int q = 0; q < 2; ++q) {
-              uint32_t o[32];
-              tc::tmem_ld32(tO + lane_off + q * 32, o);
-              tc::tmem_ld_wait();
+      }
+      float ls[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-              tmem_st_x32(tO + lane_off + q * 32, o);
-            }
-          }
+      for (int q = 0; q < 2; ++q) {
+        uint32_t pk[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float x0 = __uint_as_float(v[q * 64 + 2 * i]), x1 = __uint_as_float(v[q * 64 + 2 * i + 1]);
+          const float a = exp2f(fmaf(x0, p.scale_log2, -m)), b = exp2f(fmaf(x1, p.scale_log2, -m));
+          ls[(2 * i) & 3] += a;
+          ls[(2 * i + 1) & 3] += b;
+          pk[i] = pack_bf16(a, b);
         }
-      } while (again);
+        // P may be overwritten once the PV before has read it
+        if (q == 0 && j > 0) wait(o_done, (j & 1) ^ 1);
+        tmem_st_x32(tP + lane_off + q * 32, pk);
+      }
+      l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
       tmem_st_done();
       tc::tc_fence_before();
       __syncwarp();
