@@ -863,3 +863,32 @@ def test_topk_select_rows_edges(T, n, lds, k):
     for r in range(T):
         order = torch.sort(scores[r, :n].cpu(), descending=True, stable=True).indices[:k].sort().values
         assert torch.equal(sel[r].cpu().long(), order) and int(cnt[r]) == k
+
+
+@pytest.mark.parametrize("T,R,ld,kind", [(1, 1280, 1408, "f32"), (33, 40, 41, "f32"), (5, 1000, 1536, "bf16")])
+def test_rms_of_projection_columns(T, R, ld, kind):
+    """A column range of wider rows, widths off the block size: f16 rounding (2^-11) of an fp32 normalisation."""
+    torch.manual_seed(R)
+    x = torch.randn(T, ld, device=DEV).to(torch.float32 if kind == "f32" else torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(R, device=DEV)).bfloat16()
+    out = torch.zeros(T, R, device=DEV, dtype=torch.float16)
+    native.call("tf_rms_cols", x[:, ld - R:], 0 if kind == "f32" else 2, ld, w, out, T, R, 1e-6)
+    v = x[:, ld - R:].double()
+    want = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert ((out.double() - want).abs() <= 2.0 ** -11 * 1.01 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("M,G,R,K", [(1, 8, 128, 384), (24, 3, 1024, 512), (32, 2, 256, 128)])
+def test_block_diagonal_gemv(M, G, R, K):
+    """Every block reads its own K activations and writes its own columns (one tile, several tiles per block); f16 out."""
+    torch.manual_seed(M)
+    ws = [E.quant_fp8_device(torch.randn(R, K, device=DEV) * 0.1 * (g + 1)) for g in range(G)]
+    L = E.LayerWeights(wo_a=ws)
+    E.stack_blocks(L)
+    assert all(torch.equal(a.q.view(torch.uint8), b_.q.view(torch.uint8)) and torch.equal(a.s, b_.s) for a, b_ in zip(ws, L.wo_a))
+    x = torch.randn(M, G * K + 8, device=DEV).half()
+    out = torch.zeros(M, G * R, device=DEV, dtype=torch.float16)
+    native.call("tf_smallm_gemm_blocks", L.wo_a_all.q, L.wo_a_all.s, x, x.stride(0), out, out.stride(0), G, R, K, M)
+    for g in range(G):
+        want = x[:, g * K:(g + 1) * K].double() @ E.dequant_fp8(ws[g]).double().t()
+        assert float((out[:, g * R:(g + 1) * R].double() - want).norm() / want.norm()) < 2.0 ** -11 + 1e-5

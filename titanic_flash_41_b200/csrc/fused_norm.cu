@@ -86,7 +86,59 @@ __global__ void __launch_bounds__(1024) fused_norm_kernel(const FusedNormParams 
   row_norm_store(row, d, ss, p.eps, p.w, p.h16, p.hb, p.x8, p.x8s, r);
 }
 
+// RMSNorm of R columns of a projection's rows (fp32 or bf16) -> f16 rows [T, R].  One CTA per row; the row is
+// read twice (the second time from L1).  Replaces seven elementwise library launches.
+template <typename P>
+__global__ void __launch_bounds__(256) rms_cols_kernel(const P* __restrict__ x, long ldx, const __nv_bfloat16* __restrict__ w,
+                                                       __half* __restrict__ out, int R, float eps) {
+  tf_pdl_sync();
+  __shared__ float scratch[32];
+  const P* row = x + (long)blockIdx.x * ldx;
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < R; i += blockDim.x) {
+    const float v = (float)row[i];
+    ss += v * v;
+  }
+  const float inv = rsqrtf(block_sum(ss, scratch) / (float)R + eps);
+  for (int i = threadIdx.x; i < R; i += blockDim.x)
+    out[(long)blockIdx.x * R + i] = __float2half((float)row[i] * inv * __bfloat162float(w[i]));
+}
+
+// out = bf16(x + delta): the finished residual rows (eight elements a thread)
+__global__ void __launch_bounds__(256) residual_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ delta,
+                                                            __nv_bfloat16* __restrict__ out, long n) {
+  tf_pdl_sync();
+  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (i >= n) return;
+  const uint4 raw = *reinterpret_cast<const uint4*>(x + i);
+  const float4 a = *reinterpret_cast<const float4*>(delta + i), b = *reinterpret_cast<const float4*>(delta + i + 4);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const float2 x0 = __bfloat1622float2(h[0]), x1 = __bfloat1622float2(h[1]), x2 = __bfloat1622float2(h[2]), x3 = __bfloat1622float2(h[3]);
+  __nv_bfloat162 o[4] = {__floats2bfloat162_rn(x0.x + a.x, x0.y + a.y), __floats2bfloat162_rn(x1.x + a.z, x1.y + a.w),
+                         __floats2bfloat162_rn(x2.x + b.x, x2.y + b.y), __floats2bfloat162_rn(x3.x + b.z, x3.y + b.w)};
+  *reinterpret_cast<uint4*>(out + i) = *reinterpret_cast<uint4*>(o);
+}
+
 }  // namespace
+
+// x [T rows of R columns, pitch ldx elements] (x_kind 0 fp32, 2 bf16), w [R] bf16 -> out [T, R] f16
+TF_API int tf_rms_cols(const void* x, int x_kind, long ldx, const void* w, void* out, int T, int R, float eps,
+                       cudaStream_t st) {
+  if (T <= 0 || R <= 0 || !x || !w || !out) return T <= 0 ? 0 : -1;
+  if (x_kind == 0) tf_launch(rms_cols_kernel<float>, dim3(T), dim3(256), 0, st, (const float*)x, ldx, (const __nv_bfloat16*)w, (__half*)out, R, eps);
+  else if (x_kind == 2) tf_launch(rms_cols_kernel<__nv_bfloat16>, dim3(T), dim3(256), 0, st, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (__half*)out, R, eps);
+  else return -1;
+  return (int)cudaGetLastError();
+}
+
+// out[i] = bf16(x[i] + delta[i]), i < n (a multiple of 8; 16-byte aligned)
+TF_API int tf_residual_rows(const void* x, const float* delta, void* out, long n, cudaStream_t st) {
+  if (n <= 0) return 0;
+  if (n % 8 || (((uintptr_t)x | (uintptr_t)delta | (uintptr_t)out) & 15)) return -1;
+  tf_launch(residual_rows_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, (const __nv_bfloat16*)x, delta,
+            (__nv_bfloat16*)out, n);
+  return (int)cudaGetLastError();
+}
 
 // Exactly one of (delta) / (y_pair, ids, wts[, shared_y]) / neither feeds the residual add.
 TF_API int tf_add_norm_fused(void* x, const void* delta, const void* y_pair, const int* ids, const void* wts,

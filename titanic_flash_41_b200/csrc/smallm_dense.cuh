@@ -27,6 +27,8 @@ struct DenseParams {
   int ldy, out_kind;
   int N, K, M, tiles;
   float swiglu_limit;
+  int x_group_n;             // block-diagonal form: features [g x_group_n, (g + 1) x_group_n) read the K activations
+  int x_group_stride;        // that start at column g x_group_stride (0: one group)
 };
 
 constexpr int kDenseWarps = 8;
@@ -89,6 +91,7 @@ __global__ void __launch_bounds__(kDenseWarps * 32, MT <= 2 ? 2 : 1) smallm_dens
   int c_stage = 0;
   for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
     const int n0 = tile * FT;
+    const int x0 = p.x_group_n ? n0 / p.x_group_n * p.x_group_stride : 0;
     float acc[2][MT][4];
 #pragma unroll
     for (int ti = 0; ti < 2; ++ti)
@@ -105,7 +108,7 @@ __global__ void __launch_bounds__(kDenseWarps * 32, MT <= 2 ? 2 : 1) smallm_dens
         for (int m = 0; m < MT; ++m)
 #pragma unroll
           for (int e = 0; e < XV; ++e)
-            xv[s][m][e] = *reinterpret_cast<const uint4*>(xrow[m] + kb + s * (KB / 2) + e * 8);
+            xv[s][m][e] = *reinterpret_cast<const uint4*>(xrow[m] + x0 + kb + s * (KB / 2) + e * 8);
       float sc = 1.f, sc3 = 1.f;
       if (KIND == 0) {
         sc = __ldg(S + blk);

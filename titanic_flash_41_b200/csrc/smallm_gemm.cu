@@ -424,7 +424,7 @@ TF_API int tf_smallm_gemm(int kind, const void* W, const void* W3, const void* S
     DenseParams q;
     q.W = (const uint8_t*)W; q.W3 = (const uint8_t*)W3; q.S = (const float*)S; q.S3 = (const float*)S3;
     q.ldw = ldw; q.lds = lds; q.X = (const __half*)X; q.ldx = ldx; q.Y = Y; q.ldy = ldy; q.out_kind = out_kind;
-    q.N = N; q.K = K; q.M = M; q.tiles = 0; q.swiglu_limit = swiglu_limit;
+    q.N = N; q.K = K; q.M = M; q.tiles = 0; q.swiglu_limit = swiglu_limit; q.x_group_n = 0; q.x_group_stride = 0;
     if (kind == 2) return (int)launch_dense<2, false>(q, stream);
     return (int)(dual ? launch_dense<0, true>(q, stream) : launch_dense<0, false>(q, stream));
   }
@@ -450,6 +450,19 @@ TF_API int tf_smallm_gemm(int kind, const void* W, const void* W3, const void* S
   else if (kind == 2) e = launch<2, false>(p, slots, stream);
   else return -1;
   return (int)e;
+}
+
+// Block-diagonal FP8 matrix of `groups` blocks [R, K] stacked by rows (M <= 32): Y[r, g R + n] = sum_k X[r, g K + k]
+// W[g R + n, k], f16 out.  One launch streams all blocks; a launch per block left a 4 MB matrix on 32
+// CTAs (eight launches of 4.8 us each at R 1024, K 4096).
+TF_API int tf_smallm_gemm_blocks(const void* W, const void* S, const void* X, int ldx, void* Y, int ldy, int groups, int R,
+                                 int K, int M, cudaStream_t stream) {
+  if (groups < 1 || R % 128 || K % 128 || ldx % 8 || M < 1 || M > 32 || !W || !S || !X || !Y) return -1;
+  DenseParams q;
+  q.W = (const uint8_t*)W; q.W3 = nullptr; q.S = (const float*)S; q.S3 = nullptr; q.ldw = K; q.lds = K / 128;
+  q.X = (const __half*)X; q.ldx = ldx; q.Y = Y; q.ldy = ldy; q.out_kind = 1; q.N = groups * R; q.K = K; q.M = M;
+  q.tiles = 0; q.swiglu_limit = 0.f; q.x_group_n = R; q.x_group_stride = K;
+  return (int)launch_dense<0, false>(q, stream);
 }
 
 // Dense FP8 GEMV (M <= 32) fused with the tensor-parallel all-reduce, the residual update and the

@@ -80,6 +80,7 @@ class LayerWeights:
     q_norm: Optional[torch.Tensor] = None          # low-rank query: proj holds wq_a, then norm, then wq_b
     wq_b: Optional[Fp8Weight] = None
     wo_a: Optional[List[Fp8Weight]] = None         # grouped output projection: one [rank, per] per local group
+    wo_a_all: Optional[Fp8Weight] = None           # the same blocks stacked by rows (decode streams them in one launch)
     hc: Optional[Dict[str, Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]] = None   # "attn"/"ffn" -> (fn, base, scale)
     # unsharded dense matrices of this layer (all heads, full shared expert) for the sequence-parallel
     # prefill, where every rank runs whole rows through the dense sublayers (reference: the derived
@@ -154,6 +155,17 @@ def dequant_mxfp4(p: torch.Tensor, code: torch.Tensor) -> torch.Tensor:
     *lead, K = v.shape
     s = torch.exp2(code.float() - 127).unsqueeze(-1)
     return (v.reshape(*lead, K // 32, 32) * s).reshape(*lead, K)
+
+
+def stack_blocks(L: LayerWeights) -> None:
+    """Lay the blocks of a grouped output projection out behind one another (``wo_a_all``); ``wo_a``
+    becomes views of that one matrix."""
+    if not L.wo_a or L.wo_a_all is not None or len({(w.n, w.k) for w in L.wo_a}) != 1 or L.wo_a[0].n % 128:
+        return
+    n, k = L.wo_a[0].n, L.wo_a[0].k
+    q, s = torch.cat([w.q for w in L.wo_a]), torch.cat([w.s for w in L.wo_a])
+    L.wo_a_all = Fp8Weight(q, s, n * len(L.wo_a), k)
+    L.wo_a = [Fp8Weight(q[i * n:(i + 1) * n], s[i * n // 128:(i + 1) * n // 128], n, k, w.sfu) for i, w in enumerate(L.wo_a)]
 
 
 def _layer_prefix(cfg: ModelConfig, li: int) -> str:
@@ -484,6 +496,8 @@ class Engine:
         self.layers = layers
         self.draft_layers = draft_layers or []
         self.draft_extra = draft_extra or {}
+        for L in self.layers + self.draft_layers:
+            stack_blocks(L)
         self.embed_w, self.head_w, self.final_norm = embed, head, final_norm
         native.lib()
         native.set_pdl(bool(getattr(ecfg, "pdl", False)))
@@ -798,9 +812,8 @@ class Engine:
         if cfg.q_lora_rank:
             # low-rank query: RMSNorm of the wq_a output, then this rank's heads through wq_b
             R = cfg.q_lora_rank
-            qa = P[:T, o["qa"]:o["qa"] + R].float()
-            qa = qa * torch.rsqrt(qa.pow(2).mean(-1, keepdim=True) + cfg.rms_eps) * L.q_norm.float()
-            b["qa16"][:T].copy_(qa)
+            native.call("tf_rms_cols", P[:, o["qa"]:], 0 if P.dtype == torch.float32 else 2, P.stride(0), L.q_norm, b["qa16"],
+                        T, R, cfg.rms_eps)
             q_off = self.q_col
             self._linear(b["qa16"], L.wq_b, P[:, q_off:q_off + Hl * Dh], T)
         slot = self.src_slot.get(li, 0)
@@ -840,8 +853,12 @@ class Engine:
             # grouped low-rank output projection: block-diagonal wo_a per local head group, then wo_b
             G, R = cfg.o_groups // self.world, cfg.o_lora_rank
             per = Hl * Dh // G
-            for g in range(G):
-                self._linear(b["a16"][:, g * per:(g + 1) * per], L.wo_a[g], b["mid16"][:, g * R:(g + 1) * R], T)
+            if T <= self.SMALL_M and L.wo_a_all is not None:
+                native.call("tf_smallm_gemm_blocks", L.wo_a_all.q, L.wo_a_all.s, b["a16"], b["a16"].stride(0), b["mid16"],
+                            b["mid16"].stride(0), G, R, per, T)
+            else:
+                for g in range(G):
+                    self._linear(b["a16"][:, g * per:(g + 1) * per], L.wo_a[g], b["mid16"][:, g * R:(g + 1) * R], T)
             wo_in = b["mid16"]
         if hc:
             # the reduced sublayer output goes through the hc post-mix instead of a plain add
@@ -1309,6 +1326,13 @@ class Engine:
         if self.cfg.hc_mult > 1 or not b.get("pending"):
             return b["x"][rows].clone()
         return (b["x"][rows].float() + b["delta"][rows]).to(torch.bfloat16)
+
+    def residual_into(self, b: dict, T: int, out: torch.Tensor) -> None:
+        """The same for rows [0, T), written to ``out`` (contiguous bf16 rows) in one pass."""
+        if self.cfg.hc_mult > 1 or not b.get("pending"):
+            out.copy_(b["x"][:T])
+        else:
+            native.call("tf_residual_rows", b["x"], b["delta"], out, T * self.cfg.hidden)
 
     def _head(self, T: int, b: dict, rows: Optional[torch.Tensor], draft: bool = False,
               local: bool = False) -> Optional[torch.Tensor]:

@@ -72,7 +72,7 @@ def _encoder_layer_major(eng: Engine, region: int, toks: np.ndarray, sizes: List
             eng.run(T, b, shapes[c][0], shapes[c][1], None, li, li + 1, x_in=None if li == 0 else resid[lo:hi],
                     x_patch=_patch_for(embeds, lo, T, eng.dev) if li == 0 else None)
             # x + pending sublayer output, rounded once to bf16
-            resid[lo:hi].copy_(eng.residual_rows(b, slice(0, T)) if b.get("pending") else b["x"][:T])
+            eng.residual_into(b, T, resid[lo:hi])
             if Lw.is_index_source:
                 if li not in sel_store:
                     sel_store.clear()             # followers only ever read the latest source
