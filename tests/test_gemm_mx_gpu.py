@@ -166,7 +166,8 @@ def test_moe_plan_tables(El, e_lo, pairs):
     cap = pairs // 128 + El + 1
     for _ in range(2):
         offs, cur, tile_e, nt, pad, dst = i32(El + 1), i32(El), i32(cap), i32(1), i32(1), i32(pairs)
-        native.call("tf_moe_plan", ids.to(DEV), pairs, e_lo, El, counts, offs, cur, tile_e, cap, nt, pad, dst)
+        tile_r = i32(cap)
+        native.call("tf_moe_plan_rows", ids.to(DEV), pairs, e_lo, El, counts, offs, cur, tile_e, tile_r, cap, nt, pad, dst)
         local = ids.long() - e_lo
         mine = (local >= 0) & (local < El)
         cnt = torch.bincount(local[mine], minlength=El)
@@ -174,7 +175,37 @@ def test_moe_plan_tables(El, e_lo, pairs):
         want = torch.cat([torch.zeros(1, dtype=torch.long), torch.cumsum(tiles * 128, 0)])
         assert torch.equal(offs.cpu().long(), want) and int(nt) == int(tiles.sum()) and int(pad) == int(want[-1])
         assert torch.equal(tile_e[:int(nt)].cpu().long(), torch.arange(El).repeat_interleave(tiles))
+        first = torch.cat([torch.arange(int(t)) for t in tiles]) if int(nt) else torch.zeros(0)
+        assert torch.equal(tile_r[:int(nt)].cpu().long(), (cnt.repeat_interleave(tiles) - 128 * first).clamp(max=128).long())
         d = dst.cpu().long()
         assert bool((d[~mine] == -1).all()) and d[mine].unique().numel() == int(mine.sum())
         assert bool(((d[mine] >= want[local[mine]]) & (d[mine] < want[local[mine]] + cnt[local[mine]])).all())
         assert int(counts.abs().sum()) == 0
+
+
+def test_grouped_gemm_and_swiglu_store_only_rows_that_count():
+    """Tiles of 1, 32, 33, 127 and 128 rows: rows that count equal the form that stores whole tiles bit for bit, padding keeps
+    what it held; the activation kernel skips the same rows."""
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    rows = torch.tensor([1, 32, 33, 127, 128], dtype=torch.int32, device=DEV)
+    El, N, K, M = 5, 256, 256, 640
+    a = _random_fp8(M, K, gen)
+    sfa, sfb = torch.full((K // 128, M // 32, 128), 127, dtype=torch.uint8, device=DEV), torch.full((K // 128, El * N // 32, 128), 124, dtype=torch.uint8, device=DEV)
+    w = torch.randint(0, 256, (El * N, K // 2), dtype=torch.uint8, device=DEV, generator=gen)
+    tiles, nt = torch.arange(5, dtype=torch.int32, device=DEV), torch.tensor([5], dtype=torch.int32, device=DEV)
+    st = native.StatusWord(DEV)
+    whole, part = torch.zeros(M, N, device=DEV), torch.full((M, N), 3.0, device=DEV)
+    kw = dict(b_fp4=True, b_rows=El * N, tile_expert=tiles, num_m_tiles=nt)
+    mx.gemm(a, sfa, w, sfb, whole, M, N, K, st.t, **kw)
+    mx.gemm(a, sfa, w, sfb, part, M, N, K, st.t, tile_rows=rows, **kw)
+    st.check()
+    live = (torch.arange(M, device=DEV) % 128) < rows.repeat_interleave(128)
+    assert torch.equal(part[live], whole[live]) and bool((part[~live] == 3.0).all())
+    y = torch.randn(M, 2 * N, device=DEV, generator=gen).bfloat16()
+    q = [torch.full((M, N), 9, dtype=torch.uint8, device=DEV) for _ in range(2)]
+    sf = [torch.full((N // 128, M // 32, 128), 9, dtype=torch.uint8, device=DEV) for _ in range(2)]
+    n = torch.tensor([M], dtype=torch.int32, device=DEV)
+    for i, tr in enumerate((None, rows)):
+        native.call("tf_swiglu_rows_mx_units", y, 2 * N, q[i], sf[i], M // 32, M, N, 10.0, n, tr)
+    assert torch.equal(q[1][live], q[0][live]) and bool((q[1][~live] == 9).all())
+    assert torch.equal(mx.units_to_rowmajor(sf[1], M)[live], mx.units_to_rowmajor(sf[0], M)[live])

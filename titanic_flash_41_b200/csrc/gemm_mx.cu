@@ -62,6 +62,7 @@ struct MxGemmParams {
   int out_kind;              // 0 f32, 2 bf16
   const int* tile_expert;
   const int* num_m_tiles;
+  const int* tile_rows;      // rows of an M tile that count (null: all); the others are not stored
   TfStatusWord* status;
 };
 
@@ -241,6 +242,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       coord(tile, mi, ni);
       const int m0 = mi * BM, n0 = ni * BN;
       const int row = m0 + quad * 32 + lane;
+      const bool live = row < p.M && (!p.tile_rows || quad * 32 + lane < p.tile_rows[mi]);
       const int col0 = n0 + half * 128;
       if (!(ok = tc::mbar_wait(tfull, n_tile & 1, abort_flag))) break;
       tc::tc_fence_after();
@@ -256,7 +258,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(tempty);
         }
-        if (row < p.M) {
+        if (live) {
           const long off = (long)row * p.ldc + col0 + c;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -358,17 +360,20 @@ __global__ void __launch_bounds__(128) quant_rows_mx_units_kernel(const T* __res
 }
 
 // Clamped SwiGLU of [rows, 2I] bf16 (gate | up) -> MXFP8 rows [rows, I] + unit-layout scales.
-// One thread per (row, 32 outputs).  `num_rows` (device, optional) bounds the rows at run time.
+// One thread per (row, 32 outputs).  `num_rows` (device, optional) bounds the rows at run time, `tile_rows` (optional)
+// the rows of each 128-row tile.
 __global__ void __launch_bounds__(128) swiglu_rows_mx_units_kernel(const __nv_bfloat16* __restrict__ y, int ldy,
                                                                    uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
                                                                    int sf_units, int rows, int I, float limit,
-                                                                   const int* __restrict__ num_rows) {
+                                                                   const int* __restrict__ num_rows,
+                                                                   const int* __restrict__ tile_rows) {
   tf_pdl_sync();
   const int ks = I / 32;
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int live = num_rows ? min(rows, *num_rows) : rows;
   if (i >= (long)live * ks) return;
   const int r = (int)(i / ks), b = (int)(i % ks);
+  if (tile_rows && (r & 127) >= tile_rows[r >> 7]) return;           // padding
   const __nv_bfloat16* g = y + (long)r * ldy + b * 32;
   const __nv_bfloat16* u = g + I;
   __nv_bfloat16 gr[32], ur[32];
@@ -537,9 +542,12 @@ TF_API long tf_mx_sf_units(long rows, int tile_rows) {
 // sfa / sfb: unit-layout scales with sfa_units / sfb_units units per 128-deep k block
 // (tf_mx_sf_units(M, 128) and tf_mx_sf_units(b_rows, 256) or more).  Grouped form: tile_expert /
 // num_m_tiles as in tf_gemm_tc, b_rows = experts * N, N a multiple of 256.
-TF_API int tf_gemm_mx(const void* A, long lda, const void* B, long ldb, long b_rows, int b_fp4, const void* sfa,
-                      int sfa_units, const void* sfb, int sfb_units, void* C, int ldc, int out_kind, int M, int N,
-                      int K, const int* tile_expert, const int* num_m_tiles, void* status, cudaStream_t st) {
+// tile_rows (grouped form, optional): rows of every M tile that count.  Padding is computed but not stored: at a few rows
+// per expert the stores of whole tiles were a quarter of the weights' bytes.
+TF_API int tf_gemm_mx_rows(const void* A, long lda, const void* B, long ldb, long b_rows, int b_fp4, const void* sfa,
+                           int sfa_units, const void* sfb, int sfb_units, void* C, int ldc, int out_kind, int M, int N,
+                           int K, const int* tile_expert, const int* num_m_tiles, const int* tile_rows, void* status,
+                           cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0 || K % BK || N % 8 || (out_kind != 0 && out_kind != 2)) return -1;
   if (!A || !B || !sfa || !sfb || !C) return -1;
   if (tile_expert && (N % BN || !num_m_tiles)) return -1;
@@ -566,12 +574,19 @@ TF_API int tf_gemm_mx(const void* A, long lda, const void* B, long ldb, long b_r
   p.sfa = reinterpret_cast<const uint8_t*>(sfa); p.sfb = reinterpret_cast<const uint8_t*>(sfb);
   p.sfa_units = sfa_units; p.sfb_units = sfb_units;
   p.C = C; p.ldc = ldc; p.out_kind = out_kind;
-  p.tile_expert = tile_expert; p.num_m_tiles = num_m_tiles;
+  p.tile_expert = tile_expert; p.num_m_tiles = num_m_tiles; p.tile_rows = tile_expert ? tile_rows : nullptr;
   p.status = reinterpret_cast<TfStatusWord*>(status);
   const long tiles = m_tiles * n_tiles;
   const int grid = (int)(tiles < g_sms ? tiles : g_sms);
   tf_launch(gemm_mx_kernel, dim3(grid), dim3(kThreads), kSmemBytes, st, mA, mB, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+TF_API int tf_gemm_mx(const void* A, long lda, const void* B, long ldb, long b_rows, int b_fp4, const void* sfa,
+                      int sfa_units, const void* sfb, int sfb_units, void* C, int ldc, int out_kind, int M, int N,
+                      int K, const int* tile_expert, const int* num_m_tiles, void* status, cudaStream_t st) {
+  return tf_gemm_mx_rows(A, lda, B, ldb, b_rows, b_fp4, sfa, sfa_units, sfb, sfb_units, C, ldc, out_kind, M, N, K,
+                         tile_expert, num_m_tiles, nullptr, status, st);
 }
 
 // x [rows / x_div source rows, K] (xkind 0 f32, 1 f16, 2 bf16; row pitch ldx elements) -> q e4m3
@@ -598,12 +613,12 @@ TF_API int tf_quant_rows_mx_units(const void* x, int xkind, int ldx, int x_div, 
 }
 
 TF_API int tf_swiglu_rows_mx_units(const void* y, int ldy, void* q, void* sf, int sf_units, int rows, int I,
-                                   float limit, const int* num_rows, cudaStream_t st) {
+                                   float limit, const int* num_rows, const int* tile_rows, cudaStream_t st) {
   if (rows <= 0 || I % 128 || !y || !q || !sf || ldy % 8 || (reinterpret_cast<uintptr_t>(y) & 15)) return -1;
   const long n = (long)rows * (I / 32);
   tf_launch(swiglu_rows_mx_units_kernel, dim3((unsigned)((n + 127) / 128)), dim3(128), 0, st,
             reinterpret_cast<const __nv_bfloat16*>(y), ldy, reinterpret_cast<uint8_t*>(q),
-            reinterpret_cast<uint8_t*>(sf), sf_units, rows, I, limit, num_rows);
+            reinterpret_cast<uint8_t*>(sf), sf_units, rows, I, limit, num_rows, tile_rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

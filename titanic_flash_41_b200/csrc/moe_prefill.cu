@@ -124,15 +124,15 @@ __global__ void moe_count_kernel(const int* __restrict__ ids, int n_pairs, int e
 // threads in further passes): one thread walking 256 experts spent 36 us on its chain of loads.
 constexpr int kOffThreads = 512;
 __global__ void __launch_bounds__(kOffThreads) moe_offsets_kernel(int* counts, int El, int* offsets, int* cursor,
-                                                                  int* tile_expert, int max_tiles, int* num_tiles,
-                                                                  int* padded_rows) {
+                                                                  int* tile_expert, int* tile_rows, int max_tiles,
+                                                                  int* num_tiles, int* padded_rows) {
   tf_pdl_sync();
   __shared__ int wsum[kOffThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int before = 0;                                  // tiles of the passes before
   for (int e0 = 0; e0 < El; e0 += kOffThreads) {
     const int e = e0 + threadIdx.x;
-    const int tiles = e < El ? (counts[e] + 127) / 128 : 0;
+    const int cnt = e < El ? counts[e] : 0, tiles = (cnt + 127) / 128;
     int inc = tiles;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -153,7 +153,10 @@ __global__ void __launch_bounds__(kOffThreads) moe_offsets_kernel(int* counts, i
       offsets[e] = t0 * 128;
       cursor[e] = 0;
       counts[e] = 0;                               // ready for the next launch
-      for (int j = 0; j < tiles && t0 + j < max_tiles; ++j) tile_expert[t0 + j] = e;
+      for (int j = 0; j < tiles && t0 + j < max_tiles; ++j) {
+        tile_expert[t0 + j] = e;
+        if (tile_rows) tile_rows[t0 + j] = min(128, cnt - 128 * j);
+      }
     }
     before += all;
     __syncthreads();
@@ -353,15 +356,23 @@ TF_API int tf_swiglu_rows(const void* y, int y_kind, long ldy, void* out16, long
   return (int)cudaGetLastError();
 }
 
-// counts must be zero on entry (it is left zeroed).  tile_expert capacity = max_tiles.
+// counts must be zero on entry (it is left zeroed).  tile_expert capacity = max_tiles; tile_rows (optional, the same
+// capacity) receives the rows of a tile that belong to a pair (the rest of its 128 is padding).
+TF_API int tf_moe_plan_rows(const int* ids, int n_pairs, int e_lo, int El, int* counts, int* offsets, int* cursor,
+                            int* tile_expert, int* tile_rows, int max_tiles, int* num_tiles, int* padded_rows,
+                            int* pair_dst, cudaStream_t st) {
+  const unsigned grid = (unsigned)((n_pairs + 255) / 256);
+  tf_launch(moe_count_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, counts);
+  tf_launch(moe_offsets_kernel, dim3(1), dim3(kOffThreads), 0, st, counts, El, offsets, cursor, tile_expert, tile_rows, max_tiles, num_tiles, padded_rows);
+  tf_launch(moe_place_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, offsets, cursor, pair_dst);
+  return (int)cudaGetLastError();
+}
+
 TF_API int tf_moe_plan(const int* ids, int n_pairs, int e_lo, int El, int* counts, int* offsets, int* cursor,
                        int* tile_expert, int max_tiles, int* num_tiles, int* padded_rows, int* pair_dst,
                        cudaStream_t st) {
-  const unsigned grid = (unsigned)((n_pairs + 255) / 256);
-  tf_launch(moe_count_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, counts);
-  tf_launch(moe_offsets_kernel, dim3(1), dim3(kOffThreads), 0, st, counts, El, offsets, cursor, tile_expert, max_tiles, num_tiles, padded_rows);
-  tf_launch(moe_place_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, offsets, cursor, pair_dst);
-  return (int)cudaGetLastError();
+  return tf_moe_plan_rows(ids, n_pairs, e_lo, El, counts, offsets, cursor, tile_expert, nullptr, max_tiles, num_tiles,
+                          padded_rows, pair_dst, st);
 }
 
 // w [E, N, K/2], sc [E, N, K/32] -> out rows [out_row0, out_row0+N) of every expert's [out_N, K] fp8 matrix

@@ -124,7 +124,8 @@ class BigPath:
         ntile = self._get("ntile", (2,), i32)
         pair_dst = self._get("pair_dst", (npairs,), i32)
         e_lo = eng.rank * El
-        native.call("tf_moe_plan", b["ids"], npairs, e_lo, El, z, offsets, cursor, tile_e, max_tiles, ntile[0:1],
+        tile_r = self._get("tile_r", (max_tiles,), i32)
+        native.call("tf_moe_plan_rows", b["ids"], npairs, e_lo, El, z, offsets, cursor, tile_e, tile_r, max_tiles, ntile[0:1],
                     ntile[1:2], pair_dst)
         st = eng.status.t
         if eng.ecfg.prefill_mx and d % 128 == 0 and I % 256 == 0 and d % 256 == 0:
@@ -145,15 +146,16 @@ class BigPath:
             mx.quant_rows(b["h16"], npairs, d, xp, sfx, x_div=k, pair_dst=pair_dst)
             y1 = self._get("y1", (cap, 2 * I), torch.bfloat16)
             mx.gemm(xp, sfx, L.ew1, u1, y1, cap, I, d, st, b_fp4=True, b_rows=El * I, tile_expert=tile_e,
-                    num_m_tiles=ntile[0:1])
+                    num_m_tiles=ntile[0:1], tile_rows=tile_r)
             mx.gemm(xp, sfx, L.ew3, u3, y1[:, I:], cap, I, d, st, b_fp4=True, b_rows=El * I, tile_expert=tile_e,
-                    num_m_tiles=ntile[0:1])
+                    num_m_tiles=ntile[0:1], tile_rows=tile_r)
             aq = self._get("aq", (cap, I), torch.uint8)
             sfq = self._get("sfq_mx", (I // 128, cap // 32, 128), torch.uint8)
-            native.call("tf_swiglu_rows_mx_units", y1, 2 * I, aq, sfq, cap // 32, cap, I, cfg.swiglu_limit, ntile[1:2])
+            native.call("tf_swiglu_rows_mx_units", y1, 2 * I, aq, sfq, cap // 32, cap, I, cfg.swiglu_limit, ntile[1:2],
+                        tile_r)
             y2 = self._get("y2", (cap, d), torch.bfloat16)
             mx.gemm(aq, sfq, L.ew2, u2, y2, cap, d, I, st, b_fp4=True, b_rows=El * d, tile_expert=tile_e,
-                    num_m_tiles=ntile[0:1])
+                    num_m_tiles=ntile[0:1], tile_rows=tile_r)
             self._moe_tail(eng, L, T, b, y2, pair_dst, with_shared, out)
             return
         # expert weights of this layer as block-scaled FP8: [El, 2I, d] (w1 | w3) and [El, d, I]

@@ -46,10 +46,10 @@ def quant_rows(x: torch.Tensor, M: int, K: int, q: torch.Tensor, sf: torch.Tenso
 
 
 def gemm(a_q: torch.Tensor, sfa: torch.Tensor, b_q: torch.Tensor, sfb: torch.Tensor, out: torch.Tensor, M: int, N: int,
-         K: int, status, b_fp4: bool = False, b_rows: int = 0, tile_expert=None, num_m_tiles=None) -> None:
+         K: int, status, b_fp4: bool = False, b_rows: int = 0, tile_expert=None, num_m_tiles=None, tile_rows=None) -> None:
     okind = {torch.float32: 0, torch.bfloat16: 2}[out.dtype]
-    native.call("tf_gemm_mx", a_q, K, b_q, K // 2 if b_fp4 else K, b_rows or N, 1 if b_fp4 else 0, sfa, sfa.shape[1], sfb,
-                sfb.shape[1], out, out.stride(0), okind, M, N, K, tile_expert, num_m_tiles, status)
+    native.call("tf_gemm_mx_rows", a_q, K, b_q, K // 2 if b_fp4 else K, b_rows or N, 1 if b_fp4 else 0, sfa, sfa.shape[1], sfb,
+                sfb.shape[1], out, out.stride(0), okind, M, N, K, tile_expert, num_m_tiles, tile_rows, status)
 
 
 def units_to_rowmajor(sf: torch.Tensor, rows: int) -> torch.Tensor:
