@@ -207,3 +207,30 @@ def test_per_conversation_block_lengths_equal_shorter_blocks(world):
         assert int(n1[0]) == int(nacc[s]) and int(t1[0]) == int(tok[s]), (s, k)
         differs |= k < g and (int(full[3][s]) != int(nacc[s]) or int(full[4][s]) != int(tok[s]))
     assert differs            # the shorter blocks are not what the full blocks would have committed
+
+
+@pytest.mark.parametrize("V", [4096, 129280])
+def test_row_statistics_of_crowded_and_spread_rows(V):
+    """The first digit's private bins follow the row maximum: rows of one sign, of both, with maxima at the ends of a bin,
+    negative maxima, zeros, equal values and a range beyond the eight bins give the statistics of the full-row kernels."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    n = lambda: torch.randn(V, device=DEV, generator=g)
+    z = torch.zeros(V, device=DEV)
+    spread = torch.exp2(torch.rand(V, device=DEV, generator=g) * 40 - 36) * torch.where(n() > 0, 1.0, -1.0)
+    rows = [n() * 3, n().abs() * 2 + 1, -n().abs() - 0.5, n() * 1e-4, z, -z, z + 7.25, z - 3.5, spread, n() * 3 + 15.999,
+            torch.cat([z[:1] + 128.0, n()[1:] * 2 - 40.0]), -spread.abs() - 1e-12]
+    lg = torch.stack(rows).contiguous()
+    S = lg.shape[0]
+    temp = torch.full((S,), 0.8, device=DEV)
+    sb = native.lib().tf_rowstat_bytes()
+    st = native.StatusWord(DEV)
+    for p in (0.9, 0.999, 1.0):
+        topp = torch.full((S,), p, device=DEV)
+        ws = SampleWorkspace(V, S, DEV)
+        got, want = torch.zeros(S, sb, dtype=torch.uint8, device=DEV), torch.zeros(S, sb, dtype=torch.uint8, device=DEV)
+        u, tok = torch.rand(S, 1, dtype=torch.float64, device=DEV, generator=g), torch.zeros(S, dtype=torch.int32, device=DEV)
+        ws.sample(lg, None, None, None, u, 1, temp, topp, S, 0, V, got, 1, None, tok, 1, st.t)
+        scratch = torch.zeros(native.lib().tf_rowstats_scratch_bytes(S), dtype=torch.uint8, device=DEV)
+        native.call("tf_rowstats_per_session", lg, V, V, S, temp, topp, 1, want, scratch, st.t)
+        st.check()
+        assert torch.equal(got, want), (p, [i for i in range(S) if not torch.equal(got[i], want[i])])

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
   float* tbuf = reinterpret_cast<float*>(smem);
   float* dbuf = tbuf + p.chunk;
   unsigned long long* whist = reinterpret_cast<unsigned long long*>(dbuf + p.chunk);   // [32][256]
-  __shared__ unsigned long long gpart[4][256], wtot[8];
+  __shared__ unsigned long long gpart[4][256], fb[256], wtot[8];
   __shared__ double wm[32], cm[(kMaxG + 1) * kMaxP], Rrow[kMaxG + 1], wrow[kMaxG + 1], ptq[2 * kMaxG];
   __shared__ float redf[32];
   __shared__ int redi[32];
@@ -242,12 +242,45 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
     const int shift = 24 - 8 * level;
     const unsigned int tag = tag0 + 1 + level;
     for (int k = threadIdx.x; k < 32 * 256; k += kThreads) whist[k] = 0;
+    if (threadIdx.x < 256) fb[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t prefix = s_prefix, mask = s_mask;
     const unsigned long long above = s_above, target_prev = s_target;
-    {
-      // a thread's consecutive elements mostly fall into the same few bins (the top key bits are the
-      // sign and the exponent): add up a run privately and touch shared memory once per run
+    if (level == 0) {
+      // The top key bits are the sign and most of the exponent: nearly all of a row falls into a handful of bins,
+      // and atomics on them serialise (30,000 cycles of the 93,000 of a launch).  The eight bins next to the row
+      // maximum -- four of its sign and four of the other, or eight below a negative maximum -- therefore get a
+      // private word per thread (conflict-free); only the rest takes atomics.
+      const int top = (int)(mkey >> 24);
+      const bool pos = top >= 128;
+      auto class_of = [&](int bin) -> int {
+        if (!pos) return top - bin;
+        return bin >= 128 ? (bin >= top - 3 ? top - bin : 8) : bin + top - 250;
+      };
+      auto bin_of = [&](int cls) -> int { return !pos ? top - cls : cls < 4 ? top - cls : cls - top + 250; };
+      unsigned long long* priv = whist + warp * 256 + lane;            // [class][lane]
+      for (int k = threadIdx.x; k < n; k += kThreads) {
+        const float v = tbuf[k];
+        const int bin = (int)(fkey(v) >> 24), cls = class_of(bin);
+        const unsigned long long mass = (unsigned long long)((double)expf((v - stat.m) * inv_t) * kFix);
+        if (cls >= (pos && bin < 128 ? 4 : 0) && cls < 8) priv[cls * 32] += mass;
+        else if (mass) atomicAdd(&fb[bin], mass);
+      }
+      __syncthreads();
+      {
+        // class = threadIdx.x / 128; a thread adds eight warps' words of one lane
+        const int cls = threadIdx.x >> 7, w0 = (warp & 3) * 8, bin = bin_of(cls);
+        unsigned long long acc = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) acc += whist[(w0 + w) * 256 + cls * 32 + lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0 && acc) atomicAdd(&fb[bin], acc);
+      }
+      __syncthreads();
+    } else {
+      // few elements share the digits found so far, and these digits spread them; a run of one bin (equal logits) is
+      // added up privately and touches shared memory once
       int cur = -1;
       unsigned long long run = 0;
       for (int k = threadIdx.x; k < n; k += kThreads) {
@@ -264,11 +297,12 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
         run += mass;
       }
       if (cur >= 0) atomicAdd(&whist[warp * 256 + cur], run);
+      __syncthreads();
     }
-    __syncthreads();
     if (threadIdx.x < 256) {
-      unsigned long long acc = 0;
-      for (int w = 0; w < 32; ++w) acc += whist[w * 256 + threadIdx.x];
+      unsigned long long acc = fb[threadIdx.x];
+      if (level > 0)
+        for (int w = 0; w < 32; ++w) acc += whist[w * 256 + threadIdx.x];
       push2(p, A.hist + ((((long)(level & 1) * P + part) * p.max_rows + row) * 256 + threadIdx.x) * 2, (uint32_t)acc,
             (uint32_t)(acc >> 32), tag);
     }
