@@ -627,9 +627,8 @@ TF_API int tf_sparse_attention(const void* q, int T, int Hl, int Dh, const int* 
       cudaFuncSetAttribute(sparse_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
       cudaFuncSetAttribute(sparse_attn_tcw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTwSmem);
     }
-    const dim3 g(T < g_attn_sms ? T : g_attn_sms);
-    if (Dh == 128) tf_launch(sparse_attn_tc_kernel, g, dim3(kTcThreads), kTcSmem, st, p);
-    else tf_launch(sparse_attn_tcw_kernel, g, dim3(kTcThreads), kTwSmem, st, p);
+    if (Dh == 128) tf_launch(sparse_attn_tc_kernel, dim3(T < 2 * g_attn_sms ? T : 2 * g_attn_sms), dim3(kTcThreads), kTcSmem, st, p);
+    else tf_launch(sparse_attn_tcw_kernel, dim3(T < g_attn_sms ? T : g_attn_sms), dim3(kTwThreads), kTwSmem, st, p);
     return (int)cudaGetLastError();      // (sink, inverse rotation and the output rows are part of that kernel)
   } else if (Dh == 512 || Dh == 256) {
     const int smem = (kChunk * (Dh + 8) + Dh * (kChunk + 8)) * 2 + 4 * 16 * (kChunk + 4) * 4;

@@ -24,6 +24,8 @@
 #pragma once
 
 constexpr int kTwKeys = 64;
+constexpr int kTwProd = 8;                          // gather warps: four threads per key
+constexpr int kTwThreads = (kTwProd + 5) * 32;      // gather, 4 softmax / O^T, 1 MMA warp
 constexpr int kTwSub = 8192;                        // [64 rows x 128 B]: 64 dims of the keys, of Q, or the keys of P
 constexpr int kTwSubs = 8;                          // 512 dims
 constexpr int kTwStage = kTwSubs * kTwSub;
@@ -37,7 +39,7 @@ __device__ __forceinline__ uint64_t smem_desc_mn_w(uint32_t saddr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-__global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnParams p) {
+__global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnParams p) {
   tf_pdl_sync();
   constexpr int DH = 512;
   extern __shared__ uint8_t smem_raw[];
@@ -66,7 +68,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnPara
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(full(s), kTcProd);
+      tc::mbar_init(full(s), kTwProd);
       tc::mbar_init(empty(s), 1);
       tc::mbar_init(s_ready(s), 1);
       tc::mbar_init(s_free(s), 2);
@@ -75,12 +77,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnPara
     tc::mbar_init(p_ready, 4);
     tc::mbar_init(o_ready, 1);
     tc::mbar_init(o_free, 4);
-    tc::mbar_init(q_ready, kTcProd);
+    tc::mbar_init(q_ready, kTwProd);
     tc::mbar_init(q_free, 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
-  if (warp == kTcProd + 4) tc::tmem_alloc(tc::smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+  if (warp == kTwProd + 4) tc::tmem_alloc(tc::smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnPara
   const uint32_t tO = tmem_base + 128u;              // four blocks of 64 columns (heads), lane = dim of the block
   auto chunks_of = [&](int nkeys) { return max(1, (nkeys + kTwKeys - 1) / kTwKeys); };
 
-  if (warp < kTcProd) {
+  if (warp < kTwProd) {
     // ------------------------------------------------------------------ gather + convert
     const int key = threadIdx.x & (kTwKeys - 1), part = threadIdx.x >> 6;      // 128 dims of one key
     uint4 rawv[8];
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnPara
         const uint4* qsrc = reinterpret_cast<const uint4*>(p.q + (long)r * p.Hl * DH);
 #pragma unroll 4
         for (int j = 0; j < 16; ++j) {
-          const int piece = (int)threadIdx.x + kTcProd * 32 * j;
+          const int piece = (int)threadIdx.x + kTwProd * 32 * j;
           const int h = piece >> 6, c16 = piece & 63;           // 64 pieces per head row
           uint4 v = h < p.Hl ? qsrc[piece] : make_uint4(0u, 0u, 0u, 0u);
           uint32_t* vw = reinterpret_cast<uint32_t*>(&v);
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnPara
         if (lane == 0) tc::mbar_arrive(full(s));
       }
     }
-  } else if (warp == kTcProd + 4) {
+  } else if (warp == kTwProd + 4) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       constexpr uint32_t idesc_qk = tc::instr_desc(0, 0, 128, 64);
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnPara
     }
   } else {
     // ------------------------------------------------------------------ softmax (warps 8, 9), O^T (8-11)
-    const int quad = warp - kTcProd;
+    const int quad = warp - kTwProd;
     const bool sm = quad < 2;
     const int h = quad * 32 + lane;                   // head of a softmax thread
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
@@ -420,7 +422,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sparse_attn_tcw_kernel(AttnPara
   tc::tc_fence_before();
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) tf_report(p.st, TF_TIMEOUT, 151, blockIdx.x, 0);
-  if (warp == kTcProd + 4) {
+  if (warp == kTwProd + 4) {
     tc::tc_fence_after();
     tc::tmem_dealloc(tmem_base, 512);
   }
