@@ -624,9 +624,11 @@ TF_API int tf_sparse_attention(const void* q, int T, int Hl, int Dh, const int* 
       int dev = 0;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&g_attn_sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaFuncSetAttribute(sparse_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-      cudaFuncSetAttribute(sparse_attn_tcw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTwSmem);
     }
+    static unsigned long long limit_set[2] = {0, 0};
+    const cudaError_t e = Dh == 128 ? tf_smem_limit((const void*)sparse_attn_tc_kernel, kTcSmem, &limit_set[0])
+                                    : tf_smem_limit((const void*)sparse_attn_tcw_kernel, kTwSmem, &limit_set[1]);
+    if (e != cudaSuccess) return (int)e;
     if (Dh == 128) tf_launch(sparse_attn_tc_kernel, dim3(T < 2 * g_attn_sms ? T : 2 * g_attn_sms), dim3(kTcThreads), kTcSmem, st, p);
     else tf_launch(sparse_attn_tcw_kernel, dim3(T < g_attn_sms ? T : g_attn_sms), dim3(kTwThreads), kTwSmem, st, p);
     return (int)cudaGetLastError();      // (sink, inverse rotation and the output rows are part of that kernel)

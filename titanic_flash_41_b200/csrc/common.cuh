@@ -44,6 +44,19 @@ inline cudaError_t tf_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Raise a kernel's dynamic shared-memory limit once per device; `done` has one bit per device (thread-safe: setting
+// it twice is harmless).
+inline cudaError_t tf_smem_limit(const void* kernel, int bytes, unsigned long long* done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (__atomic_load_n(done, __ATOMIC_RELAXED) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) __atomic_fetch_or(done, bit, __ATOMIC_RELAXED);
+  return e;
+}
+
 // ---------------------------------------------------------------------------------------
 // Status words.  No kernel traps, asserts or spins without a limit: a kernel that meets a
 // bad argument or a wait that runs out records (code, detail) here and returns; the host

@@ -670,13 +670,9 @@ TF_API int tf_topk_select(const float* scores, int lds, const int* nvalid, int k
     tf_launch(topk_select_cluster_kernel<8, 16>, dim3(8, T), dim3(kSelThreads), 0, st, scores, lds, nvalid, k, out,
               count, out_scores, base);
   else if (lds <= kSelStage) {
-    static bool attr = false;
-    if (!attr) {
-      const cudaError_t e = cudaFuncSetAttribute(topk_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 kSelStage * 4);
-      if (e != cudaSuccess) return (int)e;
-      attr = true;
-    }
+    static unsigned long long limit_set = 0;
+    const cudaError_t e = tf_smem_limit((const void*)topk_select_kernel<true>, kSelStage * 4, &limit_set);
+    if (e != cudaSuccess) return (int)e;
     const int vec = lds % 4 == 0 && !(reinterpret_cast<uintptr_t>(scores) & 15);
     tf_launch(topk_select_kernel<true>, dim3(T), dim3(kSelRowThreads), (size_t)(lds + 3) / 4 * 16, st, scores, lds, nvalid, k,
               out, count, out_scores, base, vec);

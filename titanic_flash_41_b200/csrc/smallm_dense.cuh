@@ -216,12 +216,9 @@ cudaError_t launch_dense_mt(const DenseParams& p, int sms, cudaStream_t st) {
   constexpr int STAGES = MT <= 2 ? 3 : 5;
   constexpr int smem = kDenseWarps * STAGES * kDenseStage + kDenseWarps * 2 * MT * 512;
   auto kernel = smallm_dense_kernel<KIND, MT, DUAL, STAGES>;
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static unsigned long long limit_set = 0;
+  const cudaError_t e = tf_smem_limit((const void*)kernel, smem, &limit_set);
+  if (e != cudaSuccess) return e;
   const int resident = sms * (MT <= 2 ? 2 : 1);
   tf_launch(kernel, dim3(p.tiles < resident ? p.tiles : resident), dim3(kDenseWarps * 32), smem, st, p);
   return cudaGetLastError();

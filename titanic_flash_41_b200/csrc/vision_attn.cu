@@ -297,11 +297,8 @@ TF_API int tf_vis_attention(const void* q, const void* k, const void* v, void* o
       !tc::make_map_2d(&mk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, 64, 128, kTile) ||
       !tc::make_map_2d(&mv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, 64, 128, kTile))
     return -4;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(vis_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kVaSmem) != cudaSuccess) return -2;
-    attr = true;
-  }
+  static unsigned long long limit_set = 0;
+  if (tf_smem_limit((const void*)vis_attn_kernel, kVaSmem, &limit_set) != cudaSuccess) return -2;
   VisAttnParams p = {(__nv_bfloat16*)out, n, n_pad, ldo, scale * 1.4426950408889634f, (TfStatusWord*)status};
   tf_launch(vis_attn_kernel, dim3((n + kTile - 1) / kTile, heads), dim3(kVaThreads), kVaSmem, st, mq, mk, mv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
