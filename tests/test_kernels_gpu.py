@@ -892,3 +892,28 @@ def test_block_diagonal_gemv(M, G, R, K):
     for g in range(G):
         want = x[:, g * K:(g + 1) * K].double() @ E.dequant_fp8(ws[g]).double().t()
         assert float((out[:, g * R:(g + 1) * R].double() - want).norm() / want.norm()) < 2.0 ** -11 + 1e-5
+
+
+@pytest.mark.parametrize("T,d,k,shared", [(1, 128, 1, False), (3, 4096, 6, True), (5, 1280, 9, True), (2, 5120, 8, False)])
+def test_fused_boundary_row_form(T, d, k, shared):
+    """One piece a thread (narrow and full rows), more experts than are requested at once, and a width beyond it: residual
+    exact against fp32 sums in slot order, the normalised row one bf16 rounding (2^-8), its MXFP8 form exact."""
+    torch.manual_seed(d + k)
+    El = 5
+    x = torch.randn(T, d, device=DEV).bfloat16()
+    y, wts = torch.randn(T * k, d, device=DEV), torch.rand(T, k, device=DEV)
+    ids = torch.randint(0, 8, (T, k), dtype=torch.int32, device=DEV)
+    sh = torch.randn(T, d, device=DEV) if shared else None
+    w = (1 + 0.1 * torch.randn(d, device=DEV)).bfloat16()
+    h16, hb = torch.zeros(T, d, dtype=torch.float16, device=DEV), torch.zeros(T, d, dtype=torch.bfloat16, device=DEV)
+    x8, x8s = torch.zeros(T, d, dtype=torch.uint8, device=DEV), torch.zeros(T, d // 32, dtype=torch.uint8, device=DEV)
+    own = ((ids >= 2) & (ids < 2 + El)).float()[:, :, None]
+    sums = (y.view(T, k, d).double() * (wts[:, :, None] * own).double()).sum(1) + (sh.double() if shared else 0.0)
+    want_x = x.double() + sums
+    native.call("tf_add_norm_fused", x, None, y, ids, wts, sh, k, 2, 2 + El, w, h16, hb, x8, x8s, T, d, 1e-6)
+    assert ((x.double() - want_x).abs() <= 2.0 ** -8 * 1.01 * want_x.abs() + 1e-5).all()
+    want = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert ((hb.double() - want).abs() <= 2.0 ** -8 * 1.01 * want.abs() + 1e-30).all() and torch.equal(h16, hb.half())
+    q, s = torch.zeros_like(x8), torch.zeros_like(x8s)
+    native.call("tf_quant_rows_mx8", h16, d, q, s, T, d)
+    assert torch.equal(q, x8) and torch.equal(s, x8s)

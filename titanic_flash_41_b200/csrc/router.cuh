@@ -169,17 +169,14 @@ __device__ __forceinline__ void router_topk_rows_reg(const float* __restrict__ l
         }
       }
     }
+    // the largest key, then the lowest expert that has it: two warp reductions of integers (the key's order-preserving
+    // image; -0 counts as +0, as in a comparison of floats) instead of five rounds of two shuffles
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best[q], o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi[q], o);
-        if (ob > best[q] || (ob == best[q] && oi < bi[q])) {
-          best[q] = ob;
-          bi[q] = oi;
-        }
-      }
+    for (int q = 0; q < R; ++q) {
+      const uint32_t b = __float_as_uint(best[q] + 0.f);
+      const uint32_t key = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+      const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+      bi[q] = (int)__reduce_min_sync(0xffffffffu, key == top ? (uint32_t)bi[q] : 0x7fffffffu);
     }
 #pragma unroll
     for (int q = 0; q < R; ++q) {
