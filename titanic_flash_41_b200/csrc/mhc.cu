@@ -475,10 +475,12 @@ int launch_hc_cluster(HcArgs p, cudaStream_t st) {
     return 1;
   p.w = ((p.d + kHcCtas - 1) / kHcCtas + 7) / 8 * 8;
   // one row per cluster while that is one wave of two CTAs an SM (37 rows of eight CTAs); beyond it
-  // the sixteen-row form reads fn once for sixteen rows
-  const int R = p.rows <= 37 ? 1 : 16;
-  const size_t smem = (size_t)R * p.H * p.w * 2;
-  if (smem > 160 * 1024) return 1;
+  // the sixteen-row form reads fn once for sixteen rows (rows too wide for its slice stay at one)
+  constexpr size_t kMaxSlice = 160 * 1024;
+  const size_t slice = (size_t)p.H * p.w * 2;
+  const int R = p.rows <= 37 || 16 * slice > kMaxSlice ? 1 : 16;
+  const size_t smem = R * slice;
+  if (smem > kMaxSlice) return 1;
   auto kernel = R == 1 ? hc_cluster_kernel<1, HEAD> : hc_cluster_kernel<16, HEAD>;
   if (smem > 32 * 1024 &&
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
