@@ -117,10 +117,12 @@ def index():
     region = torch.zeros(T, dtype=torch.int32, device=DEV)
     nvalid = ((torch.arange(T, device=DEV) + 131072 - T + 1) // 4).int()
     scores = torch.zeros(T, C, device=DEV)
+    st = native.StatusWord(DEV)
     sel = torch.zeros(T, k, dtype=torch.int32, device=DEV)
     cnt = torch.zeros(T, dtype=torch.int32, device=DEV)
-    us = timed(lambda: native.call("tf_index_scores", q, w, region, nvalid, keys, C * krow, krow, T, Hi, Di, 32, scores, C, 0,
-                                   C), n=3, warm=1)
+    us = timed(lambda: native.call("tf_index_scores_rows", q, w, region, nvalid, keys, C * krow, krow, T, Hi, Di, 32, scores, C, 0,
+                                   C, st.t), n=3, warm=1)
+    st.check()
     print(f"index scores, {T} rows x {C} keys, {Hi} heads x {Di}: {us:.0f} us per launch, "
           f"{2.0 * T * C * Hi * Di / us / 1e6:.1f} TFLOP/s")
     us = timed(lambda: native.call("tf_topk_select", scores, C, nvalid, k, sel, cnt, None, 0, T), n=3, warm=1)

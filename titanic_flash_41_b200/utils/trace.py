@@ -149,7 +149,7 @@ class GraphClock:
 
 
 class Knockout(contextlib.AbstractContextManager):
-    """``with Knockout({"tf_index_scores", "tf_topk_select"}): ...`` skips those launches."""
+    """``with Knockout({"tf_index_scores_rows", "tf_topk_select"}): ...`` skips those launches."""
 
     def __init__(self, names: Iterable[str]):
         self.names, self._orig, self.skipped = set(names), None, 0
