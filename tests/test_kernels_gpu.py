@@ -326,6 +326,55 @@ def test_sparse_attention_of_prefill_rows_on_tcgen05_matches_reference(Hl):
     assert _rel(outs[0], outs[2]) < 1e-2 and torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("Dh", [128])
+@pytest.mark.parametrize("Hl,drift", [(64, 0.0), (64, 12.0), (33, 12.0), (1, 0.0)])
+def test_sparse_attention_of_more_rows_than_ctas_and_moving_maximum(Hl, drift, Dh):
+    """Three to seven query rows a CTA (two CTAs an SM at head dim 128, one at 512) with one to seven chunks each, rows without
+    any key among them, so that every barrier passes from row to row in both phases, and head counts that leave a softmax warp idle; ``drift`` makes later keys' scores grow by
+    hundreds, so that the reference maximum moves in some heads at every chunk and O and the sum are rescaled.
+
+    P is f16 (2^-11 relative), keys are exact in f16, the output is f16: within 1e-3 of fp64."""
+    from titanic_flash_41_b200.models.oracle import apply_rope
+    torch.manual_seed(31 + Hl)
+    T = 6 * torch.cuda.get_device_properties(0).multi_processor_count + 101
+    window, ring, C, k = 128, 512, 700, 320
+    win_row, comp_row = -(-(Dh + Dh // 32) // 16) * 16, -(-(Dh // 2 + Dh // 16) // 16) * 16
+    u = torch.randn(Dh) / Dh ** 0.5
+    win = torch.zeros(2, ring, win_row, dtype=torch.uint8)
+    win[:, :, :Dh + Dh // 32] = codecs.kv_v41_encode(torch.randn(2, ring, Dh) * 1.5)
+    comp = torch.zeros(2, C, comp_row, dtype=torch.uint8)
+    comp[:, :, :Dh // 2 + Dh // 16] = codecs.kv_v41fp4_encode(torch.randn(2, C, Dh) + drift * torch.arange(C)[:, None] / C * u * 8)
+    kvd, ckd = codecs.kv_v41_decode(win, Dh), codecs.kv_v41fp4_decode(comp, Dh)
+    pos, region = (torch.arange(T) * 7 % 400).int(), (torch.arange(T) % 2).int()
+    sel = torch.full((T, k), -1, dtype=torch.int32)
+    cnt = torch.tensor([[0, 1, 37, 128, 129, 255, 320][r % 7] for r in range(T)], dtype=torch.int32)
+    for r in range(T):
+        sel[r, :cnt[r]] = torch.sort(torch.randperm(C)[:cnt[r]]).values.int()
+    first = torch.where((cnt == 0) & (torch.arange(T) % 2 == 0), pos + 1, 0).int()         # (no window: no key at all)
+    q = (torch.randn(T, Hl, Dh) * 0.5 + (drift > 0) * 40 * u * (torch.arange(Hl) % 2)[None, :, None]).bfloat16()
+    sink = torch.randn(Hl) * 0.5
+    freqs = torch.tensor([10000.0 ** (-2.0 * j / 64) for j in range(32)])
+    dev = lambda t: t.to(DEV).contiguous()
+    st = native.StatusWord(DEV)
+    part = torch.zeros(1, device=DEV)                                  # (not read or written by this form)
+    out = torch.zeros(T, Hl * Dh, device=DEV, dtype=torch.float16)
+    native.call("tf_sparse_attention", dev(q), T, Hl, Dh, dev(pos), dev(region), dev(first), dev(win), ring * win_row, win_row,
+                ring, window, dev(comp), C * comp_row, comp_row, dev(sel), k, dev(cnt), C, 1 / math.sqrt(Dh), 1, part, part,
+                dev(sink), dev(freqs), 64, out, None, Hl * Dh, st.t)
+    st.check()
+    got = out.cpu().view(T, Hl, Dh).double()
+    for r in range(T):
+        p, rg = int(pos[r]), int(region[r])
+        if first[r] > p:
+            assert (got[r] == 0).all(), r
+            continue
+        nw = min(p + 1, window)
+        keys = torch.cat([kvd[rg, [(p - nw + 1 + i) % ring for i in range(nw)]], ckd[rg, sel[r, :int(cnt[r])].long()]]).double()
+        lg = torch.cat([q[r].double() @ keys.t() / math.sqrt(Dh), sink[:, None].double()], 1)
+        o = apply_rope((torch.softmax(lg, -1)[:, :-1] @ keys)[None].float(), torch.tensor([p]), freqs, inverse=True)[0]
+        assert _rel(got[r], o) < 1e-3, (r, _rel(got[r], o))
+
+
 def test_sampling_kernels():
     torch.manual_seed(7)
     V, rows = 5000, 4

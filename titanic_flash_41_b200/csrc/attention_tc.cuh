@@ -18,7 +18,8 @@
 // double-buffered took 2,540 cycles a chunk (388 us for 2,048 rows of 2,176 keys).  This form holds one Q, one
 // S (and P) and one O and two key tiles, 81 KB of shared memory and 256 tensor-memory columns: two CTAs share an SM,
 // and the chains of one row fill the waits of the other.  P as a tensor-memory operand takes a quarter of the
-// MMAs' shared-memory reads away: 360 us; with P in shared memory two CTAs gained nothing (383 us).
+// MMAs' shared-memory reads away; with P in shared memory two CTAs gained nothing.  370 us; the one-CTA form, whose
+// two softmax pairs need a P barrier per buffer to be sound, 400 - 412 us in the same run.
 //
 //   warps 0-3   gather: one thread per key of the chunk fetches its FP8 window row or FP4 compressed row (the next
 //               chunk's bytes are requested when this one has been converted; ids are decoded a chunk after
@@ -27,7 +28,7 @@
 //               rescaled only when a score exceeds it by 2^8), P as f16 over the columns of S that have
 //               been read; then the row: sink as an extra zero-valued logit, inverse
 //               rotation of the tail, f16 / bf16 output
-//   warp 6      one thread issues the MMAs: PV of chunk c, then QK of chunk c + 1 (in order: it overwrites S and P)
+//   warp 6      one thread issues the MMAs: PV of chunk c and, once that is done, QK of chunk c + 1 (it overwrites S and P)
 // Every mbarrier wait is bounded; on a time-out the CTA raises its abort flag, reports TF_TIMEOUT,
 // frees its tensor memory and returns.
 //
@@ -296,6 +297,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) sparse_attn_tc_kernel(AttnParam
       auto qk = [&](int i) -> bool {                                  // S = Q . Kt(stage i & 1)^T
         const int s = i & 1;
         if (!tc::mbar_wait(full(s), (i >> 1) & 1, abort_flag)) return false;
+        // S lies over the P that the PV before reads: MMAs with different accumulators are not ordered among
+        // themselves, so that PV has to be done, not only issued
+        if (i > 0 && !tc::mbar_wait(o_ready, (i & 1) ^ 1, abort_flag)) return false;
         tc::tc_fence_after();
 #pragma unroll
         for (int j = 0; j < 2; ++j)
@@ -374,7 +378,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) sparse_attn_tc_kernel(AttnParam
         if (c == 0) {
           m = cm;
         } else if (__any_sync(0xffffffffu, cm > m + 8.f)) {
-          // (QK of this chunk ran after the PV before: O is complete)
+          // (QK of this chunk was issued when the PV before was done: O is complete)
           const float nm = fmaxf(m, cm), f = exp2f(m - nm);
           m = nm;
           l *= f;
