@@ -326,7 +326,7 @@ def test_sparse_attention_of_prefill_rows_on_tcgen05_matches_reference(Hl):
     assert _rel(outs[0], outs[2]) < 1e-2 and torch.equal(outs[0], outs[1])
 
 
-@pytest.mark.parametrize("Dh", [128])
+@pytest.mark.parametrize("Dh", [128, 512])
 @pytest.mark.parametrize("Hl,drift", [(64, 0.0), (64, 12.0), (33, 12.0), (1, 0.0)])
 def test_sparse_attention_of_more_rows_than_ctas_and_moving_maximum(Hl, drift, Dh):
     """Three to seven query rows a CTA (two CTAs an SM at head dim 128, one at 512) with one to seven chunks each, rows without

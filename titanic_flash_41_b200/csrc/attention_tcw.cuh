@@ -17,8 +17,8 @@
 //               head through shared memory) and finish the row (neighbouring lanes hold a rotation pair)
 //   warp 12     one thread issues the MMAs: QK of chunk c + 1 before PV of chunk c
 //
-// Bound by shared memory: with N = 64 an MMA step reads 6 KB of operands for 16 cycles of math, 2,300 cycles a
-// chunk plus the gather's 64 KB of writes.  The mma.sync kernel dequantised every key once per
+// Bound by shared memory: with N = 64 an MMA step (128 x 64 x 16) reads 6 KB of operands, 48 cycles at 128 bytes a
+// cycle, for 32 cycles of math: 2,300 cycles a chunk, and the gather's 64 KB of writes beside them.  The mma.sync kernel dequantised every key once per
 // 16 heads and kept a transposed copy: 17.9 ms for 4,001 rows of 64 heads and up to 640 keys.
 // Every wait is bounded as in the narrow kernel.
 #pragma once
@@ -55,8 +55,10 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
   auto empty = [&](int s) { return bar0 + 8u * (2 + s); };      // PV done: stage free        (commit)
   auto s_ready = [&](int b) { return bar0 + 8u * (4 + b); };    // QK done                    (commit)
   auto s_free = [&](int b) { return bar0 + 8u * (6 + b); };     // softmax has read S         (2 warps)
-  auto p_free = [&](int b) { return bar0 + 8u * (8 + b); };     // the PV that read P[b] is done (commit)
-  const uint32_t p_ready = bar0 + 80, o_ready = bar0 + 88;      // P written, O rescaled (4 warps); PV done (commit)
+  // the PV that read P[b] is done (commit); O is complete up to that chunk.  (A single barrier for "PV done" would be
+  // ambiguous at the end of a row: while the PV before the last one still runs, the last one's parity is an older one's.)
+  auto p_free = [&](int b) { return bar0 + 8u * (8 + b); };
+  auto p_ready = [&](int b) { return bar0 + 8u * (10 + b); };   // P[b] written, O rescaled   (4 warps)
   const uint32_t o_free = bar0 + 96, q_ready = bar0 + 104, q_free = bar0 + 112;      // (4 warps), (8 warps), (commit)
   uint8_t* tail = st_g + 2 * kTwStage;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tail + 128);
@@ -72,10 +74,9 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
       tc::mbar_init(empty(s), 1);
       tc::mbar_init(s_ready(s), 1);
       tc::mbar_init(s_free(s), 2);
+      tc::mbar_init(p_ready(s), 4);
       tc::mbar_init(p_free(s), 1);
     }
-    tc::mbar_init(p_ready, 4);
-    tc::mbar_init(o_ready, 1);
     tc::mbar_init(o_free, 4);
     tc::mbar_init(q_ready, kTwProd);
     tc::mbar_init(q_free, 1);
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
             if (!(ok = qk(it + 1))) break;
             if (c + 2 == nchunks) tc::mma_commit(q_free);
           }
-          if (!(ok = tc::mbar_wait(p_ready, it & 1, abort_flag))) break;
+          if (!(ok = tc::mbar_wait(p_ready(it & 1), (it >> 1) & 1, abort_flag))) break;
           if (c == 0 && !(ok = tc::mbar_wait(o_free, (n_row & 1) ^ 1, abort_flag))) break;
           tc::tc_fence_after();
           const uint32_t kt = st_s + (it & 1) * kTwStage;
@@ -259,7 +260,6 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
                           (c | k) ? 1u : 0u);
           tc::mma_commit(empty(it & 1));
           tc::mma_commit(p_free(it & 1));
-          tc::mma_commit(o_ready);
         }
       }
     }
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
           }
           grp_bar();
           if (c > 0) {
-            wait(o_ready, (it & 1) ^ 1);
+            wait(p_free((it - 1) & 1), ((it - 1) >> 1) & 1);        // the PV of the chunk before
             tc::tc_fence_after();
 #pragma unroll 1
             for (int q = 0; q < 8; ++q) {
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
         __syncwarp();
         if (lane == 0) {
           if (sm) tc::mbar_arrive(s_free(sb));
-          tc::mbar_arrive(p_ready);
+          tc::mbar_arrive(p_ready(sb));
         }
       }
       // ---- the row: sink as one more zero-valued logit, inverse rotation of the tail, f16 / bf16 row
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
         fin[h] = scale_o;
       }
       grp_bar();
-      wait(o_ready, (it & 1) ^ 1);
+      wait(p_free((it - 1) & 1), ((it - 1) >> 1) & 1);              // the row's last PV
       tc::tc_fence_after();
       const int tail0 = DH - p.rope_dim, odd = lane & 1;
 #pragma unroll 1
