@@ -1,5 +1,6 @@
 """Image input planning / patchify (CPU) and the device vision tower against its fp32 oracle (GPU)."""
 import io
+import math
 
 import numpy as np
 import pytest
@@ -131,3 +132,79 @@ def test_dense_attention_kernel(n, heads, spread):
     err = (out[:n].view(n, heads, 64).double() - want).abs()
     assert (err <= 2.0 ** -8 * 1.01 * (mag + want.abs()) + 1e-5).all(), float((err / (mag + want.abs())).max())
     assert (out[n] == 5.0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,width,off", [(3, 64, 1), (5, 72, 0), (5, 72, 3), (2, 1024, 5), (4, 77, 0), (1, 1, 0), (3, 1100, 1)])
+def test_glue_kernels_on_and_off_the_vector_grain(n, width, off):
+    """Eight elements an access, and the one-element form for widths off eight and for operands that start ``off`` elements
+    behind a 16-byte boundary (a view into a larger tensor): stored values against fp64 of the same bf16 inputs.
+
+    Sums and products of bf16 in fp32, one rounding to bf16 (2^-8 relative at most) each; an input that lies within fp32
+    error of a rounding boundary may go either way, so that a chain of two roundings may differ by one more step."""
+    from titanic_flash_41_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(width + off)
+
+    def bf(*shape, fill=None):
+        flat = torch.zeros(math.prod(shape) + off, dtype=torch.bfloat16, device="cuda")
+        t = flat[off:].view(*shape)
+        return t.copy_(torch.randn(*shape, generator=g, device="cuda") if fill is None else torch.full(shape, fill))
+
+    def close(got, want, steps=1):
+        return bool(((got.double() - want).abs() <= steps * 2.0 ** -8 * 1.01 * want.abs() + 1e-30).all())
+    rnd = lambda t: t.bfloat16().double()
+    x, delta, bias, w = bf(n, width), bf(n, width), bf(width), bf(width)
+    d = lambda t: t.double()
+    y = bf(n, width, fill=9.0)
+    native.call("tf_vis_bias", x, bias, y, x.numel(), width)
+    assert torch.equal(y, (x.float() + bias.float()).bfloat16())
+    native.call("tf_vis_gelu", x, bias, y, x.numel(), width)
+    v = rnd(x.float() + bias.float())
+    assert bool(((d(y) - 0.5 * v * (1 + torch.erf(v * 0.5 ** 0.5))).abs() <= 2.0 ** -8 * 1.01 * d(y).abs() + 1e-6 * (1 + v.abs())).all())
+    res = (x.float() + (delta.float() + bias.float()).bfloat16().float()).bfloat16()
+    native.call("tf_vis_norm", x, delta, bias, w, y, n, width, 1e-6)
+    assert torch.equal(x, res)
+    assert close(y, d(res) * torch.rsqrt(d(res).pow(2).mean(-1, keepdim=True) + 1e-6) * d(w))
+    gu = bf(n, 2 * width)
+    native.call("tf_vis_swiglu", gu, y, n, width)
+    assert close(y, rnd((d(gu[:, :width]) * torch.sigmoid(d(gu[:, :width]))).float()) * d(gu[:, width:]), steps=2)
+    start, newline, end = bf(width), bf(width), bf(width)
+    f, out = bf(2 * 3, width), bf(2 * 4 + 2, width, fill=9.0)
+    native.call("tf_vis_span", f, bias, start, newline, end, out, 3, 10, width)
+    fb = (f.float() + bias.float()).bfloat16()
+    assert torch.equal(out, torch.cat([start[None], fb[:3], newline[None], fb[3:], newline[None], end[None]]))
+    heads, n_pad = 2, n + 2
+    qkv, qb = bf(n, 3 * heads * 64), bf(3 * heads * 64)
+    q, k, vv = (bf(heads, n_pad, 64, fill=9.0) for _ in range(3))
+    native.call("tf_vis_rope_split", qkv, qb, q, k, vv, n, n_pad, 2, heads)
+    parts = (qkv.float() + qb.float()).bfloat16().view(n, 3, heads, 64)
+    c = torch.arange(32, device="cuda")
+    row = torch.arange(n, device="cuda")[:, None]
+    ang = (torch.where(c < 16, row // 2, row % 2).double() * 10000.0 ** (-(c % 16).double() / 16))[:, None, :]
+    for got, part in ((q, 0), (k, 1)):
+        a, b = d(parts[:, part, :, :32]), d(parts[:, part, :, 32:])
+        want = torch.cat([a * ang.cos() - b * ang.sin(), b * ang.cos() + a * ang.sin()], -1).transpose(0, 1)
+        assert bool(((d(got[:, :n]) - want).abs() <= 2.0 ** -8 * 1.01 * want.abs() + 1e-5).all()) and bool((got[:, n:] == 0).all())
+    assert torch.equal(vv[:, :n], parts[:, 2].transpose(0, 1)) and bool((vv[:, n:] == 0).all())
+
+
+@pytest.mark.gpu
+def test_tower_with_weights_off_the_vector_grain():
+    """Norm weights and biases on the device as views into one flat tensor (the tower keeps them as they are): the span
+    follows the fp32 definition as with tensors of their own (the bound of the other tower test)."""
+    from titanic_flash_41_b200.config import VisionConfig
+    from titanic_flash_41_b200.models import vision as V
+    vc, d_model, gh, gw = VisionConfig(layers=2, hidden=128, intermediate=256), 256, 8, 11
+    W = {k: v.bfloat16().float() for k, v in V.init_vision_weights(vc, d_model, 3).items()}
+    flat, at, dev = torch.zeros(sum(v.numel() + 1 for v in W.values()), dtype=torch.bfloat16, device="cuda"), 0, dict(W)
+    for k, v in W.items():
+        if v.dim() == 1:
+            at += 1 if at % 2 == 0 else 2                   # an odd element: off the 16-byte (and the 4-byte) grain
+            dev[k] = flat[at:at + v.numel()].copy_(v)
+            at += v.numel()
+    patches = (torch.rand(gh * gw, 588, generator=torch.Generator().manual_seed(1)) * 2 - 1).bfloat16()
+    want = V.VisionOracle(vc, d_model, W).encode(patches.float(), gh, gw)
+    tower = V.VisionTower(vc, d_model, dev)
+    assert any(t.data_ptr() % 4 for t in tower.W.values())
+    got = tower.encode(patches, gh, gw).float().cpu()
+    assert float((got - want).norm() / want.norm()) < 0.03

@@ -15,101 +15,118 @@
 namespace {
 typedef __nv_bfloat16 B;
 
-// All of these move rows between GEMMs and are bound by memory: eight bf16 per thread and access (widths
-// are multiples of 8, rows 16-byte aligned), and the bias of a projection is added (and rounded, as a
-// separate pass would) by the kernel that reads its rows next.  One element per thread and a pass per
-// bias: 3.3 ms of an eight-layer encoding of 8,580 patches.
-struct V8 {
-  float f[8];
+// All of these move rows between GEMMs and are bound by memory: eight bf16 per thread and access (V = 8), and the
+// bias of a projection is added (and rounded, as a separate pass would) by the kernel that reads its rows next.
+// One element per thread and a pass per bias: 3.3 ms of an eight-layer encoding of 8,580 patches.  V = 1 is the
+// form for widths that eight does not divide and for operands off the 16-byte grain (a weight that is a
+// view into a larger tensor): an access of eight would fault there.
+template <int V>
+struct Vec {
+  float f[V];
 };
-__device__ __forceinline__ V8 ld8(const B* p) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  V8 v;
+template <int V>
+__device__ __forceinline__ Vec<V> ld(const B* p) {
+  Vec<V> v;
+  if constexpr (V == 8) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(p);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 f = __bfloat1622float2(h[j]);
-    v.f[2 * j] = f.x;
-    v.f[2 * j + 1] = f.y;
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(h[j]);
+      v.f[2 * j] = f.x;
+      v.f[2 * j + 1] = f.y;
+    }
+  } else {
+    v.f[0] = __bfloat162float(*p);
   }
   return v;
 }
-__device__ __forceinline__ void st8(B* p, const V8& v) {
-  __nv_bfloat162 h[4];
+template <int V>
+__device__ __forceinline__ void st(B* p, const Vec<V>& v) {
+  if constexpr (V == 8) {
+    __nv_bfloat162 h[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v.f[2 * j], v.f[2 * j + 1]);
-  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<uint4*>(h);
+    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v.f[2 * j], v.f[2 * j + 1]);
+    *reinterpret_cast<uint4*>(p) = *reinterpret_cast<uint4*>(h);
+  } else {
+    *p = __float2bfloat16_rn(v.f[0]);
+  }
 }
 // x + bias, rounded to bf16; without a bias x as it is
-__device__ __forceinline__ V8 ld8_bias(const B* p, const B* bias) {
-  V8 v = ld8(p);
+template <int V>
+__device__ __forceinline__ Vec<V> ld_bias(const B* p, const B* bias) {
+  Vec<V> v = ld<V>(p);
   if (bias) {
-    const V8 b = ld8(bias);
+    const Vec<V> b = ld<V>(bias);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v.f[j] = bf16_round(v.f[j] + b.f[j]);
+    for (int j = 0; j < V; ++j) v.f[j] = bf16_round(v.f[j] + b.f[j]);
   }
   return v;
 }
 
+template <int V>
 __global__ void __launch_bounds__(256) vis_bias_kernel(const B* x, const B* bias, B* y, long count, int width) {
   tf_pdl_sync();
-  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (i < count) st8(y + i, ld8_bias(x + i, bias + i % width));
+  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (i < count) st<V>(y + i, ld_bias<V>(x + i, bias + i % width));
 }
 
 // x += delta (+ the bias of the projection that made delta); y = rmsnorm(x) * w
+template <int V>
 __global__ void __launch_bounds__(128) vis_norm_kernel(B* x, const B* delta, const B* bias, const B* w, B* y, int width,
                                                        float eps) {
   tf_pdl_sync();
   __shared__ float red[4];
   const long row = blockIdx.x * (long)width;
   float s = 0.f;
-  for (int c = threadIdx.x * 8; c < width; c += 1024) {
-    V8 v = ld8(x + row + c);
+  for (int c = threadIdx.x * V; c < width; c += 128 * V) {
+    Vec<V> v = ld<V>(x + row + c);
     if (delta) {
-      const V8 d = ld8_bias(delta + row + c, bias ? bias + c : nullptr);
+      const Vec<V> d = ld_bias<V>(delta + row + c, bias ? bias + c : nullptr);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v.f[j] = bf16_round(v.f[j] + d.f[j]);
-      st8(x + row + c, v);
+      for (int j = 0; j < V; ++j) v.f[j] = bf16_round(v.f[j] + d.f[j]);
+      st<V>(x + row + c, v);
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s += v.f[j] * v.f[j];
+    for (int j = 0; j < V; ++j) s += v.f[j] * v.f[j];
   }
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   const float inv = rsqrtf((red[0] + red[1] + red[2] + red[3]) / width + eps);
-  for (int c = threadIdx.x * 8; c < width; c += 1024) {      // (a thread reads back what it wrote)
-    V8 v = ld8(x + row + c);
-    const V8 g = ld8(w + c);
+  for (int c = threadIdx.x * V; c < width; c += 128 * V) {      // (a thread reads back what it wrote)
+    Vec<V> v = ld<V>(x + row + c);
+    const Vec<V> g = ld<V>(w + c);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v.f[j] = v.f[j] * inv * g.f[j];
-    st8(y + row + c, v);
+    for (int j = 0; j < V; ++j) v.f[j] = v.f[j] * inv * g.f[j];
+    st<V>(y + row + c, v);
   }
 }
 
-// q, k, v: [heads][n_pad][64]; rows n .. n_pad - 1 become zeros.  A thread turns pairs 8 g .. 8 g + 7 of one head.
+// q, k, v: [heads][n_pad][64]; rows n .. n_pad - 1 become zeros.  A thread turns pairs g .. g + V - 1 of one head.
+template <int V>
 __global__ void __launch_bounds__(256) vis_rope_split_kernel(const B* qkv, const B* bias, B* q, B* k, B* v, int n,
                                                              int n_pad, int grid_w, int heads) {
   tf_pdl_sync();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)n_pad * heads * 4) return;
-  const int width = heads * 64, g = (int)(i & 3) * 8, head = (int)(i >> 2) % heads, row = (int)((i >> 2) / heads);
+  constexpr int kPer = 32 / V;                      // threads per head and row
+  if (i >= (long)n_pad * heads * kPer) return;
+  const int width = heads * 64, g = (int)(i % kPer) * V, head = (int)(i / kPer % heads), row = (int)(i / kPer / heads);
   const long dst = ((long)head * n_pad + row) * 64 + g;
   if (row >= n) {
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    const Vec<V> z = {};
 #pragma unroll
     for (int h = 0; h < 64; h += 32) {
-      *reinterpret_cast<uint4*>(q + dst + h) = z;
-      *reinterpret_cast<uint4*>(k + dst + h) = z;
-      *reinterpret_cast<uint4*>(v + dst + h) = z;
+      st<V>(q + dst + h, z);
+      st<V>(k + dst + h, z);
+      st<V>(v + dst + h, z);
     }
     return;
   }
-  float sn[8], cs[8];
+  float sn[V], cs[V];
   const float pos = (float)(g < 16 ? row / grid_w : row % grid_w);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < V; ++j) {
     const float freq = 1.f / powf(10000.f, (float)((g + j) % 16) / 16.f);
     sincosf(pos * freq, &sn[j], &cs[j]);
   }
@@ -117,33 +134,34 @@ __global__ void __launch_bounds__(256) vis_rope_split_kernel(const B* qkv, const
   const B* src = qkv + (long)row * 3 * width + col;
 #pragma unroll
   for (int part = 0; part < 2; ++part) {
-    const V8 a = ld8_bias(src + part * width, bias + part * width + col);
-    const V8 b = ld8_bias(src + part * width + 32, bias + part * width + col + 32);
-    V8 o1, o2;
+    const Vec<V> a = ld_bias<V>(src + part * width, bias + part * width + col);
+    const Vec<V> b = ld_bias<V>(src + part * width + 32, bias + part * width + col + 32);
+    Vec<V> o1, o2;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < V; ++j) {
       o1.f[j] = a.f[j] * cs[j] - b.f[j] * sn[j];
       o2.f[j] = b.f[j] * cs[j] + a.f[j] * sn[j];
     }
     B* out = part ? k : q;
-    st8(out + dst, o1);
-    st8(out + dst + 32, o2);
+    st<V>(out + dst, o1);
+    st<V>(out + dst + 32, o2);
   }
-  st8(v + dst, ld8_bias(src + 2 * width, bias + 2 * width + col));
-  st8(v + dst + 32, ld8_bias(src + 2 * width + 32, bias + 2 * width + col + 32));
+  st<V>(v + dst, ld_bias<V>(src + 2 * width, bias + 2 * width + col));
+  st<V>(v + dst + 32, ld_bias<V>(src + 2 * width + 32, bias + 2 * width + col + 32));
 }
 
+template <int V>
 __global__ void __launch_bounds__(256) vis_swiglu_kernel(const B* gu, B* y, long count, int inter) {
   tf_pdl_sync();
-  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (i >= count) return;
   const long row = i / inter;
   const int c = (int)(i - row * inter);
-  V8 g = ld8(gu + row * 2 * inter + c);
-  const V8 u = ld8(gu + row * 2 * inter + inter + c);
+  Vec<V> g = ld<V>(gu + row * 2 * inter + c);
+  const Vec<V> u = ld<V>(gu + row * 2 * inter + inter + c);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) g.f[j] = bf16_round(g.f[j] / (1.f + expf(-g.f[j]))) * u.f[j];
-  st8(y + i, g);
+  for (int j = 0; j < V; ++j) g.f[j] = bf16_round(g.f[j] / (1.f + expf(-g.f[j]))) * u.f[j];
+  st<V>(y + i, g);
 }
 
 __global__ void vis_unfold_kernel(const B* x, B* y, int h, int w, int width, long count) {
@@ -156,59 +174,68 @@ __global__ void vis_unfold_kernel(const B* x, B* y, int h, int w, int width, lon
   y[i] = (sy < h && sx < w) ? x[((long)sy * w + sx) * width + col / 9] : __float2bfloat16_rn(0.f);
 }
 
+template <int V>
 __global__ void __launch_bounds__(256) vis_gelu_kernel(const B* x, const B* bias, B* y, long count, int width) {
   tf_pdl_sync();
-  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (i >= count) return;
-  V8 v = ld8_bias(x + i, bias + i % width);
+  Vec<V> v = ld_bias<V>(x + i, bias + i % width);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) v.f[j] = (v.f[j] * 0.5f) * (1.f + erff(v.f[j] * 0.70710678118654752440f));
-  st8(y + i, v);
+  for (int j = 0; j < V; ++j) v.f[j] = (v.f[j] * 0.5f) * (1.f + erff(v.f[j] * 0.70710678118654752440f));
+  st<V>(y + i, v);
 }
 
+template <int V>
 __global__ void __launch_bounds__(256) vis_span_kernel(const B* f, const B* bias, const B* start, const B* newline,
                                                        const B* end, B* out, int width, int tokens, int d) {
   tf_pdl_sync();
-  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (i >= (long)tokens * d) return;
   const int row = (int)(i / d), col = (int)(i % d);
-  V8 v;
-  if (row == 0) v = ld8(start + col);
-  else if (row + 1 == tokens) v = ld8(end + col);
+  Vec<V> v;
+  if (row == 0) v = ld<V>(start + col);
+  else if (row + 1 == tokens) v = ld<V>(end + col);
   else {
     const int r = row - 1, x = r % (width + 1), y = r / (width + 1);
-    v = x == width ? ld8(newline + col) : ld8_bias(f + ((long)y * width + x) * d + col, bias + col);
+    v = x == width ? ld<V>(newline + col) : ld_bias<V>(f + ((long)y * width + x) * d + col, bias + col);
   }
-  st8(out + i, v);
+  st<V>(out + i, v);
 }
 
 inline unsigned blocks(long n) { return (unsigned)((n + 255) / 256); }
+// elements per access: eight when every row is a multiple of eight and every pointer on the 16-byte grain, else one
+template <typename... P>
+int grain(long width, P... ptr) {
+  return width % 8 == 0 && !((0 | ... | reinterpret_cast<uintptr_t>(ptr)) & 15) ? 8 : 1;
+}
 }  // namespace
 
 TF_API int tf_vis_bias(const void* x, const void* bias, void* y, long count, int width, cudaStream_t st) {
-  if (width % 8) return -1;
-  tf_launch(vis_bias_kernel, dim3(blocks(count / 8)), dim3(256), 0, st, (const B*)x, (const B*)bias, (B*)y, count, width);
+  const int V = grain(width | count, x, bias, y);
+  tf_launch(V == 8 ? vis_bias_kernel<8> : vis_bias_kernel<1>, dim3(blocks(count / V)), dim3(256), 0, st, (const B*)x,
+            (const B*)bias, (B*)y, count, width);
   return (int)cudaGetLastError();
 }
 // x [rows, width] += delta (optional; with its projection's bias, optional); y = rmsnorm(x) * w
 TF_API int tf_vis_norm(void* x, const void* delta, const void* bias, const void* w, void* y, int rows, int width, float eps,
                        cudaStream_t st) {
-  if (width % 8) return -1;
-  tf_launch(vis_norm_kernel, dim3(rows), dim3(128), 0, st, (B*)x, (const B*)delta, (const B*)bias, (const B*)w, (B*)y,
-            width, eps);
+  tf_launch(grain(width, x, delta, bias, w, y) == 8 ? vis_norm_kernel<8> : vis_norm_kernel<1>, dim3(rows), dim3(128), 0, st,
+            (B*)x, (const B*)delta, (const B*)bias, (const B*)w, (B*)y, width, eps);
   return (int)cudaGetLastError();
 }
 // qkv [n, 3 * heads * 64] and its bias -> q, k, v [heads][n_pad][64], rows n .. zero
 TF_API int tf_vis_rope_split(const void* qkv, const void* bias, void* q, void* k, void* v, int n, int n_pad, int grid_w,
                              int heads, cudaStream_t st) {
   if (n > n_pad || !bias) return -1;
-  tf_launch(vis_rope_split_kernel, dim3(blocks((long)n_pad * heads * 4)), dim3(256), 0, st, (const B*)qkv, (const B*)bias,
-            (B*)q, (B*)k, (B*)v, n, n_pad, grid_w, heads);
+  const int V = grain(64, qkv, bias, q, k, v);
+  tf_launch(V == 8 ? vis_rope_split_kernel<8> : vis_rope_split_kernel<1>, dim3(blocks((long)n_pad * heads * (32 / V))),
+            dim3(256), 0, st, (const B*)qkv, (const B*)bias, (B*)q, (B*)k, (B*)v, n, n_pad, grid_w, heads);
   return (int)cudaGetLastError();
 }
 TF_API int tf_vis_swiglu(const void* gu, void* y, long rows, int inter, cudaStream_t st) {
-  if (inter % 8) return -1;
-  tf_launch(vis_swiglu_kernel, dim3(blocks(rows * inter / 8)), dim3(256), 0, st, (const B*)gu, (B*)y, rows * inter, inter);
+  const int V = grain(inter, gu, y);
+  tf_launch(V == 8 ? vis_swiglu_kernel<8> : vis_swiglu_kernel<1>, dim3(blocks(rows * inter / V)), dim3(256), 0, st,
+            (const B*)gu, (B*)y, rows * inter, inter);
   return (int)cudaGetLastError();
 }
 TF_API int tf_vis_unfold(const void* x, void* y, int h, int w, int width, cudaStream_t st) {
@@ -217,14 +244,15 @@ TF_API int tf_vis_unfold(const void* x, void* y, int h, int w, int width, cudaSt
   return (int)cudaGetLastError();
 }
 TF_API int tf_vis_gelu(const void* x, const void* bias, void* y, long count, int width, cudaStream_t st) {
-  if (width % 8) return -1;
-  tf_launch(vis_gelu_kernel, dim3(blocks(count / 8)), dim3(256), 0, st, (const B*)x, (const B*)bias, (B*)y, count, width);
+  const int V = grain(width | count, x, bias, y);
+  tf_launch(V == 8 ? vis_gelu_kernel<8> : vis_gelu_kernel<1>, dim3(blocks(count / V)), dim3(256), 0, st, (const B*)x,
+            (const B*)bias, (B*)y, count, width);
   return (int)cudaGetLastError();
 }
 TF_API int tf_vis_span(const void* f, const void* bias, const void* start, const void* newline, const void* end, void* out,
                        int width, int tokens, int d, cudaStream_t st) {
-  if (d % 8) return -1;
-  tf_launch(vis_span_kernel, dim3(blocks((long)tokens * d / 8)), dim3(256), 0, st, (const B*)f, (const B*)bias,
-            (const B*)start, (const B*)newline, (const B*)end, (B*)out, width, tokens, d);
+  const int V = grain(d, f, bias, start, newline, end, out);
+  tf_launch(V == 8 ? vis_span_kernel<8> : vis_span_kernel<1>, dim3(blocks((long)tokens * d / V)), dim3(256), 0, st,
+            (const B*)f, (const B*)bias, (const B*)start, (const B*)newline, (const B*)end, (B*)out, width, tokens, d);
   return (int)cudaGetLastError();
 }
