@@ -78,3 +78,39 @@ def test_prepare_post_and_head_over_both_forms(T, H, d):
     hvb = hv.double().cpu()
     want = hvb * torch.rsqrt(hvb.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double()
     assert bf16_close(hbf, want) and torch.equal(hh, hbf.half())
+
+
+def test_boundaries_of_two_widths_from_several_threads():
+    """Host threads with streams of their own, sixteen-row clusters of 82 KB in one half and of 164 KB in the other, launched
+    back to back: a limit set to the bytes of each launch would be lowered by one thread between another's set and launch."""
+    import threading
+    from titanic_flash_41_b200.ops import native
+    from titanic_flash_41_b200.ops.mhc import HcBoundary
+    H, rows, errors = 4, 40, []
+    lib = native.lib()
+    start = threading.Barrier(8)
+
+    def work(d, seed):
+        try:
+            g = torch.Generator(device="cuda").manual_seed(seed)
+            x = torch.randn(rows, H, d, generator=g, device="cuda").bfloat16()
+            fn = torch.randn(H * (2 + H), H * d, generator=g, device="cuda") * 0.05
+            hb = HcBoundary(fn, torch.zeros(H * (2 + H), device="cuda"), torch.ones(3, device="cuda"), H, d)
+            first, v = hb.prepare(x)[0], torch.empty(rows, d, dtype=torch.bfloat16, device="cuda")
+            stream = torch.cuda.Stream()
+            torch.cuda.synchronize()
+            start.wait()
+            args = [x.data_ptr(), hb.fn.data_ptr(), hb.base.data_ptr(), hb.scale.data_ptr(), hb._coef.data_ptr(), v.data_ptr(),
+                    None, None, None, rows, H, d, 1, 1e-6, 1e-6, stream.cuda_stream]
+            refused = sum(lib.tf_hc_prepare(*args) != 0 for _ in range(4000))
+            torch.cuda.synchronize()
+            errors.append((refused, bool(torch.equal(v, first))))
+        except Exception as e:
+            errors.append(repr(e))
+    torch.zeros(1, device="cuda")
+    threads = [threading.Thread(target=work, args=((5120, 10240)[i % 2], i)) for i in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert errors == [(0, True)] * 8

@@ -467,26 +467,30 @@ __global__ void __launch_bounds__(128) hc_post_vec_kernel(const __nv_bfloat16* _
 
 inline bool aligned16(const void* a) { return !(reinterpret_cast<uintptr_t>(a) & 15); }
 
-// 0: launched, 1: these rows need the general kernel (width or an address off the vector grain, or too wide)
+constexpr int kHcGeneral = -100;
+// 0 or a CUDA error: launched; kHcGeneral: these rows need the general kernel (width or an address off the vector
+// grain, or too wide)
 template <bool HEAD>
 int launch_hc_cluster(HcArgs p, cudaStream_t st) {
   if (p.d % 8 || !aligned16(p.x) || !aligned16(p.fn) || !aligned16(p.v) || !aligned16(p.mean) || !aligned16(p.norm_w) ||
       !aligned16(p.h16) || !aligned16(p.hb))
-    return 1;
+    return kHcGeneral;
   p.w = ((p.d + kHcCtas - 1) / kHcCtas + 7) / 8 * 8;
   // one row per cluster while that is one wave of two CTAs an SM (37 rows of eight CTAs); beyond it
   // the sixteen-row form reads fn once for sixteen rows (rows too wide for its slice stay at one)
-  constexpr size_t kMaxSlice = 160 * 1024;
+  constexpr int kMaxSlice = 160 * 1024;
   const size_t slice = (size_t)p.H * p.w * 2;
   const int R = p.rows <= 37 || 16 * slice > kMaxSlice ? 1 : 16;
   const size_t smem = R * slice;
-  if (smem > kMaxSlice) return 1;
+  if (smem > kMaxSlice) return kHcGeneral;
   auto kernel = R == 1 ? hc_cluster_kernel<1, HEAD> : hc_cluster_kernel<16, HEAD>;
-  if (smem > 32 * 1024 &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return 1;
+  // the limit of any width, once: set to the bytes of each launch, a narrower engine of another thread could lower it
+  // between this thread's set and its launch
+  static unsigned long long limit_set[2] = {0, 0};
+  const cudaError_t e = tf_smem_limit((const void*)kernel, kMaxSlice, &limit_set[R == 1]);
+  if (e != cudaSuccess) return (int)e;
   tf_launch(kernel, dim3((p.rows + R - 1) / R * kHcCtas), dim3(256), smem, st, p);
-  return 0;
+  return (int)cudaGetLastError();
 }
 }  // namespace
 
@@ -501,7 +505,8 @@ TF_API int tf_hc_prepare(const void* x, const float* fn, const float* base, cons
   if (rows <= 0) return 0;
   HcArgs p = {(const __nv_bfloat16*)x, fn, base, scale, (HcCoef*)coef, (__nv_bfloat16*)v, nullptr,
               (const __nv_bfloat16*)norm_w, (__half*)h16, (__nv_bfloat16*)hb, rows, H, d, 0, iters, eps, rms_eps};
-  if (launch_hc_cluster<false>(p, st) == 0) return (int)cudaGetLastError();
+  const int c = launch_hc_cluster<false>(p, st);
+  if (c != kHcGeneral) return c;
   tf_launch(hc_prepare_kernel, dim3(rows), dim3(256), 0, st, (const __nv_bfloat16*)x, fn, base, scale, (HcCoef*)coef, (__nv_bfloat16*)v,
                                           (const __nv_bfloat16*)norm_w, (__half*)h16, (__nv_bfloat16*)hb, H, d, iters,
                                           eps, rms_eps);
@@ -519,8 +524,8 @@ TF_API int tf_hc_head(const void* x, const float* fn, const float* base, const f
   if (rows <= 0) return 0;
   HcArgs p = {(const __nv_bfloat16*)x, fn, base, scale, nullptr, (__nv_bfloat16*)v, (__nv_bfloat16*)mean,
               (const __nv_bfloat16*)norm_w, (__half*)h16, (__nv_bfloat16*)hb, rows, H, d, 0, 0, eps, rms_eps};
-  if (launch_hc_cluster<true>(p, st) != 0) return -1;
-  return (int)cudaGetLastError();
+  const int c = launch_hc_cluster<true>(p, st);
+  return c == kHcGeneral ? -1 : c;
 }
 
 // y [rows, H, d] bf16 = post * a + comb^T x with a [rows, d] f32 (the reduced sublayer output)
