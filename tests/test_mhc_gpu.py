@@ -114,3 +114,30 @@ def test_boundaries_of_two_widths_from_several_threads():
     for t in threads:
         t.join()
     assert errors == [(0, True)] * 8
+
+
+@pytest.mark.parametrize("T,H,d,off", [(3, 4, 100, 0), (1, 3, 41, 0), (40, 2, 1028, 0), (5, 4, 512, 1), (2, 4, 128, 3)])
+def test_head_collapse_of_any_width_and_alignment(T, H, d, off):
+    """Widths that eight does not divide and weights that start ``off`` floats behind a 16-byte boundary (the general
+    kernel), against fp64; mixes and bounds as in the test of the cluster forms."""
+    from titanic_flash_41_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(T * d)
+    x = torch.randn(T, H, d, generator=g, device="cuda").bfloat16()
+    fn = torch.zeros(H * H * d + off, device="cuda")[off:].view(H, H * d).copy_(torch.randn(H, H * d, generator=g, device="cuda") * 0.05)
+    base, scale = torch.randn(H, generator=g, device="cuda") * 0.3, torch.full((1,), 0.7, device="cuda")
+    nw = (1 + 0.1 * torch.randn(d, generator=g, device="cuda")).bfloat16()
+    v, mean, hb = (torch.zeros(T, d, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    h16 = torch.zeros(T, d, dtype=torch.float16, device="cuda")
+    native.call("tf_hc_head", x, fn, base, scale, v, mean, nw, h16, hb, T, H, d, 1e-6, 1e-6)
+    flat = x.double().reshape(T, -1)
+    pre = torch.sigmoid(flat @ fn.double().t() * torch.rsqrt(flat.pow(2).mean(-1, keepdim=True) + 1e-6) * 0.7 + base.double()) + 1e-6
+
+    def bf16_close(got, want):                  # one bf16 rounding, plus the coefficients' 2e-4
+        return bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-3).all())
+    assert bf16_close(v, (x.double() * pre[:, :, None]).sum(1)) and bf16_close(mean, x.double().mean(1))
+    vd = v.double()
+    want = vd * torch.rsqrt(vd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    assert bf16_close(hb, want) and torch.equal(h16, hb.half())
+    v2 = torch.zeros_like(v)
+    native.call("tf_hc_head", x, fn, base, scale, v2, None, None, None, None, T, H, d, 1e-6, 1e-6)      # without mean and norm
+    assert torch.equal(v, v2)

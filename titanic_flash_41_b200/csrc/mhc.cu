@@ -24,11 +24,15 @@ struct HcCoef {                                    // per row, 32 floats
   float pre[kMaxH], post[kMaxH], comb[kMaxH * kMaxH], pad[8];
 };
 
+// One CTA per row, any width and alignment.  HEAD: the collapse in front of the vocabulary head (H mixes, no post / comb,
+// bf16 values in both normalised rows) and the plain mean of the copies.
+template <bool HEAD>
 __global__ void __launch_bounds__(256) hc_prepare_kernel(const __nv_bfloat16* __restrict__ x,
                                                          const float* __restrict__ fn,
                                                          const float* __restrict__ base,
                                                          const float* __restrict__ scale, HcCoef* __restrict__ coef,
                                                          __nv_bfloat16* __restrict__ v_out,
+                                                         __nv_bfloat16* __restrict__ mean,
                                                          const __nv_bfloat16* __restrict__ norm_w,
                                                          __half* __restrict__ h16, __nv_bfloat16* __restrict__ hb,
                                                          int H, int d, int iters, float eps, float rms_eps) {
@@ -37,7 +41,7 @@ __global__ void __launch_bounds__(256) hc_prepare_kernel(const __nv_bfloat16* __
   __shared__ float mix[kMaxMix + 1];
   __shared__ float s_pre[kMaxH];
   __shared__ float s_vv[8];
-  const int r = blockIdx.x, nmix = H * (2 + H), n = H * d;
+  const int r = blockIdx.x, nmix = HEAD ? H : H * (2 + H), n = H * d;
   const __nv_bfloat16* xr = x + (long)r * n;
   float acc[kMaxMix + 1];
 #pragma unroll
@@ -64,7 +68,11 @@ __global__ void __launch_bounds__(256) hc_prepare_kernel(const __nv_bfloat16* __
     mix[threadIdx.x] = t;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (HEAD) {
+    if (threadIdx.x < H)
+      s_pre[threadIdx.x] = 1.f / (1.f + expf(-(mix[threadIdx.x] * rsqrtf(mix[kMaxMix] / n + rms_eps) * scale[0] +
+                                               base[threadIdx.x]))) + eps;
+  } else if (threadIdx.x == 0) {
     const float inv = rsqrtf(mix[kMaxMix] / n + rms_eps);
     HcCoef c;
     for (int h = 0; h < H; ++h) {
@@ -113,9 +121,15 @@ __global__ void __launch_bounds__(256) hc_prepare_kernel(const __nv_bfloat16* __
   float vv = 0.f;
   for (int i = threadIdx.x; i < d; i += 256) {
     float v = 0.f;
-    for (int h = 0; h < H; ++h) v = fmaf(s_pre[h], __bfloat162float(xr[h * d + i]), v);
+    float m = 0.f;
+    for (int h = 0; h < H; ++h) {
+      const float a = __bfloat162float(xr[h * d + i]);
+      v = fmaf(s_pre[h], a, v);
+      m += a;
+    }
     const __nv_bfloat16 vb = __float2bfloat16_rn(v);
     v_out[(long)r * d + i] = vb;
+    if (HEAD && mean) mean[(long)r * d + i] = __float2bfloat16_rn(m / H);
     const float vr = __bfloat162float(vb);
     vv += vr * vr;
   }
@@ -129,7 +143,8 @@ __global__ void __launch_bounds__(256) hc_prepare_kernel(const __nv_bfloat16* __
   for (int w = 0; w < 8; ++w) tot += s_vv[w];
   const float inv = rsqrtf(tot / d + rms_eps);
   for (int i = threadIdx.x; i < d; i += 256) {
-    const float y = __bfloat162float(v_out[(long)r * d + i]) * inv * __bfloat162float(norm_w[i]);
+    float y = __bfloat162float(v_out[(long)r * d + i]) * inv * __bfloat162float(norm_w[i]);
+    if (HEAD) y = bf16_round(y);
     if (h16) h16[(long)r * d + i] = __float2half(y);
     if (hb) hb[(long)r * d + i] = __float2bfloat16_rn(y);
   }
@@ -507,8 +522,8 @@ TF_API int tf_hc_prepare(const void* x, const float* fn, const float* base, cons
               (const __nv_bfloat16*)norm_w, (__half*)h16, (__nv_bfloat16*)hb, rows, H, d, 0, iters, eps, rms_eps};
   const int c = launch_hc_cluster<false>(p, st);
   if (c != kHcGeneral) return c;
-  tf_launch(hc_prepare_kernel, dim3(rows), dim3(256), 0, st, (const __nv_bfloat16*)x, fn, base, scale, (HcCoef*)coef, (__nv_bfloat16*)v,
-                                          (const __nv_bfloat16*)norm_w, (__half*)h16, (__nv_bfloat16*)hb, H, d, iters,
+  tf_launch(hc_prepare_kernel<false>, dim3(rows), dim3(256), 0, st, (const __nv_bfloat16*)x, fn, base, scale, (HcCoef*)coef, (__nv_bfloat16*)v,
+                                          nullptr, (const __nv_bfloat16*)norm_w, (__half*)h16, (__nv_bfloat16*)hb, H, d, iters,
                                           eps, rms_eps);
   return (int)cudaGetLastError();
 }
@@ -516,7 +531,7 @@ TF_API int tf_hc_prepare(const void* x, const float* fn, const float* base, cons
 // Collapse in front of the vocabulary head: pre_h = sigmoid(m_h * scale[0] + base[h]) + eps with the H
 // mixes of x [rows, H, d] against fn [H, H*d], all scaled by rsqrt(mean(x^2) + rms_eps); v = bf16(sum_h
 // pre_h x_h), h16 / hb (optional) = RMSNorm of v with norm_w (bf16 values), mean (optional) = bf16 mean of the
-// copies.  d a multiple of 8, 16-byte aligned rows.
+// copies.
 TF_API int tf_hc_head(const void* x, const float* fn, const float* base, const float* scale, void* v, void* mean,
                       const void* norm_w, void* h16, void* hb, int rows, int H, int d, float eps, float rms_eps,
                       cudaStream_t st) {
@@ -525,7 +540,10 @@ TF_API int tf_hc_head(const void* x, const float* fn, const float* base, const f
   HcArgs p = {(const __nv_bfloat16*)x, fn, base, scale, nullptr, (__nv_bfloat16*)v, (__nv_bfloat16*)mean,
               (const __nv_bfloat16*)norm_w, (__half*)h16, (__nv_bfloat16*)hb, rows, H, d, 0, 0, eps, rms_eps};
   const int c = launch_hc_cluster<true>(p, st);
-  return c == kHcGeneral ? -1 : c;
+  if (c != kHcGeneral) return c;
+  tf_launch(hc_prepare_kernel<true>, dim3(rows), dim3(256), 0, st, p.x, fn, base, scale, nullptr, p.v, p.mean, p.norm_w, p.h16,
+            p.hb, H, d, 0, eps, rms_eps);
+  return (int)cudaGetLastError();
 }
 
 // y [rows, H, d] bf16 = post * a + comb^T x with a [rows, d] f32 (the reduced sublayer output)
