@@ -57,6 +57,15 @@ def test_build_provenance_notices_changed_sources(tmp_path, monkeypatch):
     shutil.rmtree(src)
 
 
+def test_shared_memory_limits_are_set_by_the_shared_helper_only():
+    """A kernel's dynamic shared-memory limit belongs to the device, not to a launch: set to the bytes of one launch, or once
+    per process, it is wrong for a second thread or a second device.  Only the helpers of ``common.cuh`` set it (fixed
+    bytes, once per device)."""
+    from titanic_flash_41_b200.utils import build
+    sets = [p.name for p in sorted(build.CSRC.glob("*.cu*")) if "cudaFuncSetAttribute" in p.read_text()]
+    assert sets == ["common.cuh"]
+
+
 def test_stage_weights_command(tmp_path, capsys):
     from titanic_flash_41_b200.models import loader, oracle
     cfg = tiny_config(dense_quant="fp8_block128", expert_quant="mxfp4")

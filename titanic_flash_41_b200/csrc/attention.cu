@@ -634,16 +634,11 @@ TF_API int tf_sparse_attention(const void* q, int T, int Hl, int Dh, const int* 
     return (int)cudaGetLastError();      // (sink, inverse rotation and the output rows are part of that kernel)
   } else if (Dh == 512 || Dh == 256) {
     const int smem = (kChunk * (Dh + 8) + Dh * (kChunk + 8)) * 2 + 4 * 16 * (kChunk + 4) * 4;
-    static bool attr_set = false;
-    if (!attr_set) {
-      cudaFuncSetAttribute(sparse_attn_wide_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (kChunk * (512 + 8) + 512 * (kChunk + 8)) * 2 + 4 * 16 * (kChunk + 4) * 4);
-      cudaFuncSetAttribute(sparse_attn_wide_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (kChunk * (256 + 8) + 256 * (kChunk + 8)) * 2 + 4 * 16 * (kChunk + 4) * 4);
-      attr_set = true;
-    }
-    if (Dh == 512) tf_launch(sparse_attn_wide_kernel<512>, dim3(grid), dim3(warps * 32), smem, st, p);
-    else tf_launch(sparse_attn_wide_kernel<256>, dim3(grid), dim3(warps * 32), smem, st, p);
+    auto kernel = Dh == 512 ? sparse_attn_wide_kernel<512> : sparse_attn_wide_kernel<256>;
+    static unsigned long long wide_set[2] = {0, 0};
+    const cudaError_t e = tf_smem_limit((const void*)kernel, smem, &wide_set[Dh == 512]);      // (fixed by the head dim)
+    if (e != cudaSuccess) return (int)e;
+    tf_launch(kernel, dim3(grid), dim3(warps * 32), smem, st, p);
   } else if (Dh == 128) {
     const int smem = kChunk * (128 + 8) * 2;
     tf_launch(sparse_attn_kernel<128>, dim3(grid), dim3(warps * 32), smem, st, p);

@@ -57,6 +57,19 @@ inline cudaError_t tf_smem_limit(const void* kernel, int bytes, unsigned long lo
   return e;
 }
 
+// The same up to all that the device leaves beside the kernel's static shared memory, for launches whose bytes vary:
+// a limit set to the bytes of one launch could be lowered by another thread before this one launches.
+inline cudaError_t tf_smem_limit_all(const void* kernel, unsigned long long* done) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (__atomic_load_n(done, __ATOMIC_RELAXED) >> (dev & 63) & 1) return cudaSuccess;
+  e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  return e == cudaSuccess ? tf_smem_limit(kernel, optin - (int)a.sharedSizeBytes, done) : e;
+}
+
 // ---------------------------------------------------------------------------------------
 // Status words.  No kernel traps, asserts or spins without a limit: a kernel that meets a
 // bad argument or a wait that runs out records (code, detail) here and returns; the host

@@ -96,9 +96,9 @@ bool fill(CombineParams& p, const float* y_pair, const int* ids, const float* wt
   return true;
 }
 
-cudaError_t dyn_smem(size_t dyn) {
-  if (dyn <= 40 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(combine_allreduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+cudaError_t dyn_smem() {
+  static unsigned long long limit_set = 0;
+  return tf_smem_limit_all((const void*)combine_allreduce_kernel, &limit_set);
 }
 
 }  // namespace
@@ -118,7 +118,7 @@ TF_API int tf_moe_combine_allreduce(const float* y_pair, const int* ids, const f
             ar_out, norm_w, h16, hb, x8, x8s, eps, spin_limit, status))
     return -1;
   const size_t dyn = (size_t)d * sizeof(float);
-  cudaError_t a = dyn_smem(dyn);
+  cudaError_t a = dyn_smem();
   if (a != cudaSuccess) return (int)a;
   tf_launch(combine_allreduce_kernel, dim3(d / 32), dim3(256), dyn, st, p);
   return (int)cudaGetLastError();
@@ -139,7 +139,7 @@ TF_API int tf_comm_allreduce_emulated(const float* partial, int rows, int rows_a
     return -1;
   p.emu_stride = (long)rows_alloc * d;
   const size_t dyn = (size_t)d * sizeof(float);
-  cudaError_t a = dyn_smem(dyn);
+  cudaError_t a = dyn_smem();
   if (a != cudaSuccess) return (int)a;
   // every CTA of every emulated rank must be resident: a cooperative launch fails instead of waiting
   int dev = 0, coop = 0, per_sm = 0, sms = 0;

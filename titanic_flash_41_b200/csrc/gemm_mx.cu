@@ -560,8 +560,9 @@ TF_API int tf_gemm_mx_rows(const void* A, long lda, const void* B, long ldb, lon
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(gemm_mx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   }
+  static unsigned long long limit_set = 0;
+  if (tf_smem_limit((const void*)gemm_mx_kernel, kSmemBytes, &limit_set) != cudaSuccess) return -2;
   CUtensorMap mA, mB;
   if (!tc::make_map_2d(&mA, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, lda, BM)) return -4;
   if (b_fp4) {

@@ -560,25 +560,12 @@ TF_API int tf_gemm_tc(int kind, const void* A, long lda, const void* B, long ldb
     const int gemm_ctas = g_sms - g_ag.copy_ctas;
     grid = (tiles < gemm_ctas ? tiles : gemm_ctas) + g_ag.copy_ctas;   // every CTA is resident: one per SM
   }
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(gemm_tc_kernel<0, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    cudaFuncSetAttribute(gemm_tc_kernel<1, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    cudaFuncSetAttribute(gemm_tc_kernel<2, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    cudaFuncSetAttribute(gemm_tc_kernel<0, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    cudaFuncSetAttribute(gemm_tc_kernel<1, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    cudaFuncSetAttribute(gemm_tc_kernel<2, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    attr_set = true;
-  }
-  if (BN == 128) {
-    if (kind == 0) tf_launch(gemm_tc_kernel<0, 128>, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p);
-    else if (kind == 1) tf_launch(gemm_tc_kernel<1, 128>, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p);
-    else tf_launch(gemm_tc_kernel<2, 128>, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p);
-  } else {
-    if (kind == 0) tf_launch(gemm_tc_kernel<0, 256>, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p);
-    else if (kind == 1) tf_launch(gemm_tc_kernel<1, 256>, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p);
-    else tf_launch(gemm_tc_kernel<2, 256>, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p);
-  }
+  auto kernel = BN == 128 ? (kind == 0 ? gemm_tc_kernel<0, 128> : kind == 1 ? gemm_tc_kernel<1, 128> : gemm_tc_kernel<2, 128>)
+                          : (kind == 0 ? gemm_tc_kernel<0, 256> : kind == 1 ? gemm_tc_kernel<1, 256> : gemm_tc_kernel<2, 256>);
+  static unsigned long long limit_set[6] = {0, 0, 0, 0, 0, 0};
+  const cudaError_t le = tf_smem_limit((const void*)kernel, kSmemBytes, &limit_set[(kind == 0 ? 0 : kind == 1 ? 1 : 2) + (BN == 128 ? 0 : 3)]);
+  if (le != cudaSuccess) return (int)le;
+  tf_launch(kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p);
   return (int)cudaGetLastError();
 }
 

@@ -650,7 +650,8 @@ TF_API int tf_index_scores_rows(const void* q, const float* w, const int* region
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kItSmem);
+  static unsigned long long limit_set[4] = {0, 0, 0, 0};
+  const cudaError_t e = tf_smem_limit((const void*)kernel, kItSmem, &limit_set[Hi == 8 ? 0 : Hi == 16 ? 1 : Hi == 32 ? 2 : 3]);
   if (e != cudaSuccess) return (int)e;
   // key tiles per item: many, so that Q is converted seldom, while there are two items for every SM
   const int rt = kItCols / Hi, row_tiles = (T + rt - 1) / rt, key_tiles = (key_hi - key_lo + kItKeys - 1) / kItKeys;

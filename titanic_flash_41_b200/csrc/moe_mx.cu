@@ -482,12 +482,6 @@ TF_API int tf_moe_gemv_mx(const void* w1, const void* w3, const void* s1, const 
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_mx_sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(moe_mx_kernel<0, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(moe_mx_kernel<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(moe_mx_kernel<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(moe_mx_kernel<0, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(moe_mx_kernel<1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(moe_mx_kernel<2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   }
   CUtensorMap m1, m3, mx, ms1, ms3, msx;
   if (!tc::make_map_2d_plain(&ms1, s1, (uint64_t)experts * N, K / 32, K / 32, 16, kTile)) return -4;
@@ -519,14 +513,11 @@ TF_API int tf_moe_gemv_mx(const void* w1, const void* w3, const void* s1, const 
   const int smem = stages * (mats * kTile * 128 + rows * 128) + kSfBufs * sfs + 1024 + 512;
   if (smem > 227 * 1024) return -3;
   const dim3 g(grid), t(kThreads);
-  if (rows == kRows) {
-    if (dual) tf_launch(moe_mx_kernel<1, 16>, g, t, smem, st, m1, m3, mx, ms1, ms3, msx, p);
-    else if (pair) tf_launch(moe_mx_kernel<2, 16>, g, t, smem, st, m1, m3, mx, ms1, ms3, msx, p);
-    else tf_launch(moe_mx_kernel<0, 16>, g, t, smem, st, m1, m3, mx, ms1, ms3, msx, p);
-  } else {
-    if (dual) tf_launch(moe_mx_kernel<1, 32>, g, t, smem, st, m1, m3, mx, ms1, ms3, msx, p);
-    else if (pair) tf_launch(moe_mx_kernel<2, 32>, g, t, smem, st, m1, m3, mx, ms1, ms3, msx, p);
-    else tf_launch(moe_mx_kernel<0, 32>, g, t, smem, st, m1, m3, mx, ms1, ms3, msx, p);
-  }
+  const int form = dual ? 1 : pair ? 2 : 0;
+  auto kernel = rows == kRows ? (form == 1 ? moe_mx_kernel<1, 16> : form == 2 ? moe_mx_kernel<2, 16> : moe_mx_kernel<0, 16>)
+                              : (form == 1 ? moe_mx_kernel<1, 32> : form == 2 ? moe_mx_kernel<2, 32> : moe_mx_kernel<0, 32>);
+  static unsigned long long limit_set[6] = {0, 0, 0, 0, 0, 0};
+  if (tf_smem_limit((const void*)kernel, 227 * 1024, &limit_set[form + (rows == kRows ? 0 : 3)]) != cudaSuccess) return -2;
+  tf_launch(kernel, g, t, smem, st, m1, m3, mx, ms1, ms3, msx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

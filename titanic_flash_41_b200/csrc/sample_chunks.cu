@@ -602,7 +602,8 @@ TF_API int tf_sample_chunks(const float* tlogits, const float* dlogits, const vo
   p.max_rows = max_rows; p.ctr = (unsigned int*)ctr; p.spin_limit = spin_limit; p.st = (TfStatusWord*)status;
   p.emu_tl = emu_tl; p.emu_dl = emu_dl; p.emu_stat = emu_stat; p.emu_tok = emu_tok; p.emu_acc = emu_acc;
   const size_t dyn = (size_t)chunk * 8 + 32 * 256 * 8;
-  cudaError_t e = cudaFuncSetAttribute(sample_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  static unsigned long long limit_set = 0;
+  const cudaError_t e = tf_smem_limit_all((const void*)sample_chunks_kernel, &limit_set);
   if (e != cudaSuccess) return (int)e;
   const int ez = ranks_emulated > 1 ? ranks_emulated : 1;
   dim3 grid(max_rows, csplit, ez);

@@ -495,11 +495,9 @@ TF_API int tf_smallm_gemm_allreduce(const void* W, const void* S, int ldw, int l
   p.ep.h16 = (__half*)h16; p.ep.hb = (__nv_bfloat16*)hb; p.ep.x8 = (uint8_t*)x8; p.ep.x8s = (uint8_t*)x8s;
   p.ep.eps = eps;
   const size_t dyn = (size_t)N * sizeof(float);
-  if (dyn > 24 * 1024) {
-    cudaError_t a = cudaFuncSetAttribute(smallm_gemm_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)dyn);
-    if (a != cudaSuccess) return (int)a;
-  }
+  static unsigned long long limit_set = 0;
+  const cudaError_t a = tf_smem_limit_all((const void*)smallm_gemm_kernel<0, false>, &limit_set);
+  if (a != cudaSuccess) return (int)a;
   dim3 grid(N / kTileN, 1);
   tf_launch(smallm_gemm_kernel<0, false>, dim3(grid), dim3(kMaxWarps * 32), dyn, stream, p);
   return (int)cudaGetLastError();
