@@ -92,6 +92,32 @@ def test_smallm_dense_stream(M, N, K, kind):
     assert (out[M] == 9.0).all()
 
 
+@pytest.mark.parametrize("M,kind,okind", [(33, "fp8", 1), (70, "dual", 0), (64, "bf16", 2), (96, "fp8", 0)])
+def test_smallm_dense_of_more_rows_than_a_pass(M, kind, okind):
+    """Ungrouped matrices with more than 32 rows go through the dense form 32 rows at a time: ragged and full last passes, a
+    padded output pitch and the three output types.  fp32 sums of K exact products, then one rounding of the output type."""
+    torch.manual_seed(M)
+    N, K = 256, 1152
+    x = torch.randn(M, K, device=DEV).to(torch.bfloat16 if kind == "bf16" else torch.float16)
+    out = torch.full((M + 1, N + 8), 9.0, device=DEV, dtype=(torch.float32, torch.float16, torch.bfloat16)[okind])
+    ws = [E.quant_fp8_device(torch.randn(N, K, device=DEV) * 0.05) for _ in range(2)]
+    wb = (torch.randn(N, K, device=DEV) * 0.05).bfloat16()
+    if kind == "bf16":
+        native.call("tf_smallm_gemm", 2, wb, None, None, None, 0, 0, K * 2, 0, x, K, out, N + 8, okind, N, K, M,
+                    None, None, None, None, None, 1, 0, M, 0.0)
+        want = x.double() @ wb.double().t()
+    else:
+        w3 = ws[1] if kind == "dual" else None
+        native.call("tf_smallm_gemm", 0, ws[0].q, w3.q if w3 else None, ws[0].s, w3.s if w3 else None, 0, 0, K, K // 128,
+                    x, K, out, N + 8, okind, N, K, M, None, None, None, None, None, 1, 0, M, 0.0)
+        want = x.double() @ E.dequant_fp8(ws[0]).double().t()
+        if w3 is not None:
+            want = want * torch.sigmoid(want) * (x.double() @ E.dequant_fp8(w3).double().t())
+    err = float((out[:M, :N].double() - want).norm() / want.norm())
+    assert err < 2e-6 * K ** 0.5 + (0.0, 2.0 ** -11, 2.0 ** -8)[okind]
+    assert (out[M] == 9.0).all() and (out[:, N:] == 9.0).all()
+
+
 def test_smallm_bf16_head():
     torch.manual_seed(1)
     N, K, M = 2048, 512, 9

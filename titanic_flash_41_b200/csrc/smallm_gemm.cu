@@ -4,16 +4,17 @@
 //                                            MXFP4 = packed e2m1 + one UE8M0 per 32 along K (kind 1),
 //                                            or bf16 (kind 2, bf16 activations)
 //
-// At these row counts the op is bound by reading W once from HBM, so the kernel is organised
-// around the weight stream: every lane issues 16-byte loads of consecutive K of one weight row,
-// converts in registers (cvt e4m3x2->f16x2; e2m1 through an exponent-field trick) and feeds
-// m16n8k16 tensor-core tiles in which 16 weight rows are the MMA's M and the (few) activation
-// rows its N.  The K index of an MMA slot is a permutation chosen so that the 16-byte weight load
-// IS the A fragment; the activation fragment follows the same permutation.  Per K step a warp
-// first issues the loads of ALL its weight tiles (two 16-row tiles, times two matrices in the
-// dual form: 8 x 16 B per lane in flight), then the activation fragments once, then the MMAs,
-// which keeps enough bytes in flight to follow HBM.  K is split over the warps of a CTA and
-// reduced through shared memory in a fixed order: results are run-to-run deterministic.
+// At these row counts the op is bound by reading W once from HBM.  Ungrouped FP8 and bf16 matrices run on the
+// asynchronous ring of smallm_dense.cuh (32 rows a pass); the register-fed kernel of this file serves the grouped
+// forms, MXFP4 and the fused all-reduce.  It is organised around the weight stream: every lane issues 16-byte
+// loads of consecutive K of one weight row, converts in registers (cvt e4m3x2->f16x2; e2m1 through an exponent-
+// field trick) and feeds m16n8k16 tensor-core tiles in which 16 weight rows are the MMA's M and the (few)
+// activation rows its N.  The K index of an MMA slot is a permutation chosen so that the 16-byte weight load IS
+// the A fragment; the activation fragment follows the same permutation.  Per K step a warp first issues the loads
+// of ALL its weight tiles (two 16-row tiles, times two matrices in the dual form: 8 x 16 B per lane in flight),
+// then the activation fragments once, then the MMAs, which keeps enough bytes in flight to follow HBM.  K is split
+// over the warps of a CTA and reduced through shared memory in a fixed order: results are run-to-run
+// deterministic.
 //
 // Grouped form (routed experts): blockIdx.y walks a compacted list of active experts; rows of a
 // group are gathered through `sorted_pairs`.  `dual` computes W1 and W3 tiles together and
@@ -26,7 +27,7 @@
 namespace {
 
 constexpr int kWarps = 4;   // K is split four ways inside a CTA; four CTAs fit on an SM
-constexpr int kMaxWarps = 8;   // dense matrices with few 32-feature tiles split K eight ways instead (more warps per SM)
+constexpr int kMaxWarps = 8;   // the fused all-reduce form, one CTA for every 32 features, splits K eight ways instead
 constexpr int kTileN = 32;   // output columns per CTA (two m16 tiles per warp)
 
 struct SmallMParams {
@@ -83,7 +84,7 @@ __device__ __forceinline__ uint4 ld_stream(const uint8_t* p) {
   return v;
 }
 
-// One group (dense matrix or one expert): NT = 2 (or 4 in the dual form) weight tiles of 16 rows.
+// One group (the matrix of the fused all-reduce, or one expert): NT = 2 (or 4 in the dual form) weight tiles of 16 rows.
 template <int KIND, int MT, bool DUAL>
 __device__ __forceinline__ void run_rows(const SmallMParams& p, const uint8_t* Wg, const uint8_t* W3g,
                                          const void* Sg, const void* S3g, int rows, const int* pairs,
@@ -398,9 +399,9 @@ smallm_gemm_kernel(SmallMParams p) {
 }
 
 template <int KIND, bool DUAL>
-cudaError_t launch(const SmallMParams& p, int slots, cudaStream_t st, int warps = kWarps) {
+cudaError_t launch(const SmallMParams& p, int slots, cudaStream_t st) {
   dim3 grid((p.N + kTileN - 1) / kTileN, slots > 0 ? slots : 1);
-  tf_launch(smallm_gemm_kernel<KIND, DUAL>, dim3(grid), dim3(warps * 32), 0, st, p);
+  tf_launch(smallm_gemm_kernel<KIND, DUAL>, dim3(grid), dim3(kWarps * 32), 0, st, p);
   return cudaGetLastError();
 }
 
@@ -419,14 +420,22 @@ TF_API int tf_smallm_gemm(int kind, const void* W, const void* W3, const void* S
                           int max_rows, float swiglu_limit, cudaStream_t stream) {
   (void)max_rows;
   if (N % kTileN != 0 || K % 128 != 0 || (ldx % 8) != 0 || (ldw % 16) != 0) return -1;
-  const bool dual = W3 != nullptr;
-  if (!group_expert && (kind == 0 || (kind == 2 && !dual)) && M >= 1 && M <= 32) {
+  const bool dual = W3 != nullptr && kind != 2;            // (the bf16 form has one matrix)
+  if (!group_expert && (kind == 0 || kind == 2)) {
     DenseParams q;
     q.W = (const uint8_t*)W; q.W3 = (const uint8_t*)W3; q.S = (const float*)S; q.S3 = (const float*)S3;
     q.ldw = ldw; q.lds = lds; q.X = (const __half*)X; q.ldx = ldx; q.Y = Y; q.ldy = ldy; q.out_kind = out_kind;
-    q.N = N; q.K = K; q.M = M; q.tiles = 0; q.swiglu_limit = swiglu_limit; q.x_group_n = 0; q.x_group_stride = 0;
-    if (kind == 2) return (int)launch_dense<2, false>(q, stream);
-    return (int)(dual ? launch_dense<0, true>(q, stream) : launch_dense<0, false>(q, stream));
+    q.N = N; q.K = K; q.tiles = 0; q.swiglu_limit = swiglu_limit; q.x_group_n = 0; q.x_group_stride = 0;
+    for (int r0 = 0; r0 < M; r0 += 32) {                    // 32 rows a pass over the weights
+      q.M = M - r0 < 32 ? M - r0 : 32;
+      const cudaError_t e = kind == 2 ? launch_dense<2, false>(q, stream)
+                            : dual    ? launch_dense<0, true>(q, stream)
+                                      : launch_dense<0, false>(q, stream);
+      if (e != cudaSuccess) return (int)e;
+      q.X += 32L * ldx;
+      q.Y = (uint8_t*)q.Y + 32L * ldy * (out_kind == 0 ? 4 : 2);
+    }
+    return 0;
   }
   SmallMParams p;
   p.W = (const uint8_t*)W; p.W3 = (const uint8_t*)W3; p.S = S; p.S3 = S3;
@@ -439,13 +448,7 @@ TF_API int tf_smallm_gemm(int kind, const void* W, const void* W3, const void* S
   p.k_per_warp = ((K + kWarps - 1) / kWarps + 127) / 128 * 128;
   p.use_comm = 0;
   cudaError_t e;
-  // dense FP8 with so few tiles that an SM gets two CTAs or fewer: eight K-splitting warps per CTA
-  int warps = kWarps;
-  if (kind == 0 && !dual && !group_expert && N / kTileN <= 320 && K >= 8 * 256) {
-    warps = kMaxWarps;
-    p.k_per_warp = ((K + warps - 1) / warps + 127) / 128 * 128;
-  }
-  if (kind == 0) e = dual ? launch<0, true>(p, slots, stream) : launch<0, false>(p, slots, stream, warps);
+  if (kind == 0) e = dual ? launch<0, true>(p, slots, stream) : launch<0, false>(p, slots, stream);
   else if (kind == 1) e = dual ? launch<1, true>(p, slots, stream) : launch<1, false>(p, slots, stream);
   else if (kind == 2) e = launch<2, false>(p, slots, stream);
   else return -1;
