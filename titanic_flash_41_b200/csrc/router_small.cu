@@ -5,7 +5,7 @@
 // on memory latency.  Here one CTA owns two expert rows and its eight warps an eighth of the inputs
 // each: every lane walks its part in 16-byte steps with one accumulator per expert and activation row (the rows
 // come out of L1 / L2, once for both experts), the warps' partial sums meet in shared memory and
-// are added in warp order.  Fixed summation order: bitwise reproducible.  Row counts up to 4 and 8 have
+// are added by pairs.  Fixed summation order: bitwise reproducible.  Row counts up to 4 and 8 have
 // forms of their own: with sixteen accumulators (and sixteen clamped loads) for any count, one expert
 // and four warps a CTA, one row took 11 us and sixteen 12.4 us.
 //
@@ -82,10 +82,15 @@ router_logits_small_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const _
     if (threadIdx.x < kRouterExperts * ROWS) {
       const int q = threadIdx.x / ROWS, r = threadIdx.x % ROWS;
       if (t0 + r < T && e0 + q < E) {
-        float v = 0.f;
+        // by pairs: a chain over eight warps rounds more than one over four
+        float v[kRouterWarps];
 #pragma unroll
-        for (int w = 0; w < kRouterWarps; ++w) v += red[w][q][r];
-        out[(long)(t0 + r) * ldo + e0 + q] = v;
+        for (int w = 0; w < kRouterWarps; ++w) v[w] = red[w][q][r];
+#pragma unroll
+        for (int o = kRouterWarps / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int w = 0; w < o; ++w) v[w] += v[w + o];
+        out[(long)(t0 + r) * ldo + e0 + q] = v[0];
       }
     }
     __syncthreads();
