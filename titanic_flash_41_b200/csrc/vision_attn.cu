@@ -126,20 +126,15 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     if (lane == 0) {
       tc::mbar_expect_tx(q_full, kTileBytes);
       tc::tma_load_2d(q_s, &mapQ, 0, hrow + row0, q_full);
-      bool ok = true;
       for (int j = 0; j < tiles; ++j) {
         const int s = j % kRing;
         const uint32_t ph = ((j / kRing) & 1) ^ 1;
-        if (!(ok = tc::mbar_wait(k_empty(s), ph, abort_flag))) break;
+        if (!tc::mbar_wait(k_empty(s), ph, abort_flag)) break;
         tc::mbar_expect_tx(k_full(s), kTileBytes);
         tc::tma_load_2d(k_s + s * kTileBytes, &mapK, 0, hrow + j * kTile, k_full(s));
-        if (!(ok = tc::mbar_wait(v_empty(s), ph, abort_flag))) break;
+        if (!tc::mbar_wait(v_empty(s), ph, abort_flag)) break;
         tc::mbar_expect_tx(v_full(s), kTileBytes);
         tc::tma_load_2d(v_s + s * kTileBytes, &mapV, 0, hrow + j * kTile, v_full(s));
-      }
-      if (!ok) {
-        const long long t0 = clock64();
-        while (clock64() - t0 < 400000) {}       // copies in flight land before the smem goes back
       }
     }
   } else if (warp == 4) {
@@ -275,7 +270,13 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) tf_report(p.st, TF_TIMEOUT, 160, blockIdx.x, blockIdx.y);
+  if (*abort_flag) {
+    // whichever role gave up (the producer may have issued its last copy and left before): copies in flight land
+    // before the shared memory goes back
+    const long long t0 = clock64();
+    while (clock64() - t0 < 400000) {}
+    if (threadIdx.x == 0) tf_report(p.st, TF_TIMEOUT, 160, blockIdx.x, blockIdx.y);
+  }
   if (warp == 4) {
     tc::tc_fence_after();
     tc::tmem_dealloc(tS, kVaCols);
