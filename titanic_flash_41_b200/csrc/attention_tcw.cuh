@@ -17,9 +17,11 @@
 //               head through shared memory) and finish the row (neighbouring lanes hold a rotation pair)
 //   warp 12     one thread issues the MMAs: QK of chunk c + 1 before PV of chunk c
 //
-// Bound by shared memory: with N = 64 an MMA step (128 x 64 x 16) reads 6 KB of operands, 48 cycles at 128 bytes a
-// cycle, for 32 cycles of math: 2,300 cycles a chunk, and the gather's 64 KB of writes beside them.  The mma.sync kernel dequantised every key once per
-// 16 heads and kept a transposed copy: 17.9 ms for 4,001 rows of 64 heads and up to 640 keys.
+// Shared memory would allow 2,300 cycles a chunk: with N = 64 an MMA step (128 x 64 x 16) reads 6 KB of operands, 48
+// cycles at 128 bytes a cycle, for 32 cycles of math, and the gather writes 64 KB beside them.  Measured 7,000 - 8,000 (0.98 ms
+// for 4,001 rows of 64 heads and up to 640 keys; tensor pipe 20 % active): bound by the chain of gather, QK, softmax and PV
+// of the two chunks in flight.  The mma.sync kernel dequantised every key once per 16 heads and kept a
+// transposed copy: 17.9 ms.
 // Every wait is bounded as in the narrow kernel.
 #pragma once
 

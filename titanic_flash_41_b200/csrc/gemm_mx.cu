@@ -414,8 +414,9 @@ __global__ void __launch_bounds__(128) swiglu_rows_mx_units_kernel(const __nv_bf
 // scales of a 128-deep k block) this is the transpose of a [rows][K/128] matrix: word (kb, row) lands at
 // kb * units * 32 + row.  Bound by HBM, so a CTA moves 128 rows x 32 words through shared memory and
 // both sides are whole 128-byte lines (a 33-word pitch keeps the column reads free of bank conflicts).
-// One thread per byte scattered over 512-byte strides took 272 us for 524,288 rows of K = 4096 (134 MB
-// moved, 0.5 TB/s); a 197-row prefill of four layers (twelve of these) went from 9.44 to 6.95 ms.  `s` or `out` off a 4-byte boundary: byte by byte.
+// 524,288 rows of K = 4096 (134 MB moved): 272 us with one thread per byte scattered over 512-byte strides, 58 us
+// in this form, 20 us in 16-byte pieces (sf_to_units_vec_kernel below), which K / 128 of a multiple of eight takes; this
+// form serves the other widths and addresses off the 16-byte grain.  `s` or `out` off a 4-byte boundary: byte by byte.
 constexpr int kTrRows = 128, kTrWords = 32;
 __global__ void __launch_bounds__(256) sf_to_units_kernel(const uint8_t* __restrict__ s, uint8_t* __restrict__ out,
                                                           long rows, int kb_n, int units, int words) {

@@ -14,9 +14,12 @@
 //               f16 (value times block scale), two stages
 //   warps 4-7   epilogue, one 32-lane quadrant each; also blank the columns past a row's valid keys
 //   warp 8      one thread issues the MMAs (128 x 256 x 128, two accumulators of 256 columns)
-// Bound by the MMAs (1,021 cycles a tile; the epilogue's 256 x 2 operations a thread run beside them).
-// Every wait is bounded: on a time-out the CTA raises its abort flag, frees its tensor memory and leaves; the
-// score rows it did not write keep what they held, and the status word of the step says so.
+// Bound by the epilogue: a tile takes about 5,500 cycles (2,048 rows x 32,768 keys x 8 heads: 324 us), in which its MMAs
+// keep the tensor pipe busy for a fifth; a warp walks its 256 columns in eight dependent steps of tensor-memory load,
+// sums, row limit and store.
+// Every wait is bounded: on a time-out the CTA raises its abort flag and the other roles leave; the epilogue stops waiting
+// and runs out its items, so that the scores it writes from then on are void (the status word of the step says so).
+// Then the tensor memory is freed.
 #pragma once
 #include "tc.cuh"
 

@@ -12,8 +12,9 @@
 // and one's exponentials run while the other waits for its MMAs.
 //
 // Bound by the exponentials: 128 x 128 of them take 1,024 cycles of the SM's special function units
-// against 256 cycles of MMAs.  The products went through HBM before (fp32 scores and bf16 probabilities of
-// one head at a time): 4.1 ms a layer of 8,580 patches x 16 heads.
+// against 512 cycles of MMAs (2.1 M multiply-adds of a tile pair at 4,096 a cycle).  The products went through
+// HBM before (fp32 scores and bf16 probabilities of one head at a time): 4.1 ms a layer of 8,580 patches x
+// 16 heads.
 //
 // Every mbarrier wait is bounded; on a time-out the CTA raises its abort flag, reports TF_TIMEOUT, lets
 // copies in flight land, frees its tensor memory and returns.
