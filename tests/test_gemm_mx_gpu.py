@@ -209,3 +209,67 @@ def test_grouped_gemm_and_swiglu_store_only_rows_that_count():
         native.call("tf_swiglu_rows_mx_units", y, 2 * N, q[i], sf[i], M // 32, M, N, 10.0, n, tr)
     assert torch.equal(q[1][live], q[0][live]) and bool((q[1][~live] == 9).all())
     assert torch.equal(mx.units_to_rowmajor(sf[1], M)[live], mx.units_to_rowmajor(sf[0], M)[live])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 136, 128), (33, 128, 256), (197, 9864, 512), (255, 384, 896), (257, 512, 1152), (1500, 4096, 640)])
+def test_gemm_mx_dense_tiles(M, N, K):
+    """Row tiles of every width the tile rule takes, a last tile of a few rows, feature blocks that end inside a CTA's 128
+    features or in the pair's second CTA: the same operands in fp64.  fp32 accumulation of K exact products: 2e-5 as above."""
+    gen = torch.Generator(device=DEV).manual_seed(M + K)
+    aq, bq = _random_fp8(M, K, gen), _random_fp8(N, K, gen)
+    sa = torch.randint(118, 126, (M, K // 32), device=DEV, dtype=torch.uint8, generator=gen)
+    sb = torch.randint(118, 126, (N, K // 32), device=DEV, dtype=torch.uint8, generator=gen)
+    deq = lambda q, s: (q.view(F8).double().view(-1, K // 32, 32) * torch.exp2(s.double() - 127)[:, :, None]).view(-1, K)
+    want = deq(aq, sa) @ deq(bq, sb).t()
+    st = native.StatusWord(DEV)
+    for dt, tol in ((torch.float32, 2e-5), (torch.bfloat16, 4e-3)):
+        c = torch.full((M + 1, N + 8), 7.0, device=DEV, dtype=dt)
+        mx.gemm(aq, mx.units_from_rowmajor(sa, K, 128), bq, mx.units_from_rowmajor(sb, K), c, M, N, K, st.t)
+        st.check()
+        assert _rel(c[:M, :N], want) < tol
+        assert bool((c[:, N:] == 7.0).all()) and bool((c[M] == 7.0).all())
+
+
+@pytest.mark.parametrize("K,tile_max,two", [(512, 32, True), (768, 96, True), (1280, 160, False), (1024, 192, True), (2304, 256, False)])
+def test_gemm_mx_experts_tiles(K, tile_max, two):
+    """Experts of 0, 1, 31, 33, tile_max and more rows through the tile plan, scales row-major as stored (rows of a multiple
+    of 16 bytes and of 8 bytes off it), one and two matrices: live rows against fp64, padding keeps what it held."""
+    gen = torch.Generator(device=DEV).manual_seed(K)
+    counts = [1, 31, 0, 33, tile_max, tile_max + 1, 300]
+    El, N, n = len(counts), 256, sum(counts)
+    ids = torch.repeat_interleave(torch.arange(El), torch.tensor(counts))[torch.randperm(n)].int().to(DEV)
+    i32 = lambda k: torch.full((k,), -5, dtype=torch.int32, device=DEV)
+    cap, room = -(-(n + El * 31) // 32) * 32, n // tile_max + El
+    offs, cur, te, r0, tr, nt, pad, dst = i32(El + 1), i32(El), i32(room), i32(room), i32(room), i32(1), i32(1), i32(n)
+    native.call("tf_moe_plan_tiles", ids, n, 0, El, torch.zeros(El, dtype=torch.int32, device=DEV), offs, cur, te, r0, tr, tile_max,
+                room, nt, pad, dst)
+    want_offs = [0]
+    for c in counts:
+        want_offs.append(want_offs[-1] + -(-c // 32) * 32)
+    assert offs.tolist() == want_offs and int(pad) == want_offs[-1] <= cap
+    seen = []
+    for t in range(int(nt)):
+        e, a, m = int(te[t]), int(r0[t]), int(tr[t])
+        assert a % 32 == 0 and 0 < m <= tile_max
+        seen += list(range(a, a + m))
+    assert sorted(dst.tolist()) == sorted(seen) and len(set(seen)) == n
+    aq = _random_fp8(cap, K, gen)
+    sa = torch.randint(118, 126, (cap, K // 32), device=DEV, dtype=torch.uint8, generator=gen)
+    pk = [torch.randint(0, 256, (El, N, K // 2), device=DEV, dtype=torch.uint8, generator=gen) for _ in range(2)]
+    sc = [torch.randint(118, 126, (El, N, K // 32), device=DEV, dtype=torch.uint8, generator=gen) for _ in range(2)]
+    a = (aq.view(F8).double().view(cap, K // 32, 32) * torch.exp2(sa.double() - 127)[:, :, None]).view(cap, K)
+    st = native.StatusWord(DEV)
+    for dt, tol in ((torch.float32, 2e-5), (torch.bfloat16, 4e-3)):
+        c = torch.full((cap, 2 * N + 8), 5.0, device=DEV, dtype=dt)
+        mx.gemm_experts(aq, mx.units_from_rowmajor(sa, K, 128), pk[0], pk[1] if two else None, sc[0], sc[1] if two else None, El * N,
+                        c, cap, N, K, (te, r0, tr, nt, tile_max, room), st.t)
+        st.check()
+        expert = torch.full((cap,), -1, device=DEV)
+        expert[dst.long()] = ids.long()
+        for e in range(El):
+            rows = expert == e
+            for j in range(2 if two else 1):
+                if int(rows.sum()):
+                    w = E.dequant_mxfp4(pk[j][e], sc[j][e]).double()
+                    assert _rel(c[rows, j * N:(j + 1) * N], a[rows] @ w.t()) < tol
+        assert bool((c[expert < 0] == 5.0).all()) and bool((c[:, (2 if two else 1) * N:] == 5.0).all())

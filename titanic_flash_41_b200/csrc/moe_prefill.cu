@@ -122,49 +122,67 @@ __global__ void moe_count_kernel(const int* __restrict__ ids, int n_pairs, int e
 // single CTA: padded offsets, tile table, cursors reset.  tile_expert has room for max_tiles ints.
 // One thread per expert and a block-wide prefix sum of the tile counts (experts beyond the block's
 // threads in further passes): one thread walking 256 experts spent 36 us on its chain of loads.
+// tile_max 0: segments of whole 128-row tiles.  Otherwise segments of whole 32 rows, cut into as few tiles of at most
+// tile_max rows as there can be, all of one size (a multiple of 32) but the last.
 constexpr int kOffThreads = 512;
 __global__ void __launch_bounds__(kOffThreads) moe_offsets_kernel(int* counts, int El, int* offsets, int* cursor,
-                                                                  int* tile_expert, int* tile_rows, int max_tiles,
-                                                                  int* num_tiles, int* padded_rows) {
+                                                                  int* tile_expert, int* tile_row0, int* tile_rows,
+                                                                  int tile_max, int max_tiles, int* num_tiles,
+                                                                  int* padded_rows) {
   tf_pdl_sync();
-  __shared__ int wsum[kOffThreads / 32];
+  __shared__ int wsum[kOffThreads / 32], wrow[kOffThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int before = 0;                                  // tiles of the passes before
+  const int align = tile_max ? 32 : 128;
+  int before = 0, rbefore = 0;                     // tiles and padded rows of the passes before
   for (int e0 = 0; e0 < El; e0 += kOffThreads) {
     const int e = e0 + threadIdx.x;
-    const int cnt = e < El ? counts[e] : 0, tiles = (cnt + 127) / 128;
-    int inc = tiles;
+    const int cnt = e < El ? counts[e] : 0, rows = (cnt + align - 1) / align * align;
+    const int tiles = tile_max ? (cnt + tile_max - 1) / tile_max : rows / 128;
+    int inc = tiles, rinc = rows;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += v;
+      const int v = __shfl_up_sync(0xffffffffu, inc, o), r = __shfl_up_sync(0xffffffffu, rinc, o);
+      if (lane >= o) {
+        inc += v;
+        rinc += r;
+      }
     }
-    if (lane == 31) wsum[warp] = inc;
+    if (lane == 31) {
+      wsum[warp] = inc;
+      wrow[warp] = rinc;
+    }
     __syncthreads();
-    int pre = before, all = 0;
+    int pre = before, all = 0, rpre = rbefore, rall = 0;
 #pragma unroll
     for (int w = 0; w < kOffThreads / 32; ++w) {
-      const int v = wsum[w];
-      if (w < warp) pre += v;
+      const int v = wsum[w], r = wrow[w];
+      if (w < warp) {
+        pre += v;
+        rpre += r;
+      }
       all += v;
+      rall += r;
     }
-    const int t0 = pre + inc - tiles;
+    const int t0 = pre + inc - tiles, r0 = rpre + rinc - rows;
     if (e < El) {
-      offsets[e] = t0 * 128;
+      offsets[e] = r0;
       cursor[e] = 0;
       counts[e] = 0;                               // ready for the next launch
+      const int size = tile_max && tiles ? ((cnt + tiles - 1) / tiles + 31) / 32 * 32 : 128;
       for (int j = 0; j < tiles && t0 + j < max_tiles; ++j) {
         tile_expert[t0 + j] = e;
-        if (tile_rows) tile_rows[t0 + j] = min(128, cnt - 128 * j);
+        if (tile_row0) tile_row0[t0 + j] = r0 + size * j;
+        if (tile_rows) tile_rows[t0 + j] = min(size, cnt - size * j);
       }
     }
     before += all;
+    rbefore += rall;
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    offsets[El] = before * 128;
+    offsets[El] = rbefore;
     *num_tiles = min(before, max_tiles);
-    *padded_rows = before * 128;
+    *padded_rows = rbefore;
   }
 }
 __global__ void moe_place_kernel(const int* __restrict__ ids, int n_pairs, int e_lo, int El,
@@ -363,7 +381,22 @@ TF_API int tf_moe_plan_rows(const int* ids, int n_pairs, int e_lo, int El, int* 
                             int* pair_dst, cudaStream_t st) {
   const unsigned grid = (unsigned)((n_pairs + 255) / 256);
   tf_launch(moe_count_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, counts);
-  tf_launch(moe_offsets_kernel, dim3(1), dim3(kOffThreads), 0, st, counts, El, offsets, cursor, tile_expert, tile_rows, max_tiles, num_tiles, padded_rows);
+  tf_launch(moe_offsets_kernel, dim3(1), dim3(kOffThreads), 0, st, counts, El, offsets, cursor, tile_expert,
+            (int*)nullptr, tile_rows, 0, max_tiles, num_tiles, padded_rows);
+  tf_launch(moe_place_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, offsets, cursor, pair_dst);
+  return (int)cudaGetLastError();
+}
+
+// The plan of tf_gemm_mx_experts: segments of whole 32 rows (padded_rows <= n_pairs + 31 * El), tiles of at most tile_max rows
+// (a multiple of 32; at most n_pairs / tile_max + El of them).
+TF_API int tf_moe_plan_tiles(const int* ids, int n_pairs, int e_lo, int El, int* counts, int* offsets, int* cursor,
+                             int* tile_expert, int* tile_row0, int* tile_rows, int tile_max, int max_tiles, int* num_tiles,
+                             int* padded_rows, int* pair_dst, cudaStream_t st) {
+  if (n_pairs <= 0 || tile_max < 32 || tile_max % 32 || !tile_row0 || !tile_rows || max_tiles < n_pairs / tile_max + El) return -1;
+  const unsigned grid = (unsigned)((n_pairs + 255) / 256);
+  tf_launch(moe_count_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, counts);
+  tf_launch(moe_offsets_kernel, dim3(1), dim3(kOffThreads), 0, st, counts, El, offsets, cursor, tile_expert, tile_row0,
+            tile_rows, tile_max, max_tiles, num_tiles, padded_rows);
   tf_launch(moe_place_kernel, dim3(grid), dim3(256), 0, st, ids, n_pairs, e_lo, El, offsets, cursor, pair_dst);
   return (int)cudaGetLastError();
 }

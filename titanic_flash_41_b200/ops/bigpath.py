@@ -25,8 +25,7 @@ class BigPath:
         self.e = engine
         self.buf = {}
         self._converted = None      # layer whose experts currently sit in the FP8 staging copy
-        self._mx_layer = None       # layer whose expert scales currently sit in the block-scaled layout
-        self._mx_u = []
+        self._mx_layer = None       # layer whose experts took the block-scaled form last
         self.resident = engine.world >= 4          # per-layer FP8 expert copies stay on the device
         self._resident = {}
 
@@ -110,9 +109,6 @@ class BigPath:
         cfg = eng.cfg
         d, I, El, k = cfg.hidden, cfg.moe_inter, eng.El, cfg.topk
         npairs = T * k
-        cap = npairs + El * 127
-        cap = -(-cap // 128) * 128
-        max_tiles = cap // 128
         i32 = torch.int32
         z = self.buf.get("counts")
         if z is None:
@@ -120,44 +116,38 @@ class BigPath:
             self.buf["counts"] = z
         offsets = self._get("offsets", (El + 1,), i32)
         cursor = self._get("cursor", (El,), i32)
-        tile_e = self._get("tile_e", (max_tiles,), i32)
         ntile = self._get("ntile", (2,), i32)
         pair_dst = self._get("pair_dst", (npairs,), i32)
         e_lo = eng.rank * El
-        tile_r = self._get("tile_r", (max_tiles,), i32)
-        native.call("tf_moe_plan_rows", b["ids"], npairs, e_lo, El, z, offsets, cursor, tile_e, tile_r, max_tiles, ntile[0:1],
-                    ntile[1:2], pair_dst)
         st = eng.status.t
-        if eng.ecfg.prefill_mx and d % 128 == 0 and I % 256 == 0 and d % 256 == 0:
-            # block-scaled form: the packed e2m1 weights are read as stored; their UE8M0 scales are
-            # re-ordered into the kernel's layout once per layer visit (a few hundred MB of traffic
-            # against the GBs of the FP8 re-expression below)
-            if self._mx_layer is not L:
-                u = self._get("mx_units", (3, (d // 128) * mx.sf_units(El * I, 256) * 128), torch.uint8)
-                self._mx_u = []
-                for j, (sc, rows, kk) in enumerate(((L.es1, El * I, d), (L.es3, El * I, d), (L.es2, El * d, I))):
-                    uu = u[j][: (kk // 128) * mx.sf_units(rows, 256) * 128].view(kk // 128, mx.sf_units(rows, 256), 128)
-                    native.call("tf_mx_sf_to_units", sc, uu, rows, kk, uu.shape[1])
-                    self._mx_u.append(uu)
-                self._mx_layer = L
-            u1, u3, u2 = self._mx_u
+        if eng.ecfg.prefill_mx and d % 256 == 0 and I % 256 == 0:
+            # block-scaled form: the packed e2m1 weights and their UE8M0 scales are read as stored
+            self._mx_layer = L
+            tile_max = mx.expert_tile_rows(npairs, El * eng.world)
+            cap = -(-(npairs + El * 31) // 32) * 32
+            max_tiles = npairs // tile_max + El
+            tile_e, tile_r0, tile_r = (self._get(nm, (max_tiles,), i32) for nm in ("tile_e", "tile_r0", "tile_r"))
+            native.call("tf_moe_plan_tiles", b["ids"], npairs, e_lo, El, z, offsets, cursor, tile_e, tile_r0, tile_r, tile_max,
+                        max_tiles, ntile[0:1], ntile[1:2], pair_dst)
             xp = self._get("xp", (cap, d), torch.uint8)
             sfx = self._get("sfx_mx", (d // 128, cap // 32, 128), torch.uint8)
             mx.quant_rows(b["h16"], npairs, d, xp, sfx, x_div=k, pair_dst=pair_dst)
             y1 = self._get("y1", (cap, 2 * I), torch.bfloat16)
-            mx.gemm(xp, sfx, L.ew1, u1, y1, cap, I, d, st, b_fp4=True, b_rows=El * I, tile_expert=tile_e,
-                    num_m_tiles=ntile[0:1], tile_rows=tile_r)
-            mx.gemm(xp, sfx, L.ew3, u3, y1[:, I:], cap, I, d, st, b_fp4=True, b_rows=El * I, tile_expert=tile_e,
-                    num_m_tiles=ntile[0:1], tile_rows=tile_r)
+            tiles = (tile_e, tile_r0, tile_r, ntile[0:1], tile_max, max_tiles)
+            mx.gemm_experts(xp, sfx, L.ew1, L.ew3, L.es1, L.es3, El * I, y1, cap, I, d, tiles, st)
             aq = self._get("aq", (cap, I), torch.uint8)
             sfq = self._get("sfq_mx", (I // 128, cap // 32, 128), torch.uint8)
-            native.call("tf_swiglu_rows_mx_units", y1, 2 * I, aq, sfq, cap // 32, cap, I, cfg.swiglu_limit, ntile[1:2],
-                        tile_r)
+            native.call("tf_swiglu_pairs_mx_units", y1, 2 * I, aq, sfq, cap // 32, pair_dst, npairs, I, cfg.swiglu_limit)
             y2 = self._get("y2", (cap, d), torch.bfloat16)
-            mx.gemm(aq, sfq, L.ew2, u2, y2, cap, d, I, st, b_fp4=True, b_rows=El * d, tile_expert=tile_e,
-                    num_m_tiles=ntile[0:1], tile_rows=tile_r)
+            mx.gemm_experts(aq, sfq, L.ew2, None, L.es2, None, El * d, y2, cap, d, I, tiles, st)
             self._moe_tail(eng, L, T, b, y2, pair_dst, with_shared, out)
             return
+        cap = npairs + El * 127
+        cap = -(-cap // 128) * 128
+        max_tiles = cap // 128
+        tile_e = self._get("tile_e", (max_tiles,), i32)
+        native.call("tf_moe_plan", b["ids"], npairs, e_lo, El, z, offsets, cursor, tile_e, max_tiles, ntile[0:1], ntile[1:2],
+                    pair_dst)
         # expert weights of this layer as block-scaled FP8: [El, 2I, d] (w1 | w3) and [El, d, I]
         def convert(w13, s13, w2, s2):
             native.call("tf_mxfp4_to_fp8_block", L.ew1, L.es1, w13, s13, El, I, d, 0, 2 * I)

@@ -52,6 +52,22 @@ def gemm(a_q: torch.Tensor, sfa: torch.Tensor, b_q: torch.Tensor, sfb: torch.Ten
                 sfb.shape[1], out, out.stride(0), okind, M, N, K, tile_expert, num_m_tiles, tile_rows, status)
 
 
+def expert_tile_rows(pairs: int, experts: int) -> int:
+    """Largest rows of an expert's tile (a multiple of 32): twice the rows an expert gets on average, so that nearly every
+    expert fits one tile and its weights are fetched once, up to the 256 columns of the instruction.  Small tiles leave
+    shared memory for more stages of weights."""
+    return min(256, max(32, -(-2 * pairs // (32 * experts)) * 32))
+
+
+def gemm_experts(a_q, sfa, w, w_2, s, s_2, b_rows, out, M, N, K, tiles, status) -> None:
+    """Rows of experts x their MXFP4 matrices as stored (``w_2``: a second matrix, its columns behind the first's);
+    ``tiles`` = (expert, first row, rows, number of tiles, largest rows of a tile, room for tiles)."""
+    tile_e, tile_r0, tile_r, num, tile_max, max_tiles = tiles
+    okind = {torch.float32: 0, torch.bfloat16: 2}[out.dtype]
+    native.call("tf_gemm_mx_experts", a_q, sfa, sfa.shape[1], w, w_2, s, s_2, b_rows, out, out.stride(0), okind, M, N, K,
+                tile_e, tile_r0, tile_r, num, tile_max, max_tiles, status)
+
+
 def units_to_rowmajor(sf: torch.Tensor, rows: int) -> torch.Tensor:
     """Inverse of the unit layout (tests, debugging): -> ``[rows, K/32]`` uint8."""
     kb, units, _ = sf.shape
