@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) sparse_attn_tc_kernel(AttnParam
     }
   } else if (warp == kTcProd + 2) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc = tc::instr_desc(0, 0, 128, 128);      // f16 x f16, M 128, N 128, both K-major
       constexpr uint32_t idesc_pv = idesc | (1u << 16);               // B (the key tile as V) MN-major
       int it = 0, n_row = 0;

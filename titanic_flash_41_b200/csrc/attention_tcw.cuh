@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kTwThreads, 1) sparse_attn_tcw_kernel(AttnPara
     }
   } else if (warp == kTwProd + 4) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_qk = tc::instr_desc(0, 0, 128, 64);
       constexpr uint32_t idesc_pv = idesc_qk | (1u << 15);            // A (the key tile as V^T) MN-major
       int it = 0, n_row = 0;

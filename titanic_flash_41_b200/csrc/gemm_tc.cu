@@ -229,7 +229,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tc::prefetch_tmap(&mapA);
       tc::prefetch_tmap(&mapB);
       int it = 0;
@@ -268,7 +268,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc = (KIND == 0) ? tc::instr_desc(1, 1, BM, BN) : tc::instr_desc(0, 0, BM, BN);
       int it = 0, grp = 0;
       bool ok = true;

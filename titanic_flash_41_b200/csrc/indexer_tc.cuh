@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kItThreads, 1) index_score_tc_kernel(ScorePara
       const ItItem it = get(item);
       if (it.tiles == 0) continue;
       const int qb = n_item & 1;
-      if (lane == 0) {
+      if (tc::elect_one()) {
         ok = tc::mbar_wait(q_ready(qb), (n_item >> 1) & 1, abort_flag);
         for (int t = 0; t < it.tiles && ok; ++t) {
           const int s = (kt + t) & 1;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kItThreads, 1) index_score_tc_kernel(ScorePara
         }
         if (ok) tc::mma_commit(q_free(qb));
       }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      ok = __all_sync(0xffffffffu, ok);
       kt += it.tiles;
       ++n_item;
     }

@@ -160,7 +160,7 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap mapW1, const __grid_constant__
   const int items = *p.n_groups * tiles_n;
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tc::prefetch_tmap(&mapW1);
       if (DUAL) tc::prefetch_tmap(&mapW3);
       tc::prefetch_tmap(&mapX);
@@ -210,7 +210,7 @@ moe_mx_kernel(const __grid_constant__ CUtensorMap mapW1, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int it = 0, sfit = 0, n_item = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++n_item) {

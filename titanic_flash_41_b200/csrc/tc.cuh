@@ -164,6 +164,9 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// One thread of a converged warp, for the roles that issue copies and MMAs.  Not `lane == 0`: there the compiler cannot know
+// that one lane is active and wraps every instruction with uniform operands in a loop over the lanes that might be; a TMA copy
+// or an MMA then takes 100 - 150 cycles to issue instead of about 25.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

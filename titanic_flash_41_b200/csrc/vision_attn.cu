@@ -124,7 +124,7 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
   if (warp == 5) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tc::mbar_expect_tx(q_full, kTileBytes);
       tc::tma_load_2d(q_s, &mapQ, 0, hrow + row0, q_full);
       for (int j = 0; j < tiles; ++j) {
@@ -140,7 +140,7 @@ vis_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_qk = tc::instr_desc(1, 1, 128, 128);
       constexpr uint32_t idesc_pv = tc::instr_desc(1, 1, 128, 64) | (1u << 16);       // B MN-major
       auto qk = [&](int j) -> bool {
