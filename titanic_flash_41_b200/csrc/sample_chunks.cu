@@ -37,6 +37,8 @@ namespace {
 
 constexpr int kChunkMax = 16384;
 constexpr int kThreads = 1024;
+constexpr int kUnroll = 4;                   // elements of a thread in flight; the staged chunk is padded to whole rounds of them
+constexpr int kHistCopies = 8;                // histograms of the lower digits, one for four warps
 constexpr int kMaxP = 16;          // chunks per row
 constexpr int kMaxG = 15;          // proposals per conversation
 constexpr double kFix = 1099511627776.0;     // 2^40
@@ -148,8 +150,9 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
   tf_pdl_sync();
   extern __shared__ __align__(16) unsigned char smem[];
   float* tbuf = reinterpret_cast<float*>(smem);
-  float* dbuf = tbuf + p.chunk;
-  unsigned long long* whist = reinterpret_cast<unsigned long long*>(dbuf + p.chunk);   // [32][256]
+  const int padded = (p.chunk + kThreads * kUnroll - 1) / (kThreads * kUnroll) * (kThreads * kUnroll);
+  float* dbuf = tbuf + padded;
+  unsigned long long* whist = reinterpret_cast<unsigned long long*>(dbuf + padded);    // [32][256]
   __shared__ unsigned long long gpart[4][256], fb[256], wtot[8];
   __shared__ double wm[32], cm[(kMaxG + 1) * kMaxP], Rrow[kMaxG + 1], wrow[kMaxG + 1], ptq[2 * kMaxG];
   __shared__ float redf[32];
@@ -190,6 +193,24 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
     *reinterpret_cast<float4*>(tbuf + k) = *reinterpret_cast<const float4*>(trow + k);
     if (has_d) *reinterpret_cast<float4*>(dbuf + k) = *reinterpret_cast<const float4*>(drow + k);
   }
+  // Padding: no mass in any sum below.  With whole rounds the loops run unrolled to their end; a last round of fewer elements
+  // ran one element at a time, each waiting for the one before.
+  for (int k = n + threadIdx.x; k < padded; k += kThreads) {
+    tbuf[k] = -INFINITY;
+    if (has_d) dbuf[k] = -INFINITY;
+  }
+  // the proposal's logits, if this chunk owns it: requested now, used in step 3
+  const long base = (long)part * n;
+  int prop = -1;
+  float t_prop = 0.f, d_prop = 0.f;
+  if (g > 0 && i < g && threadIdx.x == 0) {
+    const int x = p.proposals[s * g + i];
+    if (x >= base && x < base + n) {
+      prop = x;
+      t_prop = trow[x - base];
+      if (has_d) d_prop = drow[x - base];
+    }
+  }
   __syncthreads();
   // IEEE reciprocal (not the fast-math approximation): every kernel and the host agree on 1 / T bit for bit
   const float inv_t = __frcp_rn(p.sess_temp[s]);
@@ -198,9 +219,10 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
   // ---- 1. row maximum
   float m = -INFINITY;
   int bad = 0;
-  for (int k = threadIdx.x; k < n; k += kThreads) {
+#pragma unroll kUnroll
+  for (int k = threadIdx.x; k < padded; k += kThreads) {
     const float v = tbuf[k];
-    if (!(v < INFINITY) || isnan(v)) bad = 1;
+    if (!(v < INFINITY)) bad = 1;                          // (a NaN fails the comparison)
     m = fmaxf(m, v);
   }
   m = warp_max(m);
@@ -241,7 +263,8 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
   for (int level = 0; level < levels; ++level) {
     const int shift = 24 - 8 * level;
     const unsigned int tag = tag0 + 1 + level;
-    for (int k = threadIdx.x; k < 32 * 256; k += kThreads) whist[k] = 0;
+    const int words = (level == 0 ? 32 : kHistCopies) * 256;
+    for (int k = threadIdx.x; k < words; k += kThreads) whist[k] = 0;
     if (threadIdx.x < 256) fb[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t prefix = s_prefix, mask = s_mask;
@@ -259,10 +282,13 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
       };
       auto bin_of = [&](int cls) -> int { return !pos ? top - cls : cls < 4 ? top - cls : cls - top + 250; };
       unsigned long long* priv = whist + warp * 256 + lane;            // [class][lane]
-      for (int k = threadIdx.x; k < n; k += kThreads) {
+#pragma unroll kUnroll
+      for (int k = threadIdx.x; k < padded; k += kThreads) {
         const float v = tbuf[k];
         const int bin = (int)(fkey(v) >> 24), cls = class_of(bin);
-        const unsigned long long mass = (unsigned long long)((double)expf((v - stat.m) * inv_t) * kFix);
+        const float e = expf((v - stat.m) * inv_t);
+        const unsigned long long mass = (unsigned long long)((double)e * kFix);
+        if (!has_d) dbuf[k] = e;                         // (step 4 reads the weights back where no draft row is staged)
         if (cls >= (pos && bin < 128 ? 4 : 0) && cls < 8) priv[cls * 32] += mass;
         else if (mass) atomicAdd(&fb[bin], mass);
       }
@@ -283,26 +309,28 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
       // added up privately and touches shared memory once
       int cur = -1;
       unsigned long long run = 0;
-      for (int k = threadIdx.x; k < n; k += kThreads) {
+      unsigned long long* copy = whist + (warp % kHistCopies) * 256;
+#pragma unroll kUnroll
+      for (int k = threadIdx.x; k < padded; k += kThreads) {
         const float v = tbuf[k];
         const uint32_t key = fkey(v);
         if ((key & mask) != prefix) continue;
         const int bin = (key >> shift) & 255;
-        const unsigned long long mass = (unsigned long long)((double)expf((v - stat.m) * inv_t) * kFix);
         if (bin != cur) {
-          if (cur >= 0) atomicAdd(&whist[warp * 256 + cur], run);
+          if (cur >= 0) atomicAdd(&copy[cur], run);
           cur = bin;
           run = 0;
         }
-        run += mass;
+        run += (unsigned long long)((double)expf((v - stat.m) * inv_t) * kFix);
       }
-      if (cur >= 0) atomicAdd(&whist[warp * 256 + cur], run);
+      if (cur >= 0) atomicAdd(&copy[cur], run);
       __syncthreads();
     }
     if (threadIdx.x < 256) {
       unsigned long long acc = fb[threadIdx.x];
       if (level > 0)
-        for (int w = 0; w < 32; ++w) acc += whist[w * 256 + threadIdx.x];
+#pragma unroll
+        for (int w = 0; w < kHistCopies; ++w) acc += whist[w * 256 + threadIdx.x];
       push2(p, A.hist + ((((long)(level & 1) * P + part) * p.max_rows + row) * 256 + threadIdx.x) * 2, (uint32_t)acc,
             (uint32_t)(acc >> 32), tag);
     }
@@ -383,21 +411,17 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
   if (threadIdx.x == 0 && lc == 0) p.tstat[ez * p.emu_stat + (long)row * p.stat_stride] = stat;
 
   // ---- 3. probabilities of the proposals (published by the chunk that owns the token)
-  const long base = (long)part * n;
   RowStat ds;
   float d_inv = inv_t;
   ds.m = 0.f; ds.thr = 0; ds.z = 1.0;
   if (has_d && p.dstat) ds = p.dstat[s * g + i];
   if (g > 0) {
-    if (i < g && threadIdx.x == 0) {
-      const int x = p.proposals[s * g + i];
-      if (x >= base && x < base + n) {
-        const double pt = prob_of(tbuf[x - base], stat, inv_t);
-        const double q = (point || !has_d) ? 1.0 : prob_of(dbuf[x - base], ds, d_inv);
-        const long w0 = A.prop + ((long)par * p.max_rows + row) * 4;
-        push_double(p, w0, pt, tag0 + 5);
-        push_double(p, w0 + 2, q, tag0 + 5);
-      }
+    if (prop >= 0) {
+      const double pt = prob_of(t_prop, stat, inv_t);
+      const double q = (point || !has_d) ? 1.0 : prob_of(d_prop, ds, d_inv);
+      const long w0 = A.prop + ((long)par * p.max_rows + row) * 4;
+      push_double(p, w0, pt, tag0 + 5);
+      push_double(p, w0 + 2, q, tag0 + 5);
     }
     if (threadIdx.x < 2 * g) {
       const int j = threadIdx.x >> 1, h = threadIdx.x & 1;
@@ -426,26 +450,29 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
   const int point_tok = (i < gs && point) ? p.proposals[s * g + i] : -1;
   auto residual = [&](int k) -> double {
     const float l = tbuf[k];
-    double val = fkey(l) >= stat.thr ? wz * (double)expf((l - stat.m) * inv_t) : 0.0;
-    if (qz > 0.0) {
+    if (has_d) {
+      double val = fkey(l) >= stat.thr ? wz * (double)expf((l - stat.m) * inv_t) : 0.0;
       const float d = dbuf[k];
       if (fkey(d) >= ds.thr) val -= qz * (double)expf((d - ds.m) * d_inv);
-    } else if (base + k == point_tok) {
-      val -= 1.0;
+      return val > 0.0 ? val : 0.0;
     }
+    double val = fkey(l) >= stat.thr ? wz * (double)(levels ? dbuf[k] : expf((l - stat.m) * inv_t)) : 0.0;
+    if (base + k == point_tok) val -= 1.0;
     return val > 0.0 ? val : 0.0;
   };
   double my_mass = 0.0;
-  for (int k = threadIdx.x; k < n; k += kThreads) my_mass += residual(k);
+#pragma unroll kUnroll
+  for (int k = threadIdx.x; k < padded; k += kThreads) my_mass += residual(k);
   double wsum = my_mass;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
   if (lane == 0) wm[warp] = wsum;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < 32; ++w) t += wm[w];
-    push_double(p, A.mass + (((long)par * P + part) * p.max_rows + row) * 2, t, tag0 + 6);
+  if (warp == 0) {
+    double t = wm[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) push_double(p, A.mass + (((long)par * P + part) * p.max_rows + row) * 2, t, tag0 + 6);
   }
   if (threadIdx.x < R1 * P) {
     const int ii = threadIdx.x / P, q = threadIdx.x % P;
@@ -487,27 +514,32 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
 
   // ---- 5. the chunk that holds the draw finds the token: warp, lane, element
   if (i == tau && part == s_chunk) {
-    if (threadIdx.x == 0) {
-      double before = 0.0;
-      int w = 0;
-      for (; w < 31; ++w) {
-        if (before + wm[w] > s_draw) break;
-        before += wm[w];
+    // (prefix sums over the lanes: an fp64 addition takes about eighty cycles here, walks of 31 warps and 16 elements 8,000)
+    auto prefix = [&](double x) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double up = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += up;
       }
+      return x;
+    };
+    if (warp == 0) {
+      const double mass_w = wm[lane], upto = prefix(mass_w), draw = s_draw;
+      const unsigned int over = __ballot_sync(0xffffffffu, upto > draw), some = __ballot_sync(0xffffffffu, mass_w > 0.0);
+      int w = over ? __ffs(over) - 1 : 31;
       // rounding can leave the draw past the last positive warp: step back to one that has mass
-      while (w > 0 && !(wm[w] > 0.0)) --w;
-      s_warp = w;
-      s_draw -= before;
+      const unsigned int up_to_w = some & (0xffffffffu >> (31 - w));
+      w = up_to_w ? 31 - __clz(up_to_w) : 0;
+      const double before = __shfl_sync(0xffffffffu, upto - mass_w, w);
+      if (lane == 0) {
+        s_warp = w;
+        s_draw = draw - before;
+      }
     }
     __syncthreads();
     if (warp == s_warp) {
       // inclusive scan of the lane masses in lane order
-      double incl = my_mass;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
+      const double incl = prefix(my_mass);
       const double excl = incl - my_mass, draw = s_draw;
       const bool hit = my_mass > 0.0 && excl <= draw && draw < incl;
       unsigned int hits = __ballot_sync(0xffffffffu, hit);
@@ -517,21 +549,14 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
         hits = pos ? (1u << (31 - __clz(pos))) : 1u;
       }
       const int winner = __ffs(hits) - 1;
+      // the winner's elements (at most sixteen), one a lane, in its order
+      const int k_own = (warp * 32 + winner) + lane * kThreads;
+      const double val = k_own < n ? residual(k_own) : 0.0;
+      const double rest = __shfl_sync(0xffffffffu, draw - excl, winner);
+      const unsigned int past = __ballot_sync(0xffffffffu, prefix(val) > rest && val > 0.0), with = __ballot_sync(0xffffffffu, val > 0.0);
+      const int el = past ? __ffs(past) - 1 : 31 - __clz(with);            // (none past the draw: the last that has mass)
       if (lane == winner) {
-        double rest = draw - excl, acc = 0.0;
-        int tok = -1, last_pos = -1;
-        for (int k = threadIdx.x; k < n; k += kThreads) {
-          const double v = residual(k);
-          if (v > 0.0) {
-            last_pos = k;
-            if (acc + v > rest) {
-              tok = k;
-              break;
-            }
-            acc += v;
-          }
-        }
-        if (tok < 0) tok = last_pos;
+        int tok = with ? warp * 32 + winner + el * kThreads : -1;
         if (tok < 0) {
           tf_report(p.st, TF_NONFINITE, 24, s, tau);
           tok = 0;
@@ -601,7 +626,7 @@ TF_API int tf_sample_chunks(const float* tlogits, const float* dlogits, const vo
   p.tok_stride = tok_stride; p.peers = (const unsigned long long*)peers; p.world = world; p.rank = rank;
   p.max_rows = max_rows; p.ctr = (unsigned int*)ctr; p.spin_limit = spin_limit; p.st = (TfStatusWord*)status;
   p.emu_tl = emu_tl; p.emu_dl = emu_dl; p.emu_stat = emu_stat; p.emu_tok = emu_tok; p.emu_acc = emu_acc;
-  const size_t dyn = (size_t)chunk * 8 + 32 * 256 * 8;
+  const size_t dyn = (size_t)((chunk + kThreads * kUnroll - 1) / (kThreads * kUnroll) * (kThreads * kUnroll)) * 8 + 32 * 256 * 8;
   static unsigned long long limit_set = 0;
   const cudaError_t e = tf_smem_limit_all((const void*)sample_chunks_kernel, &limit_set);
   if (e != cudaSuccess) return (int)e;
