@@ -110,3 +110,19 @@ def _rs_case(M, N, K):
         torch.cuda.synchronize()
         st.check()
         assert _rel(out, a.float() @ b.float().t()) < 5e-3
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 1088), (33, 384, 2048), (257, 128, 1088), (1300, 1152, 1152), (2049, 256, 1088)])
+def test_bf16_by_pairs_of_sms(M, N, K):
+    """Rows and feature blocks that end inside a pair's tile (one CTA's 128 features or fewer rows than a tile), both output
+    types, rows beyond M and columns beyond N untouched: exact products, fp32 sums (2e-5; bf16 rounding 4e-3)."""
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = (torch.randn(r, K, device="cuda", generator=gen).bfloat16() for r in (M, N))
+    want = a.double() @ b.double().t()
+    st = native.StatusWord("cuda")
+    for dt, ok, tol in ((torch.float32, 0, 2e-5), (torch.bfloat16, 2, 4e-3)):
+        c = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=dt)
+        native.call("tf_gemm_tc", 0, a, K, b, K, c, N + 8, M, N, K, None, 0, None, 0, ok, None, None, 0, st.t)
+        st.check()
+        assert float((c[:M, :N].double() - want).norm() / want.norm()) < tol
+        assert bool((c[:, N:] == 7.0).all()) and bool((c[M] == 7.0).all())

@@ -48,6 +48,10 @@
 // Every mbarrier wait is bounded: on a time-out the CTA raises its abort flag, reports TF_TIMEOUT, lets
 // copies in flight land, frees its tensor memory and returns.
 //
+// The same kernel without scales (MX = 0) multiplies bf16 x bf16 (64 k a block, the vision tower and the router logits of
+// gemm_tc.cu): warp 2 only passes on that its CTA's operands have landed, and two accumulators always fit.
+// 8192^3: 1.59 PFLOP/s (1.35 by the one-SM form of gemm_tc.cu).
+//
 // Reference behaviour: block-scaled dense and expert GEMMs of the prefill path
 // (src/blockscaled.rs:21-87 scale format; src/fp8_linear.rs:122 call site; the b12x
 // `gemm.dense` / `moe.grouped` bundles).
@@ -55,6 +59,7 @@
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 
+#include "gemm_pair.h"
 #include "tc.cuh"
 
 namespace {
@@ -148,6 +153,13 @@ __device__ __forceinline__ void mma_mx(uint32_t tmem_d, uint64_t da, uint64_t db
       ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
       : "memory");
 }
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // block-scaled instruction descriptor: A (the weights) e4m3 (0) or e2m1 (5), B (the rows) e4m3, both K-major, UE8M0 scales,
 // M = 256; + `sf` in both scale-id fields: which byte of the 32-bit scale columns this 32-k step uses
 __device__ __forceinline__ uint32_t idesc_mx(uint32_t afmt, uint32_t rows) {
@@ -161,7 +173,7 @@ struct MxTile {
   int mat;
 };
 
-template <int OUT_F32>
+template <int OUT_F32, int MX>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW,
                const __grid_constant__ CUtensorMap mapW2, const __grid_constant__ CUtensorMap mapS,
@@ -187,13 +199,14 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)pair_rank();
-  const int kblocks = p.K / BK;
+  constexpr int BKE = MX ? BK : 64;                        // elements of a 128-byte k block
+  const int kblocks = p.K / BKE;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
-      tc::mbar_init(full(s), 2);
+      tc::mbar_init(full(s), MX ? 2 : 1);
       tc::mbar_init(empty(s), 1);
-      tc::mbar_init(sf_full(s), 8);
+      tc::mbar_init(sf_full(s), MX ? 8 : 2);
     }
     for (int b = 0; b < 2; ++b) {
       tc::mbar_init(tfull(b), 1);
@@ -268,9 +281,9 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
           if (!(ok = tc::mbar_wait(empty(s), ph ^ 1, abort_flag))) break;
           tc::mbar_expect_tx(full(s), tx);
           const uint32_t sa = base + s * stage_bytes, sx = sa + 128 * 128;
-          tc::tma_load_2d(sa, mw, kb * BK, t.wrow, full(s));
-          tc::tma_load_2d(sx, &mapX, kb * BK, xrow, full(s));
-          for (int i = 1; i < loads; ++i) tc::tma_load_2d(sx + i * box_bytes, &mapX, kb * BK, xrow + i * p.box_rows, full(s));
+          tc::tma_load_2d(sa, mw, kb * BKE, t.wrow, full(s));
+          tc::tma_load_2d(sx, &mapX, kb * BKE, xrow, full(s));
+          for (int i = 1; i < loads; ++i) tc::tma_load_2d(sx + i * box_bytes, &mapX, kb * BKE, xrow + i * p.box_rows, full(s));
           if (++s == stages) { s = 0; ph ^= 1; }
         }
       }
@@ -286,7 +299,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
     }
   } else if (warp == kThreads / 32 - 1) {
     // ------------------------------------------------------------------ TMA producer: scales
-    if (tc::elect_one()) {
+    if (MX && tc::elect_one()) {
       int s = 0, b = 0;
       uint32_t ph = 0, bph = 0;
       bool ok = true;
@@ -333,7 +346,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       uint32_t ph = 0, aph = 0;
       bool ok = true;
       for (int item = first; item < items && ok; item += step) {
-        const uint32_t id = idesc_mx(p.b_fp4 ? 5u : 0u, (uint32_t)tile_of(item).n);
+        const uint32_t n = (uint32_t)tile_of(item).n, id = MX ? idesc_mx(p.b_fp4 ? 5u : 0u, n) : tc::instr_desc(1, 1, BF, n);
         const uint32_t td = tmem_base + ab * p.tile_n;
         if (!(ok = tc::mbar_wait(tempty(ab), aph ^ 1, abort_flag))) break;
         for (int kb = 0; kb < kblocks; ++kb) {
@@ -345,14 +358,29 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
           const uint64_t da = tc::smem_desc_sw128(sa), db = tc::smem_desc_sw128(sa + 128 * 128);
           const uint32_t sfw = sf_base + s * kSfCols, sfx = sfw + 4;
 #pragma unroll
-          for (uint32_t k = 0; k < 4; ++k)
-            mma_mx(td, da + 2 * k, db + 2 * k, id | (k << 4) | (k << 29), sfw, sfx, (kb | k) ? 1u : 0u);
+          for (uint32_t k = 0; k < 4; ++k) {
+            if (MX) mma_mx(td, da + 2 * k, db + 2 * k, id | (k << 4) | (k << 29), sfw, sfx, (kb | k) ? 1u : 0u);
+            else mma_bf16(td, da + 2 * k, db + 2 * k, id, (kb | k) ? 1u : 0u);
+          }
           commit_pair(empty(s));             // frees the stage and, with it, the stage's scale columns
           if (++s == stages) { s = 0; ph ^= 1; }
         }
         if (ok) commit_pair(tfull(ab));
         if (++ab == p.bufs) { ab = 0; aph ^= 1; }
       }
+    }
+  } else if (!MX && warp < 6) {
+    // ------------------------------------------------------------------ this CTA's operands have landed: passed on
+    if (warp == 2 && tc::elect_one()) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int item = first; item < items && ok; item += step)
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!(ok = tc::mbar_wait(full(s), ph, abort_flag))) break;
+          arrive_first(sf_full(s));
+          if (++s == stages) { s = 0; ph ^= 1; }
+        }
     }
   } else if (warp < 6) {
     // ------------------------------------------------------------------ scale movers
@@ -474,7 +502,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) tf_report(p.status, TF_TIMEOUT, 140, blockIdx.x, p.b_fp4);
+  if (*abort_flag && threadIdx.x == 0) tf_report(p.status, TF_TIMEOUT, MX ? 140 : 141, blockIdx.x, p.b_fp4);
   pair_sync();                                 // nobody leaves while the other CTA may still arrive at its barriers
   if (warp == 1) {
     tc::tc_fence_after();
@@ -739,6 +767,7 @@ inline int dense_rows(int M, int fbs, int pairs, int b_fp4) {
 }
 
 struct MxCall {
+  int mx;                    // 0: bf16 x bf16
   const void *A, *B, *B2;
   long lda, ldb, b_rows;
   int b_fp4, sfa_units, sfb_units, sf_rows;
@@ -755,9 +784,10 @@ int launch_mx(const MxCall& a, void* status, cudaStream_t st) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  auto kernel = a.out_kind == 0 ? gemm_mx_kernel<1> : gemm_mx_kernel<0>;
-  static unsigned long long limit_set[2] = {0, 0};
-  if (tf_smem_limit((const void*)kernel, kSmemMax, &limit_set[a.out_kind == 0]) != cudaSuccess) return -2;
+  auto kernel = a.mx ? (a.out_kind == 0 ? gemm_mx_kernel<1, 1> : gemm_mx_kernel<0, 1>)
+                     : (a.out_kind == 0 ? gemm_mx_kernel<1, 0> : gemm_mx_kernel<0, 0>);
+  static unsigned long long limit_set[4] = {0, 0, 0, 0};
+  if (tf_smem_limit((const void*)kernel, kSmemMax, &limit_set[(a.out_kind == 0) + 2 * (a.mx != 0)]) != cudaSuccess) return -2;
   const int pairs = g_sms / 2, mats = a.B2 ? 2 : 1, fbs = (a.N + BF - 1) / BF * mats;
   MxGemmParams p;
   p.tile_n = a.tile_expert ? (a.tile_max + 31) / 32 * 32 : dense_rows(a.M, fbs, pairs, a.b_fp4);
@@ -768,12 +798,14 @@ int launch_mx(const MxCall& a, void* status, cudaStream_t st) {
   p.sf_kind = !a.sf_rows ? 0 : a.K / 32 % 16 == 0 ? 1 : 2;
   const int room = kSmemMax - 1024 - kTailBytes - (p.sf_kind ? kSfSlots * kSfSlotBytes : 0);
   p.stages = room / p.stage_bytes < kMaxStages ? room / p.stage_bytes : kMaxStages;
-  p.bufs = 2 * p.tile_n + p.stages * kSfCols <= kTmemCols ? 2 : 1;
+  p.bufs = 2 * p.tile_n + (a.mx ? p.stages * kSfCols : 0) <= kTmemCols ? 2 : 1;
   CUtensorMap mX, mW, mW2, mS, mS2, mSo, mSo2;
-  if (!tc::make_map_2d(&mX, a.A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.M, a.K, a.lda, p.box_rows)) return -4;
+  const CUtensorMapDataType dt = a.mx ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const int es = a.mx ? 1 : 2;
+  if (!tc::make_map_2d(&mX, a.A, dt, es, a.M, a.K, a.lda, p.box_rows)) return -4;
   auto weights = [&](CUtensorMap* m, const void* B) {
     return a.b_fp4 ? a.ldb == a.K / 2 && make_map_fp4(m, B, a.b_rows, a.K)
-                   : tc::make_map_2d(m, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.b_rows, a.K, a.ldb, 128);
+                   : tc::make_map_2d(m, B, dt, es, a.b_rows, a.K, a.ldb, 128);
   };
   if (!weights(&mW, a.B) || (a.B2 && !weights(&mW2, a.B2))) return -4;
   if (!a.B2) mW2 = mW;
@@ -800,6 +832,14 @@ int launch_mx(const MxCall& a, void* status, cudaStream_t st) {
 
 }  // namespace
 
+int tf_gemm_pair_bf16(const void* A, long lda, const void* B, long ldb, void* C, int ldc, int out_kind, int M, int N, int K,
+                      void* status, cudaStream_t st) {
+  MxCall a = {};
+  a.A = A; a.B = B; a.lda = 2 * lda; a.ldb = 2 * ldb; a.b_rows = N;
+  a.C = C; a.ldc = ldc; a.out_kind = out_kind; a.M = M; a.N = N; a.K = K;
+  return launch_mx(a, status, st);
+}
+
 // Scale units needed for `rows` rows that tiles of `tile_rows` rows may touch (whole tiles).
 TF_API long tf_mx_sf_units(long rows, int tile_rows) {
   return (rows + tile_rows - 1) / tile_rows * tile_rows / 32;
@@ -823,7 +863,7 @@ TF_API int tf_gemm_mx_rows(const void* A, long lda, const void* B, long ldb, lon
   if (sfb_units < (tile_expert ? b_rows / 32 : f_tiles * (BF / 32))) return -1;
   if ((reinterpret_cast<uintptr_t>(sfa) & 15) || (reinterpret_cast<uintptr_t>(sfb) & 15)) return -1;
   if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc * (out_kind == 0 ? 4 : 2)) % 16) return -1;
-  const MxCall a = {A, B, nullptr, lda, ldb, b_rows, b_fp4, sfa_units, sfb_units, 0, sfa, sfb, nullptr, C, ldc, out_kind,
+  const MxCall a = {1, A, B, nullptr, lda, ldb, b_rows, b_fp4, sfa_units, sfb_units, 0, sfa, sfb, nullptr, C, ldc, out_kind,
                     M, N, K, tile_expert, nullptr, tile_expert ? tile_rows : nullptr, num_m_tiles, 128, (int)m_tiles};
   return launch_mx(a, status, st);
 }
@@ -841,7 +881,7 @@ TF_API int tf_gemm_mx_experts(const void* A, const void* sfa, int sfa_units, con
   if (tile_max < 1 || tile_max > kMaxRows || max_tiles < 1 || M % 32 || sfa_units < M / 32) return -1;
   if (reinterpret_cast<uintptr_t>(sfa) & 15) return -1;
   if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc * (out_kind == 0 ? 4 : 2)) % 16) return -1;
-  const MxCall a = {A, B, B2, K, K / 2, b_rows, 1, sfa_units, 0, 1, sfa, sb, sb2, C, ldc, out_kind,
+  const MxCall a = {1, A, B, B2, K, K / 2, b_rows, 1, sfa_units, 0, 1, sfa, sb, sb2, C, ldc, out_kind,
                     M, N, K, tile_expert, tile_row0, tile_rows, num_tiles, tile_max, max_tiles};
   return launch_mx(a, status, st);
 }

@@ -17,6 +17,7 @@
 //
 // Replaces for the B200 build: the b12x `gemm.dense` / FlashInfer MXFP8 bundles and the cuBLAS
 // GemmEx calls of the reference (src/fp8_linear.rs:122, src/blas.rs:24).
+#include "gemm_pair.h"
 #include "tc.cuh"
 
 namespace {
@@ -530,14 +531,21 @@ TF_API int tf_gemm_tc(int kind, const void* A, long lda, const void* B, long ldb
   if (out_kind != 0 && out_kind != 2) return -1;
   if ((out_kind == 0 ? ldc % 4 : ldc % 8) != 0) return -1;
   if (kind == 2 && (!sa || !sb)) return -1;
-  CUtensorMap ma, mb;
-  const int es = kind == 0 ? 2 : 1;
-  const CUtensorMapDataType dt = kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   if (!g_sms) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   }
+  // bf16 matrices by pairs of SMs: 8192^3 812 -> 691 us (1.59 PFLOP/s), 8580 x 8192 x 1024 137 -> 99, 16384 x 256 x 4096 64 -> 44.
+  // A short K over no more 128 x 128 tiles than SMs stays here: setting a pair up costs more than it saves
+  // (1521 x 1024 x 1024 13.2 us here, 15.2 by pairs; x 640 12.3 and 14.3; at K 4096 both 24.6), and so do the forms that the
+  // pair kernel does not have (experts, reduce-scatter, all-gather).
+  const bool small = K <= 1024 && (long)((M + BM - 1) / BM) * (N / 128) <= g_sms;
+  if (kind == 0 && experts <= 0 && !g_rs.peers && !g_ag.peers && g_force_bn == 0 && !small)
+    return tf_gemm_pair_bf16(A, lda, B, ldb, C, ldc, out_kind, M, N, K, status, stream);
+  CUtensorMap ma, mb;
+  const int es = kind == 0 ? 2 : 1;
+  const CUtensorMapDataType dt = kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   // 128x256 tiles once they still fill the machine; 128x128 otherwise
   const int BN = (N % 256 == 0 && (long)((M + BM - 1) / BM) * (N / 256) >= g_sms && g_force_bn != 128) ? 256 : 128;
   if (!tc::make_map_2d(&ma, A, dt, es, M, K, (uint64_t)lda * es, BM)) return -2;
