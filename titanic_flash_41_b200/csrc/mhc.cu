@@ -155,14 +155,17 @@ __global__ void __launch_bounds__(256) hc_prepare_kernel(const __nv_bfloat16* __
 // [c w, c w + w) of EVERY residual copy: its part of the mixes, and afterwards its columns of the
 // collapsed and normalised rows, come from the one slice of x that it stages in shared memory, so x
 // is read from HBM once.  Partial mixes and sums of squares meet through distributed shared memory
-// (added in CTA order).  Warp q computes mixes 3q .. 3q + 2 of all R rows: a weight pair is loaded
-// once for R rows, two columns per packed fp32 FMA.
-//   R = 1   few rows (decode): bound by the latency of streaming fn (1.97 MB at 4 x 5120) from L2; eight
+// (added in CTA order).
+//   R = 1   warp q computes mixes 3q .. 3q + 2, two columns per packed fp32 FMA.  Few rows (decode): bound by the latency of streaming fn (1.97 MB at 4 x 5120) from L2; eight
 //           CTAs a row shorten the stream eightfold.  One CTA per row took 202 us for 24 rows; a decode
 //           step with 14 of these and 6 head collapses (then a chain of library calls): 10.1 -> 6.8 ms
-//   R = 16  many rows (prefill): fn crosses L2 once per 16 rows (one row per CTA moves 2 MB per row:
-//           1.14 ms for 4,001 rows; four of these, four tf_hc_post and one head of a prefill: 58.2 ->
-//           50.2 ms together with the scale re-ordering of csrc/gemm_mx.cu, 55.5 before)
+//   R = 16  many rows (prefill): fn crosses L2 once per 16 rows.  The mixes are a product of 16 rows by 24 mixes on the
+//           tensor cores (mma.sync, bf16): x is bf16, and an fp32 weight is the sum of three bf16 numbers (8 of
+//           its 24 bits each), so every product is exact as in an fp32 FMA and sums are fp32.  A warp takes every eighth
+//           step of 16 columns.  The Sinkhorn steps of a row (20 dependent pairs of sums and divisions) are done by
+//           one CTA of the cluster, two rows at once by one warp, while the others collapse.
+//           4,001 rows of 4 x 5,120: 440 us with packed fp32 FMAs and pieces loaded one by one, 240 so (mixes 24,000 of a CTA's
+//           58,000 cycles before the split by truncation and the walk without divisions); x alone takes 25 us.
 // HEAD: the collapse in front of the vocabulary head (H mixes, no post / comb) and the plain mean
 // of the copies.
 // ---------------------------------------------------------------------------------------------
@@ -176,6 +179,19 @@ __device__ __forceinline__ void fma_f2(unsigned long long& c, unsigned long long
 }
 __device__ __forceinline__ float2 bf2_to_f2(uint32_t u) {
   return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+__device__ __forceinline__ void mma_bf16_16816(float c[4], const uint32_t a[4], const uint32_t b[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// the upper halves of a pair as a bf16 pair (its first eight significant bits); v becomes what is left of it, exactly
+__device__ __forceinline__ uint32_t take_bf2(float2& v) {
+  const uint32_t x = __float_as_uint(v.x), y = __float_as_uint(v.y);
+  v.x -= __uint_as_float(x & 0xffff0000u);
+  v.y -= __uint_as_float(y & 0xffff0000u);
+  return __byte_perm(x, y, 0x7632);
 }
 
 struct HcArgs {
@@ -205,6 +221,8 @@ __global__ void __cluster_dims__(kHcCtas, 1, 1) __launch_bounds__(256) hc_cluste
   __shared__ float vv[R];
   const int H = p.H, d = p.d, w = p.w, n = H * d, nmix = HEAD ? H : H * (2 + H);
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(hc_smem);          // [R][H][w]
+  // (many rows: rows 16 bytes off a multiple of 128, so that the eight rows of a fragment load lie in different banks)
+  const int pitch = H * w + (R > 1 ? 8 : 0);
   const int c = (int)cluster.block_rank();
   const int row0 = (int)(blockIdx.x / kHcCtas) * R;
   const int c0 = c * w, wc = max(0, min(w, d - c0));
@@ -228,24 +246,18 @@ __global__ void __cluster_dims__(kHcCtas, 1, 1) __launch_bounds__(256) hc_cluste
     ss = warp_sum(ss);
     if (lane == 0) red[0][warp] = ss;
   } else {
+    // asynchronous copies: a warp's rows are all requested before any is waited for (loaded and stored one piece after another,
+    // the twenty pieces of a lane were twenty trips to HBM, half of the launch)
     for (int r = warp; r < R; r += 8) {
-      float ss = 0.f;
       const bool live = row0 + r < p.rows;
       for (int i = lane; i < H * w8; i += 32) {
         const int h = i / w8, k = (i - h * w8) * 8;
-        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-        if (live) raw = *reinterpret_cast<const uint4*>(p.x + (long)(row0 + r) * n + (long)h * d + c0 + k);
-        *reinterpret_cast<uint4*>(xs + (r * H + h) * w + k) = raw;
-        const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = bf2_to_f2(u[j]);
-          ss += f.x * f.x + f.y * f.y;
-        }
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(xs + r * pitch + h * w + k);
+        const __nv_bfloat16* src = p.x + (long)(live ? row0 + r : row0) * n + (long)h * d + c0 + k;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
       }
-      ss = warp_sum(ss);
-      if (lane == 0) part[r][kMaxMix] = ss;
     }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   if (R == 1 && threadIdx.x == 0) {
@@ -255,8 +267,8 @@ __global__ void __cluster_dims__(kHcCtas, 1, 1) __launch_bounds__(256) hc_cluste
     part[0][kMaxMix] = t;
   }
 
-  // ---- mixes 3 warp .. 3 warp + 2 over this CTA's columns
-  {
+  if (R == 1) {
+    // ---- mixes 3 warp .. 3 warp + 2 over this CTA's columns
     unsigned long long acc[3][R];
 #pragma unroll
     for (int m = 0; m < 3; ++m)
@@ -293,6 +305,106 @@ __global__ void __cluster_dims__(kHcCtas, 1, 1) __launch_bounds__(256) hc_cluste
           if (lane == 0 && q0 + m < nmix) part[r][q0 + m] = t;
         }
     }
+  } else {
+    // ---- mixes of the sixteen rows: A = rows, B = the three parts of fn; inside a step lane t of a quad takes columns
+    // 4t .. 4t + 3 of both (any order of the columns does, as long as it is the same one)
+    __shared__ float wpart[R > 1 ? 8 : 1][R][kCols];
+    float acc[3][4];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
+    const int g = lane >> 2, t4 = (lane & 3) * 4;
+    const int sh = (wc + 15) / 16, total = H * sh, tiles = (nmix + 7) / 8;
+    const int span = max(sh, 1) * 16;         // columns of a copy in whole steps (a CTA may have none)
+    struct Place {                            // of a step: copy and first column (walked, not divided out)
+      int h, i;
+    };
+    auto advance = [&](Place& q) {
+      q.i += 8 * 16;
+      while (q.i >= span) {
+        q.i -= span;
+        ++q.h;
+      }
+    };
+    Place ahead = {0, warp * 16}, at = ahead;
+    while (ahead.i >= span) {
+      ahead.i -= span;
+      ++ahead.h;
+    }
+    at = ahead;
+    const float* fn_row = p.fn + (long)g * n + c0 + t4;
+    auto load_fn = [&](float4 (&f)[3]) {
+      const float* src = fn_row + (long)ahead.h * d + ahead.i;
+      const bool on = ahead.h < H && ahead.i + t4 < wc;
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        f[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (on && m < tiles && m * 8 + g < nmix) f[m] = __ldg(reinterpret_cast<const float4*>(src + (long)(m * 8) * n));
+      }
+      advance(ahead);
+    };
+    constexpr int kAhead = 3;                 // steps of fn requested ahead
+    float4 ring[kAhead][3];
+    float ss0 = 0.f, ss1 = 0.f;               // sums of squares of rows g and g + 8 (every element passes through one lane)
+    const __nv_bfloat16* x_row = xs + g * pitch + t4;
+    auto step_of = [&](const float4 (&f)[3]) {
+      uint2 lo = make_uint2(0u, 0u), hi = lo;
+      if (at.i + t4 < wc) {
+        lo = *reinterpret_cast<const uint2*>(x_row + at.h * w + at.i);
+        hi = *reinterpret_cast<const uint2*>(x_row + 8 * pitch + at.h * w + at.i);
+      }
+      advance(at);
+      const uint32_t a[4] = {lo.x, hi.x, lo.y, hi.y};
+      const float2 q0 = bf2_to_f2(lo.x), q1 = bf2_to_f2(lo.y), q2 = bf2_to_f2(hi.x), q3 = bf2_to_f2(hi.y);
+      ss0 += (q0.x * q0.x + q0.y * q0.y) + (q1.x * q1.x + q1.y * q1.y);
+      ss1 += (q2.x * q2.x + q2.y * q2.y) + (q3.x * q3.x + q3.y * q3.y);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        if (m >= tiles) break;
+        float2 u = make_float2(f[m].x, f[m].y), v = make_float2(f[m].z, f[m].w);
+        uint32_t b[3][2];
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) {
+          b[piece][0] = take_bf2(u);
+          b[piece][1] = take_bf2(v);
+        }
+        // the step's sum from zero, smallest parts first, then one rounded fp32 addition: the tensor core truncates what it adds
+        // to its accumulator (all steps into one: pre at 20,480 columns 5.4e-7 from fp64; so 1.1e-7, fp32 FMAs 1.3e-7)
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int piece = 2; piece >= 0; --piece) mma_bf16_16816(d, a, b[piece]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][e] += d[e];
+      }
+    };
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) load_fn(ring[k]);
+    for (int step = warp; step < total; step += 8 * kAhead) {
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const float4 f[3] = {ring[k][0], ring[k][1], ring[k][2]};
+        load_fn(ring[k]);
+        if (step + 8 * k < total) step_of(f);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) wpart[warp][g + (e >> 1) * 8][m * 8 + (lane & 3) * 2 + (e & 1)] = acc[m][e];
+    ss0 += __shfl_xor_sync(0xffffffffu, ss0, 1);
+    ss1 += __shfl_xor_sync(0xffffffffu, ss1, 1);
+    ss0 += __shfl_xor_sync(0xffffffffu, ss0, 2);
+    ss1 += __shfl_xor_sync(0xffffffffu, ss1, 2);
+    if ((lane & 3) == 0) {
+      wpart[warp][g][kMaxMix] = ss0;
+      wpart[warp][g + 8][kMaxMix] = ss1;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < R * kCols; i += 256) {
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = (&wpart[q][0][0])[i];
+      (&part[0][0])[i] = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
   }
   cluster.sync();
   for (int i = threadIdx.x; i < R * kCols; i += 256) {
@@ -305,63 +417,68 @@ __global__ void __cluster_dims__(kHcCtas, 1, 1) __launch_bounds__(256) hc_cluste
   }
   __syncthreads();
 
-  // ---- coefficients: one warp per row; lane i * 4 + j of the first sixteen holds comb[i][j] (the
-  // other sixteen repeat them, so that every shuffle is by whole warps)
+  // ---- coefficients.  pre of every row in every CTA; post and comb of row r in CTA r % 8 (one row: in CTA 0).
   for (int r = warp; r < R; r += 8) {
     const float inv = rsqrtf(mix[r][kMaxMix] / n + p.rms_eps);
-    float pre = 0.f, post = 0.f;
-    if (lane < H) {
-      pre = 1.f / (1.f + expf(-(mix[r][lane] * inv * p.scale[0] + p.base[lane]))) + p.eps;
-      if (!HEAD) post = 2.f / (1.f + expf(-(mix[r][H + lane] * inv * p.scale[1] + p.base[H + lane])));
-      s_pre[r][lane] = pre;
-    }
-    if (!HEAD) {
-      const int i = (lane >> 2) & 3, j = lane & 3;
-      const bool on = i < H && j < H;
-      const int q = on ? 2 * H + i * H + j : 0;
-      const float m0 = on ? mix[r][q] * inv * p.scale[2] + p.base[q] : -1e30f;
-      float mx = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 1));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      float m = on ? expf(m0 - mx) : 0.f;
-      auto row_sum = [&](float v) {
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        return v + __shfl_xor_sync(0xffffffffu, v, 2);
-      };
-      auto col_sum = [&](float v) {
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        return v + __shfl_xor_sync(0xffffffffu, v, 8);
-      };
-      const float s0 = row_sum(m);
-      m = on ? m / s0 + p.eps : 0.f;
-      const float s1 = col_sum(m);
-      m = on ? m / (s1 + p.eps) : 0.f;
-      for (int it = 1; it < p.iters; ++it) {
-        const float sr = row_sum(m);
-        m = on ? m / (sr + p.eps) : 0.f;
-        const float sc = col_sum(m);
-        m = on ? m / (sc + p.eps) : 0.f;
-      }
-      if (c == 0 && row0 + r < p.rows) {
-        HcCoef* k = p.coef + row0 + r;
-        if (lane < H) {
-          k->pre[lane] = pre;
-          k->post[lane] = post;
-        }
-        if (lane < 16 && on) k->comb[i * kMaxH + j] = m;
-      }
-    }
+    if (lane < H) s_pre[r][lane] = 1.f / (1.f + expf(-(mix[r][lane] * inv * p.scale[0] + p.base[lane]))) + p.eps;
   }
   __syncthreads();
+  // The warp at the coefficients of many rows has nothing that the others wait for: it arrives at their barrier first.
+  const bool apart = R > 1 && !HEAD && warp == 7;
+  auto arrive = [&]() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); };
+  if (apart) arrive();
+  if (!HEAD && (R == 1 ? c == 0 && warp == 0 : warp == 7)) {
+    // lane i * 4 + j of a half warp holds comb[i][j]; the second half: the second row (one row: the same again, so that
+    // every shuffle is by whole warps)
+    const int r = R == 1 ? 0 : c + kHcCtas * (lane >> 4), hl = lane & 15;
+    const float inv = rsqrtf(mix[r][kMaxMix] / n + p.rms_eps);
+    float post = 0.f;
+    if (hl < H) post = 2.f / (1.f + expf(-(mix[r][H + hl] * inv * p.scale[1] + p.base[H + hl])));
+    const int i = hl >> 2, j = hl & 3;
+    const bool on = i < H && j < H;
+    const int q = on ? 2 * H + i * H + j : 0;
+    const float m0 = on ? mix[r][q] * inv * p.scale[2] + p.base[q] : -1e30f;
+    float mx = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    float m = on ? expf(m0 - mx) : 0.f;
+    auto row_sum = [&](float v) {
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      return v + __shfl_xor_sync(0xffffffffu, v, 2);
+    };
+    auto col_sum = [&](float v) {
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      return v + __shfl_xor_sync(0xffffffffu, v, 8);
+    };
+    const float s0 = row_sum(m);
+    m = on ? m / s0 + p.eps : 0.f;
+    const float s1 = col_sum(m);
+    m = on ? m / (s1 + p.eps) : 0.f;
+    for (int it = 1; it < p.iters; ++it) {
+      const float sr = row_sum(m);
+      m = on ? m / (sr + p.eps) : 0.f;
+      const float sc = col_sum(m);
+      m = on ? m / (sc + p.eps) : 0.f;
+    }
+    if (row0 + r < p.rows && (R > 1 || lane < 16)) {
+      HcCoef* k = p.coef + row0 + r;
+      if (hl < H) {
+        k->pre[hl] = s_pre[r][hl];
+        k->post[hl] = post;
+      }
+      if (on) k->comb[i * kMaxH + j] = m;
+    }
+  }
 
   // ---- collapse: this CTA's columns; the bf16 result replaces copy 0 in shared memory
   const bool norm = p.norm_w != nullptr;
-  for (int r = R == 1 ? 0 : warp; r < R; r += 8) {
+  const int busy = R > 1 && !HEAD ? 7 : 8;        // (the last warp is at the coefficients)
+  for (int r = R == 1 ? 0 : warp < busy ? warp : R; r < R; r += busy) {
     const int gr = row0 + r;
     float pre[kMaxH];
 #pragma unroll
     for (int h = 0; h < kMaxH; ++h) pre[h] = h < H ? s_pre[r][h] : 0.f;
     float ss = 0.f;
-    __nv_bfloat16* xr = xs + (long)r * H * w;
+    __nv_bfloat16* xr = xs + (long)r * pitch;
     for (int i = (R == 1 ? (int)threadIdx.x : lane) * 2; i < wc; i += R == 1 ? 512 : 64) {
       float a = 0.f, b = 0.f, ma = 0.f, mb = 0.f;
 #pragma unroll
@@ -398,16 +515,17 @@ __global__ void __cluster_dims__(kHcCtas, 1, 1) __launch_bounds__(256) hc_cluste
       vv[0] = t;
     }
   }
-  cluster.sync();                             // (also: nobody leaves before its partials have been read)
+  if (!apart) arrive();                       // (also: nobody leaves before its partials have been read)
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (norm) {
-    for (int r = R == 1 ? 0 : warp; r < R; r += 8) {
+    for (int r = R == 1 ? 0 : warp < busy ? warp : R; r < R; r += busy) {
       const int gr = row0 + r;
       float tot = 0.f;
 #pragma unroll
       for (int k = 0; k < kHcCtas; ++k) tot += cluster.map_shared_rank(&vv[0], k)[r];
       if (gr >= p.rows) continue;
       const float inv = rsqrtf(tot / d + p.rms_eps);
-      const __nv_bfloat16* xr = xs + (long)r * H * w;
+      const __nv_bfloat16* xr = xs + (long)r * pitch;
       for (int i = (R == 1 ? (int)threadIdx.x : lane) * 2; i < wc; i += R == 1 ? 512 : 64) {
         const float2 f = bf2_to_f2(*reinterpret_cast<const uint32_t*>(xr + i));
         const float2 g = bf2_to_f2(*reinterpret_cast<const uint32_t*>(p.norm_w + c0 + i));
@@ -496,13 +614,13 @@ int launch_hc_cluster(HcArgs p, cudaStream_t st) {
   constexpr int kMaxSlice = 160 * 1024;
   const size_t slice = (size_t)p.H * p.w * 2;
   const int R = p.rows <= 37 || 16 * slice > kMaxSlice ? 1 : 16;
-  const size_t smem = R * slice;
-  if (smem > kMaxSlice) return kHcGeneral;
+  const size_t smem = R * slice + (R > 1 ? R * 16 : 0);
+  if (R * slice > kMaxSlice) return kHcGeneral;
   auto kernel = R == 1 ? hc_cluster_kernel<1, HEAD> : hc_cluster_kernel<16, HEAD>;
   // the limit of any width, once: set to the bytes of each launch, a narrower engine of another thread could lower it
   // between this thread's set and its launch
   static unsigned long long limit_set[2] = {0, 0};
-  const cudaError_t e = tf_smem_limit((const void*)kernel, kMaxSlice, &limit_set[R == 1]);
+  const cudaError_t e = tf_smem_limit((const void*)kernel, kMaxSlice + 16 * 16, &limit_set[R == 1]);
   if (e != cudaSuccess) return (int)e;
   tf_launch(kernel, dim3((p.rows + R - 1) / R * kHcCtas), dim3(256), smem, st, p);
   return (int)cudaGetLastError();

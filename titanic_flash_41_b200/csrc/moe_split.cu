@@ -22,7 +22,8 @@
 //               scales (512 inputs at a time: row-major as stored, 16 bytes a row)
 // The structure of a CTA is that of moe_mx.cu; here K may end inside 512 inputs, and rows of scales may be 8 bytes off the
 // 16-byte grain (K = 2,304: 72 bytes), which two boxes over pairs of rows fetch.
-// SPLITMEASURED
+// 24 rows x 6 of 384 experts, 5,120 -> 2,304 -> 5,120, seven launches of a decode step (two of 24 rows, five of 4): FC1 1,437 ->
+// 667 us, FC2 783 -> 361; 24 rows stream at 0.9 of the copy rate, 4 rows (414 items over 148 SMs) at 0.75.
 //
 // Every wait is bounded: on a time-out the CTA raises its abort flag, reports TF_TIMEOUT, frees its tensor memory and returns.
 //
