@@ -924,6 +924,30 @@ def test_index_scores_of_prefill_rows_on_tcgen05(T, Hi, C, lo, hi):
     assert bool((scores[:, hi:] == 7.0).all()) and bool((scores[:, :lo] == 7.0).all())
 
 
+@pytest.mark.parametrize("scales", [(120, 127), (103, 104), (142, 143), (0, 110)])
+def test_index_scores_of_prefill_rows_take_every_block_scale(scales):
+    """Key blocks whose scales lie on both sides of the line between the f16 product and the fp32 one (2^-23 to 2^15): a key
+    element is its value rounded once to f16, whichever way it is formed.  Values of one half where larger ones would
+    overflow f16; queries exact in f16; the bound is that of the test above."""
+    torch.manual_seed(sum(scales))
+    T, Hi, Di, C = 40, 8, 128, 300
+    nib = torch.randint(0, 16, (C, Di)) if max(scales) < 140 else torch.randint(0, 2, (C, Di)) + 8 * torch.randint(0, 2, (C, Di))
+    sc = torch.tensor(scales)[torch.randint(0, 2, (C, Di // 32))]
+    keys = torch.cat([nib[:, 0::2] | nib[:, 1::2] << 4, sc], 1).to(torch.uint8).to(DEV).contiguous()
+    val = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, 0, -0.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64)[nib]
+    kd = (val * torch.exp2(sc.double() - 127).repeat_interleave(32, 1)).half().double().to(DEV)
+    q = (torch.randint(-64, 65, (T, Hi, Di), device=DEV) / 16.0).bfloat16()
+    w = torch.randn(T, Hi, device=DEV)
+    region, nvalid = torch.zeros(T, dtype=torch.int32, device=DEV), torch.full((T,), C, dtype=torch.int32, device=DEV)
+    scores, st = torch.zeros(T, C, device=DEV), native.StatusWord(DEV)
+    native.call("tf_index_scores_rows", q, w, region, nvalid, keys, C * 68, 68, T, Hi, Di, 32, scores, C, 0, C, st.t)
+    st.check()
+    s = torch.einsum("thd,cd->thc", q.double(), kd)
+    size = torch.einsum("thd,cd->thc", q.double().abs(), kd.abs())
+    want, mag = (s.relu() * w.double()[:, :, None]).sum(1), (size * w.double().abs()[:, :, None]).sum(1)
+    assert bool(((scores.double() - want).abs() <= 1e-5 * mag).all())
+
+
 def test_index_scores_and_router_logits_round_no_more_than_the_kernels_they_replaced():
     """Error against fp64 (2-norm over 2-norm): 6.4e-8 for the index scores of 64 heads and 8.06e-8 for the router logits of
     256 x 4,096 with the kernels before; one chain over all heads or warps gives 1.05e-7 and 8.4e-8.  The bounds lie between."""
