@@ -689,6 +689,31 @@ def test_topk_select_of_few_long_rows_matches_a_stable_sort(T, n_max):
         assert torch.equal(osc[r].cpu(), s[order])
 
 
+@pytest.mark.parametrize("lds,k", [(33, 1), (1025, 1000), (4099, 512), (32800, 2048), (49152, 2048)])
+def test_topk_select_of_many_rows_matches_a_stable_sort(lds, k):
+    """One CTA per row, the row in shared memory: rows of one or two words of scores a thread, not a multiple of four,
+    negative, infinite and equal scores (0 and -0 are different keys, so neither is drawn next to the other)."""
+    T = 34
+    gen = torch.Generator().manual_seed(lds)
+    scores = torch.randn(T, lds, generator=gen)
+    scores[:, 3::5] = scores[:, 2:3]
+    scores[1] = -1.5
+    scores[2, ::2] = -float("inf")
+    scores[3, ::3] = float("inf")
+    scores[4] = 2.0 + (torch.arange(lds) % 64) * 2.0 ** -21                  # equal but for the last bits
+    nvalid = torch.tensor([lds - (i * 7) % (lds // 2 + 1) for i in range(T)], dtype=torch.int32)
+    dev = scores.to(DEV)
+    sel, cnt = torch.zeros(T, k, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+    osc = torch.zeros(T, k, device=DEV)
+    native.call("tf_topk_select", dev, lds, nvalid.to(DEV), k, sel, cnt, osc, 0, T)
+    torch.cuda.synchronize()
+    for r in range(T):
+        n = int(nvalid[r])
+        order = sorted(torch.sort(scores[r, :n], descending=True, stable=True).indices[:k].tolist())
+        assert sel[r].cpu().tolist() == order + [-1] * (k - len(order)) and int(cnt[r]) == len(order)
+        assert torch.equal(osc[r].cpu()[:len(order)], scores[r, order])
+
+
 @pytest.mark.parametrize("T", [1, 4, 16, 27])
 def test_router_topk_group_in_registers_equals_the_shared_memory_form(T):
     """256 experts or fewer: the single-launch kernel keeps each row in registers; selection bias per

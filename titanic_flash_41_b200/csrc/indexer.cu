@@ -249,13 +249,13 @@ __device__ __forceinline__ uint32_t float_key(float f) {
 // scores [T, lds]; n[r] valid entries; out ids [T, k] ascending, -1 padded; count[r] = min(n, k).
 // `base` is added to every id (key-sharded scoring passes the shard offset).
 //
-// One CTA per row.  The row is read once into shared memory (STAGE; up to kSelStage scores, two CTAs an
-// SM up to half of that) and passed over five times there: histograms of 12, 10 and 10 key bits (a first digit
-// this fine spreads scores that share two or three octaves over enough bins for plain shared atomics), a
-// count per warp and the ordered compaction, in which every warp owns a contiguous stretch and finds its place
-// from ballots.  The bin of the k-th largest comes from a prefix sum over the bins.  Byte digits, a walk over
-// 256 bins by one thread, five reads from global memory and a block-wide scan with three barriers per
-// 1,024 scores took 3.45 ms for 16,384 rows of 16,384 scores on average.
+// One CTA per row.  A row of up to kSelStage scores is read once, into shared memory and the histogram of its top 12 key
+// bits (a first digit this fine spreads scores that share two or three octaves over enough bins for plain shared atomics).
+// The bin of the k-th largest comes from a prefix sum over the bins.  One pass over the row then leaves two bits for each
+// score, kept or still open, and the next digit's histogram; what follows (the two lower digits of ten bits, the equals,
+// the compaction) walks only the words of open or kept scores, a word of 32 scores a thread.
+// 2,048 rows of 32,768 scores: 204 us, of which reading them takes 41.  Five passes over the row in shared memory, two of
+// them ballots of every score for the counts and the compaction, took 343.
 constexpr int kSelRowThreads = 1024;
 constexpr int kSelStage = 48 * 1024;                 // scores a CTA can hold
 constexpr int kSelBins = 4096;
@@ -294,13 +294,143 @@ __device__ __forceinline__ void select_bin(const int* hist, int need, int* wsum,
   __syncthreads();
 }
 
-template <bool STAGE>
 __global__ void __launch_bounds__(kSelRowThreads) topk_select_kernel(const float* __restrict__ scores, int lds,
                                                                      const int* __restrict__ nvalid, int k,
                                                                      int* __restrict__ out, int* __restrict__ count,
                                                                      float* __restrict__ out_scores, int base, int vec) {
   tf_pdl_sync();
   extern __shared__ __align__(16) float row_s[];
+  __shared__ int hist[kSelBins], hist_mid[1024], hist_low[1024];
+  uint32_t *keep_w = reinterpret_cast<uint32_t*>(hist), *open_w = keep_w + kSelStage / 32;     // (once its bin is found)
+  static_assert(2 * (kSelStage / 32) <= kSelBins, "");
+  __shared__ int wsum[32];
+  __shared__ int s_bin, s_need;
+  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = min(nvalid[r], lds);
+  const float* s = scores + (long)r * lds;
+  int* o = out + (long)r * k;
+  if (n <= k) {
+    for (int i = tid; i < k; i += kSelRowThreads) {
+      o[i] = i < n ? base + i : -1;
+      if (out_scores) out_scores[(long)r * k + i] = i < n ? s[i] : -INFINITY;
+    }
+    if (tid == 0 && count) count[r] = n;
+    return;
+  }
+  for (int i = tid; i < kSelBins; i += kSelRowThreads) hist[i] = 0;
+  hist_mid[tid] = hist_low[tid] = 0;
+  __syncthreads();
+  if (vec) {
+#pragma unroll 4
+    for (int i = tid * 4; i < n; i += kSelRowThreads * 4) {        // (lds is a multiple of 4: the last piece stays in the row)
+      const float4 v = *reinterpret_cast<const float4*>(s + i);
+      *reinterpret_cast<float4*>(row_s + i) = v;
+      atomicAdd(&hist[float_key(v.x) >> 20], 1);
+      if (i + 1 < n) atomicAdd(&hist[float_key(v.y) >> 20], 1);
+      if (i + 2 < n) atomicAdd(&hist[float_key(v.z) >> 20], 1);
+      if (i + 3 < n) atomicAdd(&hist[float_key(v.w) >> 20], 1);
+    }
+  } else {
+#pragma unroll 4
+    for (int i = tid; i < n; i += kSelRowThreads) {
+      const float v = s[i];
+      row_s[i] = v;
+      atomicAdd(&hist[float_key(v) >> 20], 1);
+    }
+  }
+  __syncthreads();
+  select_bin<kSelBins>(hist, k, wsum, &s_bin, &s_need);
+  uint32_t bin = (uint32_t)s_bin;
+  int need = s_need;
+  // 32 scores to a word: above the bin of the k-th largest (kept) or in it (open, counted by the next ten bits)
+  const int words = (n + 31) / 32;
+#pragma unroll 4
+  for (int w = warp; w < words; w += kSelRowThreads / 32) {
+    const int i = w * 32 + lane;
+    const uint32_t key = i < n ? float_key(row_s[i]) : 0u;
+    const bool above = i < n && key >> 20 > bin, in = i < n && key >> 20 == bin;
+    const unsigned ma = __ballot_sync(0xffffffffu, above), mi = __ballot_sync(0xffffffffu, in);
+    if (in) atomicAdd(&hist_mid[(key >> 10) & 1023], 1);
+    if (lane == 0) {
+      keep_w[w] = ma;
+      open_w[w] = mi;
+    }
+  }
+  __syncthreads();
+  select_bin<1024>(hist_mid, need, wsum, &s_bin, &s_need);
+  bin = (uint32_t)s_bin;
+  need = s_need;
+  // From here a thread owns whole words, one or two neighbours.  Its walk over the open scores starts at bit `lane`, so that
+  // the threads of a warp read different banks where all are open.
+  const int own = (words + kSelRowThreads - 1) / kSelRowThreads, w0 = min(tid * own, words), w1 = min(w0 + own, words);
+  auto split = [&](int w, int shift, int* next) {
+    uint32_t keep = 0, open = 0;
+    for (uint32_t m = open_w[w], x = __funnelshift_r(m, m, lane); x; x &= x - 1) {
+      const int bit = (__ffs(x) - 1 + lane) & 31;
+      const uint32_t key = float_key(row_s[w * 32 + bit]), d = (key >> shift) & 1023;
+      if (d > bin) keep |= 1u << bit;
+      if (d == bin) {
+        open |= 1u << bit;
+        if (next) atomicAdd(&next[key & 1023], 1);
+      }
+    }
+    keep_w[w] |= keep;
+    open_w[w] = open;
+  };
+  for (int w = w0; w < w1; ++w) split(w, 10, hist_low);
+  __syncthreads();
+  select_bin<1024>(hist_low, need, wsum, &s_bin, &s_need);
+  bin = (uint32_t)s_bin;
+  need = s_need;                         // equals of the k-th largest that are kept, lowest positions first
+  const bool some = hist_low[bin & 1023] != need;
+  int mine = 0;
+  for (int w = w0; w < w1; ++w) {
+    split(w, 0, nullptr);
+    mine += __popc(some ? open_w[w] : keep_w[w] | open_w[w]);
+  }
+  // sum of `v` over the threads before this one
+  auto before = [&](int v) {
+    int inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += u;
+    }
+    if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    return __reduce_add_sync(0xffffffffu, lane < warp ? wsum[lane] : 0) + inc - v;
+  };
+  int pos = before(mine);
+  if (some) {
+    mine = 0;
+    for (int w = w0; w < w1; ++w) {
+      uint32_t m = open_w[w];
+      const int left = max(need - pos, 0);
+      pos += __popc(m);
+      while (__popc(m) > left) m &= ~(0x80000000u >> __clz(m));  // the last ones
+      open_w[w] = m;
+      mine += __popc(keep_w[w] | m);
+    }
+    __syncthreads();                     // (wsum has been read)
+    pos = before(mine);
+  }
+  for (int w = w0; w < w1; ++w)
+    for (uint32_t m = keep_w[w] | open_w[w]; m; m &= m - 1, ++pos) {
+      const int i = w * 32 + __ffs(m) - 1;
+      if (pos < k) {
+        o[pos] = base + i;
+        if (out_scores) out_scores[(long)r * k + pos] = row_s[i];
+      }
+    }
+  if (tid == 0 && count) count[r] = k;
+}
+
+// longer rows, read from global memory five times
+__global__ void __launch_bounds__(kSelRowThreads) topk_select_long_kernel(const float* __restrict__ scores, int lds,
+                                                                          const int* __restrict__ nvalid, int k,
+                                                                          int* __restrict__ out, int* __restrict__ count,
+                                                                          float* __restrict__ out_scores, int base) {
+  tf_pdl_sync();
   __shared__ int hist[kSelBins];
   __shared__ int wsum[32], weq[32];
   __shared__ int s_bin, s_need;
@@ -316,18 +446,9 @@ __global__ void __launch_bounds__(kSelRowThreads) topk_select_kernel(const float
     if (tid == 0 && count) count[r] = n;
     return;
   }
-  const float* src = STAGE ? row_s : s;
   for (int i = tid; i < kSelBins; i += kSelRowThreads) hist[i] = 0;
-  if (STAGE) {
-    if (vec) {
-      for (int i = tid * 4; i < n; i += kSelRowThreads * 4)      // (lds is a multiple of 4: the last piece stays in the row)
-        *reinterpret_cast<float4*>(row_s + i) = *reinterpret_cast<const float4*>(s + i);
-    } else {
-      for (int i = tid; i < n; i += kSelRowThreads) row_s[i] = s[i];
-    }
-  }
   __syncthreads();
-  for (int i = tid; i < n; i += kSelRowThreads) atomicAdd(&hist[float_key(src[i]) >> 20], 1);
+  for (int i = tid; i < n; i += kSelRowThreads) atomicAdd(&hist[float_key(s[i]) >> 20], 1);
   __syncthreads();
   select_bin<kSelBins>(hist, k, wsum, &s_bin, &s_need);
   uint32_t prefix = (uint32_t)s_bin << 20;
@@ -337,7 +458,7 @@ __global__ void __launch_bounds__(kSelRowThreads) topk_select_kernel(const float
     hist[tid] = 0;
     __syncthreads();
     for (int i = tid; i < n; i += kSelRowThreads) {
-      const uint32_t d = float_key(src[i]) ^ prefix;             // zero above the digits still open: same prefix
+      const uint32_t d = float_key(s[i]) ^ prefix;             // zero above the digits still open: same prefix
       if (d >> (shift + 10) == 0) atomicAdd(&hist[(d >> shift) & 1023], 1);
     }
     __syncthreads();
@@ -351,7 +472,7 @@ __global__ void __launch_bounds__(kSelRowThreads) topk_select_kernel(const float
   int gt = 0, eq = 0;
   for (int i0 = lo; i0 < hi; i0 += 32) {
     const int i = i0 + lane;
-    const uint32_t key = i < hi ? float_key(src[i]) : 0u;
+    const uint32_t key = i < hi ? float_key(s[i]) : 0u;
     gt += __popc(__ballot_sync(0xffffffffu, i < hi && key > thr));
     eq += __popc(__ballot_sync(0xffffffffu, i < hi && key == thr));
   }
@@ -366,7 +487,7 @@ __global__ void __launch_bounds__(kSelRowThreads) topk_select_kernel(const float
   const unsigned below = (1u << lane) - 1u;
   for (int i0 = lo; i0 < hi; i0 += 32) {
     const int i = i0 + lane;
-    const float v = i < hi ? src[i] : 0.f;
+    const float v = i < hi ? s[i] : 0.f;
     const uint32_t key = float_key(v);
     const unsigned mg = __ballot_sync(0xffffffffu, i < hi && key > thr), me = __ballot_sync(0xffffffffu, i < hi && key == thr);
     const int eq_rank = eq + __popc(me & below);
@@ -672,14 +793,14 @@ TF_API int tf_topk_select(const float* scores, int lds, const int* nvalid, int k
               count, out_scores, base);
   else if (lds <= kSelStage) {
     static unsigned long long limit_set = 0;
-    const cudaError_t e = tf_smem_limit((const void*)topk_select_kernel<true>, kSelStage * 4, &limit_set);
+    const cudaError_t e = tf_smem_limit((const void*)topk_select_kernel, kSelStage * 4, &limit_set);
     if (e != cudaSuccess) return (int)e;
     const int vec = lds % 4 == 0 && !(reinterpret_cast<uintptr_t>(scores) & 15);
-    tf_launch(topk_select_kernel<true>, dim3(T), dim3(kSelRowThreads), (size_t)(lds + 3) / 4 * 16, st, scores, lds, nvalid, k,
+    tf_launch(topk_select_kernel, dim3(T), dim3(kSelRowThreads), (size_t)(lds + 3) / 4 * 16, st, scores, lds, nvalid, k,
               out, count, out_scores, base, vec);
   } else {
-    tf_launch(topk_select_kernel<false>, dim3(T), dim3(kSelRowThreads), 0, st, scores, lds, nvalid, k, out, count, out_scores,
-              base, 0);
+    tf_launch(topk_select_long_kernel, dim3(T), dim3(kSelRowThreads), 0, st, scores, lds, nvalid, k, out, count, out_scores,
+              base);
   }
   return (int)cudaGetLastError();
 }
