@@ -420,7 +420,7 @@ class StepPlan:
         """Hash every block's rows; ``prevs[i]`` are the (up to ngram-1) tokens right before block i."""
         from . import engram as EG
         md = EG.metadata_for(cfg)
-        self.engram_ids = np.concatenate([EG.hash_positions(md, prev, list(t), start)
+        self.engram_ids = np.concatenate([EG.hash_positions(md, prev, np.asarray(t).tolist(), start)
                                           for (region, start, t), prev in zip(self.blocks, prevs)]).astype(np.int64)
         return self
 
@@ -457,23 +457,30 @@ class StepPlan:
     @staticmethod
     def build(blocks: Sequence[Tuple[int, int, Sequence[int]]], logits: str = "all") -> "StepPlan":
         """blocks: (region, start position, tokens).  logits: "all" | "last" (last row per block)."""
-        toks, pos, reg, first, last, lrows = [], [], [], [], [], []
-        r0 = 0
-        sizes = set()
-        for region, start, t in blocks:
-            n = len(t)
-            sizes.add(n)
-            toks += list(t)
-            pos += list(range(start, start + n))
-            reg += [region] * n
-            first += [r0] * n
-            last += [start + n - 1] * n
-            lrows += list(range(r0, r0 + n)) if logits == "all" else [r0 + n - 1]
-            r0 += n
+        # Arrays are filled block by block: as lists of Python numbers 16,384 rows took 4.2 ms, during which the GPU waits for
+        # a prefill's first launch (129,553 rows, planned in eight chunks: 33 ms).
         i32 = lambda a: np.asarray(a, dtype=np.int32)
-        gr = sizes.pop() if len(sizes) == 1 else 1
-        return StepPlan(i32(toks), i32(pos), i32(reg), i32(first), i32(last), i32(lrows), gr,
-                        blocks=[(r, s, list(t)) for r, s, t in blocks])
+        blocks = list(blocks)
+        sizes = [len(t) for _, _, t in blocks]
+        total = sum(sizes)
+        toks, pos, reg, first, last = (np.empty(total, dtype=np.int32) for _ in range(5))
+        lrows, kept = [], []
+        r0 = 0
+        for (region, start, t), n in zip(blocks, sizes):
+            rows = slice(r0, r0 + n)
+            plain = isinstance(t, np.ndarray) and t.dtype == np.int32
+            toks[rows] = t if plain else i32(list(t))
+            span = range(start, start + n)
+            i32([span.start, span.stop - 1])               # (raises where a position does not fit)
+            pos[rows] = np.arange(span.start, span.stop)
+            reg[rows], first[rows], last[rows] = region, r0, span.stop - 1
+            if logits != "all":
+                lrows.append(r0 + n - 1)
+            kept.append((region, start, toks[rows] if plain else list(t)))
+            r0 += n
+        lrows = np.arange(total, dtype=np.int32) if logits == "all" else i32(lrows)
+        gr = sizes[0] if sizes and len(set(sizes)) == 1 else 1
+        return StepPlan(toks, pos, reg, first, last, lrows, gr, blocks=kept)
 
     @property
     def T(self) -> int:

@@ -220,7 +220,7 @@ class SpPrefill:
         key = (region, p0 + lo, T)
         hit = self._plans.get(key)
         if hit is None:                                             # one plan per slice, shared by all layers
-            plan = StepPlan.build([(region, p0 + lo, tokens[lo:hi].tolist())], logits="last")
+            plan = StepPlan.build([(region, p0 + lo, tokens[lo:hi])], logits="last")
             hit = self._plans[key] = (plan,) + tuple(v.plan_shape(plan, v.cfg.compress_ratio))
         plan, nmax, rpg = hit
         b = v._bufs(T)

@@ -54,7 +54,7 @@ def _encoder_layer_major(eng: Engine, region: int, toks: np.ndarray, sizes: List
     n = int(toks.shape[0])
     resid = torch.empty(n, cfg.hidden * cfg.hc_mult, dtype=torch.bfloat16, device=eng.dev)
     offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
-    plans = [_recent(StepPlan.build([(region, start + int(offs[c]), toks[offs[c]:offs[c + 1]].tolist())],
+    plans = [_recent(StepPlan.build([(region, start + int(offs[c]), toks[offs[c]:offs[c + 1]])],
                                     logits="last"), cfg, prev, toks, int(offs[c]))
              for c in range(len(sizes))]
     shapes = [eng.plan_shape(p, cfg.compress_ratio) for p in plans]
@@ -168,7 +168,7 @@ def run_prefill(eng: Engine, region: int, tokens, chunk: int, start: int = 0, ne
         # path through the encoder layers, the rest is split over the ranks
         k = (-start) % cfg.max_ratio
         if 0 < k and n - k >= max(cfg.window, 1) and sp.usable(start + k, n - k):
-            plan = _recent(StepPlan.build([(region, start, toks[:k].tolist())], logits="last"), cfg, prev, toks, 0)
+            plan = _recent(StepPlan.build([(region, start, toks[:k])], logits="last"), cfg, prev, toks, 0)
             b = eng._bufs(k)
             eng.upload_plan(plan, b)
             nmax, rpg = eng.plan_shape(plan, cfg.compress_ratio)
@@ -196,7 +196,7 @@ def run_prefill(eng: Engine, region: int, tokens, chunk: int, start: int = 0, ne
             logits = eng._head(sizes[-1], eng._bufs(sizes[-1]), torch.tensor([sizes[-1] - 1], device=eng.dev))
         sizes = []
     for T in sizes:
-        plan = _recent(StepPlan.build([(region, start + done, toks[done:done + T].tolist())], logits="last"),
+        plan = _recent(StepPlan.build([(region, start + done, toks[done:done + T])], logits="last"),
                        cfg, prev, toks, done)
         b = eng._bufs(T)
         eng.upload_plan(plan, b)
@@ -217,7 +217,7 @@ def run_prefill(eng: Engine, region: int, tokens, chunk: int, start: int = 0, ne
             return None
     if late < L and tail_n > 0:
         p0 = start + n - tail_n
-        plan = _recent(StepPlan.build([(region, p0, toks[n - tail_n:].tolist())], logits="last"),
+        plan = _recent(StepPlan.build([(region, p0, toks[n - tail_n:])], logits="last"),
                        cfg, prev, toks, n - tail_n)
         plan.min_pos = np.full(tail_n, p0, dtype=np.int32)     # older rows never ran in the late group
         b = eng._bufs(tail_n)
