@@ -1065,3 +1065,12 @@ def test_fused_boundary_row_form(T, d, k, shared):
     q, s = torch.zeros_like(x8), torch.zeros_like(x8s)
     native.call("tf_quant_rows_mx8", h16, d, q, s, T, d)
     assert torch.equal(q, x8) and torch.equal(s, x8s)
+
+
+@pytest.mark.parametrize("T,d,m", [(1, 8, 1), (33, 2056, 3), (70, 5120, 4)])
+def test_expanded_rows_are_copies(T, d, m):
+    """Fewer and more pieces than threads, a ragged last round; rows behind the last one stay."""
+    src = torch.randn(T, d, device=DEV).bfloat16()
+    out = torch.full((T + 1, m, d), 3.0, device=DEV, dtype=torch.bfloat16)
+    native.call("tf_expand_rows", src, out, T, d, m)
+    assert torch.equal(out[:T], src[:, None, :].expand(T, m, d)) and bool((out[T] == 3.0).all())

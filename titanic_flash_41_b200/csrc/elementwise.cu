@@ -27,6 +27,18 @@ __global__ void embed_kernel(const int* __restrict__ tokens, const __nv_bfloat16
   for (int i = threadIdx.x; i < d / 8; i += blockDim.x) dst[i] = src[i];
 }
 
+// Row r of src -> rows m r .. m r + m - 1 of out (every residual copy starts as the embedding).  Bound by the stores: each
+// 16 bytes are loaded once and stored m times.  4,001 rows of 5,120 to four copies: 32 us (6.4 TB/s); a strided tensor copy took 174.
+__global__ void __launch_bounds__(256) expand_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ out, int d8, int m) {
+  tf_pdl_sync();
+  const uint4* s = src + (long)blockIdx.x * d8;
+  uint4* o = out + (long)blockIdx.x * m * d8;
+  for (int i = threadIdx.x; i < d8; i += blockDim.x) {
+    const uint4 v = s[i];
+    for (int j = 0; j < m; ++j) o[(long)j * d8 + i] = v;
+  }
+}
+
 // --------------------------------------------------------------------------- residual + norm
 // x (bf16 residual stream) += delta (optional, f32 or bf16); then h = rmsnorm(x) * w written as
 // f16 (decode GEMMs), bf16, and/or FP8 e4m3 with one fp32 scale per 128 along K (tensor-core
@@ -551,6 +563,14 @@ TF_API int tf_embed(const int* tokens, const void* table, void* out, int T, int 
   if (d % 8) return -1;
   tf_launch(embed_kernel, dim3(T), dim3(128), 0, st, tokens, (const __nv_bfloat16*)table, (__nv_bfloat16*)out, d, vocab,
                                   (TfStatusWord*)status);
+  return (int)cudaGetLastError();
+}
+
+// src [T, d] bf16 -> out [T, m, d]; d a multiple of 8, both 16-byte aligned
+TF_API int tf_expand_rows(const void* src, void* out, int T, int d, int m, cudaStream_t st) {
+  if (d % 8 || m < 1 || (((uintptr_t)src | (uintptr_t)out) & 15)) return -1;
+  if (T <= 0) return 0;
+  tf_launch(expand_rows_kernel, dim3(T), dim3(256), 0, st, (const uint4*)src, (uint4*)out, d / 8, m);
   return (int)cudaGetLastError();
 }
 

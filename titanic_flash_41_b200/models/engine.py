@@ -716,7 +716,9 @@ class Engine:
             b["qa16"] = torch.zeros(T, cfg.q_lora_rank, dtype=torch.float16, device=dev)
             b["qfull"] = torch.zeros(T, Hl * Dh, dtype=b["P"].dtype, device=dev)
         if cfg.o_groups:
-            b["mid16"] = torch.zeros(T, (cfg.o_groups // self.world) * cfg.o_lora_rank, dtype=torch.float16, device=dev)
+            # (the big GEMM writes bf16: its quantiser reads that as it is, without a pass to f16 for each group)
+            b["mid16"] = torch.zeros(T, (cfg.o_groups // self.world) * cfg.o_lora_rank, device=dev,
+                                     dtype=torch.bfloat16 if big and cfg.o_lora_rank % 8 == 0 else torch.float16)
         if self.engram:
             ec = cfg.engram
             n_ids = (ec.ngram - 1) * ec.heads
@@ -1321,7 +1323,7 @@ class Engine:
                 e.index_copy_(0, x_patch[0], x_patch[1].to(e.dtype))
             if cfg.hc_mult > 1:
                 # every residual copy starts as the embedding (reference: kernels/core.cu:530-543)
-                b["x"].view(T, cfg.hc_mult, cfg.hidden).copy_(e[:T, None, :].expand(T, cfg.hc_mult, cfg.hidden))
+                native.call("tf_expand_rows", e, b["x"], T, cfg.hidden, cfg.hc_mult)
         else:
             b["x"][:T].copy_(x_in)
         b.pop("pending_combine", None)
