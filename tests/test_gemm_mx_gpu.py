@@ -273,3 +273,31 @@ def test_gemm_mx_experts_tiles(K, tile_max, two):
                     w = E.dequant_mxfp4(pk[j][e], sc[j][e]).double()
                     assert _rel(c[rows, j * N:(j + 1) * N], a[rows] @ w.t()) < tol
         assert bool((c[expert < 0] == 5.0).all()) and bool((c[:, (2 if two else 1) * N:] == 5.0).all())
+
+
+@pytest.mark.parametrize("M", [1, 130, 200, 256])
+def test_grouped_gemm_stores_no_row_behind_the_last_and_none_of_an_empty_tile(M):
+    """Grouped rows that end inside a 128-row tile, with and without the rows of each tile, an empty tile among them, and a
+    count of tiles beyond the list: C keeps what it held behind row M and in every row that does not count."""
+    gen = torch.Generator(device=DEV).manual_seed(M)
+    El, N, K, tiles = 2, 256, 256, -(-M // 128)
+    a = _random_fp8(M, K, gen)
+    sfa = torch.full((K // 128, tiles * 4, 128), 127, dtype=torch.uint8, device=DEV)
+    sfb = torch.full((K // 128, El * N // 32, 128), 124, dtype=torch.uint8, device=DEV)
+    w = torch.randint(0, 256, (El * N, K // 2), dtype=torch.uint8, device=DEV, generator=gen)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    te, st = i32([1, 0][:tiles]), native.StatusWord(DEV)
+    full = a.view(F8).double() @ E.dequant_mxfp4(w.view(El, N, K // 2), torch.full((El, N, K // 32), 124, dtype=torch.uint8, device=DEV)).double().transpose(1, 2)
+    for rows in (None, [0, 128], [128, 0], [1, 77]):
+        for dt, tol in ((torch.float32, 2e-5), (torch.bfloat16, 4e-3)):
+            c = torch.full((M + 256, N), 3.0, device=DEV, dtype=dt)
+            mx.gemm(a, sfa, w, sfb, c, M, N, K, st.t, b_fp4=True, b_rows=El * N, tile_expert=te, num_m_tiles=i32([tiles + (rows is not None)]),
+                    tile_rows=None if rows is None else i32(rows[:tiles]))
+            st.check()
+            live = torch.zeros(M + 256, dtype=torch.bool, device=DEV)
+            for t in range(tiles):
+                n = min(128 if rows is None else rows[t], M - 128 * t)
+                live[128 * t:128 * t + n] = True
+                if n > 0:
+                    assert _rel(c[128 * t:128 * t + n], full[int(te[t])][128 * t:128 * t + n]) < tol
+            assert bool((c[~live] == 3.0).all())

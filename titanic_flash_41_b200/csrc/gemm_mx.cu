@@ -95,6 +95,7 @@ struct MxGemmParams {
   const int* tile_row0;      // first row of a tile (null: 128 * tile)
   const int* tile_rows;      // rows of a tile that count (null: 128); the others are not stored
   const int* num_tiles;
+  int max_tiles;             // room of the lists
   TfStatusWord* status;
 };
 
@@ -167,7 +168,7 @@ __device__ __forceinline__ uint32_t idesc_mx(uint32_t afmt, uint32_t rows) {
 }
 
 struct MxTile {
-  int row0, rows, n;         // first row, rows that count, columns of the MMA (a multiple of 32)
+  int row0, rows, n;         // first row, rows that count and that C has (0 or less: none), columns of the MMA (a multiple of 32)
   int f0;                    // first feature inside its matrix
   int wrow;                  // the same as a row of B
   int mat;
@@ -233,7 +234,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   // set-up done: wait for the kernel before this one (operands and tile lists are its outputs)
   tf_pdl_sync();
   const int fb1 = (p.N + BF - 1) / BF, fbs = fb1 * p.mats;  // feature blocks of one matrix, of all
-  const int rt = p.tile_expert ? *p.num_tiles : (p.M + p.tile_n - 1) / p.tile_n;
+  const int rt = p.tile_expert ? min(*p.num_tiles, p.max_tiles) : (p.M + p.tile_n - 1) / p.tile_n;
   const int items = rt * fbs;
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
   // Order of the tiles.  The pairs running at one time should share their operands: experts take all feature
@@ -247,7 +248,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       ri = item / fbs;
       fb = item - ri * fbs;
       t.row0 = p.tile_row0 ? p.tile_row0[ri] : 128 * ri;
-      t.rows = p.tile_rows ? p.tile_rows[ri] : 128;
+      t.rows = min(p.tile_rows ? p.tile_rows[ri] : 128, p.M - t.row0);
     } else {
       const int g = item / (kGroupRows * fbs), r = item - g * kGroupRows * fbs, gm = min(kGroupRows, rt - g * kGroupRows);
       ri = g * kGroupRows + r % gm;
@@ -255,8 +256,8 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       t.row0 = ri * p.tile_n;
       t.rows = min(p.tile_n, p.M - t.row0);
     }
-    t.rows = max(1, min(t.rows, p.tile_n));
-    t.n = (t.rows + 31) & ~31;
+    t.rows = min(t.rows, p.tile_n);
+    t.n = (max(t.rows, 1) + 31) & ~31;                      // (an empty tile is walked like one of a row; nothing is stored)
     t.mat = fb >= fb1;
     t.f0 = (fb - (t.mat ? fb1 : 0)) * BF;
     t.wrow = t.f0 + (p.tile_expert ? p.tile_expert[ri] * p.N : 0) + rank * 128;
@@ -823,6 +824,7 @@ int launch_mx(const MxCall& a, void* status, cudaStream_t st) {
   p.sfa_units = a.sfa_units; p.sfb_units = a.sfb_units;
   p.C = a.C; p.ldc = a.ldc;
   p.tile_expert = a.tile_expert; p.tile_row0 = a.tile_row0; p.tile_rows = a.tile_rows; p.num_tiles = a.num_tiles;
+  p.max_tiles = a.max_tiles;
   p.status = reinterpret_cast<TfStatusWord*>(status);
   const long tiles = (a.tile_expert ? a.max_tiles : (a.M + p.tile_n - 1) / p.tile_n) * (long)fbs;
   const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
