@@ -83,3 +83,42 @@ def test_split_refuses_bad_arguments():
     for N, K in ((128, 256), (256, 128), (256, 384)):               # plain form: N of 256; K of 256
         with pytest.raises(native.NativeError):
             native.call("tf_moe_gemv_split", t, None, t, None, 1, t, t, 1, t, N, None, None, N, K, t, t, t, t, t, 1, 0.0, st.t)
+
+
+def _both(x, w1, w3, w2, groups, limit):
+    """Both GEMVs over the groups: (f16 activations as rows of their pieces' sum, f32 rows by pair)."""
+    El, I, K = w1[0].shape[0], w1[0].shape[1], x.shape[1]
+    ge, gs, gc, ng, sp, nl = groups
+    pairs, pitch, st = sp.numel(), native.lib().tf_moe_split_pitch, native.StatusWord(DEV)
+    u8 = lambda *s: torch.full(s, 0x55, dtype=torch.uint8, device=DEV)
+    x3, x3s, a3, a3s = u8(3 * pairs, K), u8(3 * pairs, pitch(K)), u8(3 * pairs, I), u8(3 * pairs, pitch(I))
+    y = torch.full((pairs, K), 7.0, device=DEV)
+    native.call("tf_moe_split_rows", x, K, sp, nl, 1, pairs, x3, x3s, K)
+    native.call("tf_moe_gemv_split", w1[0], w3[0], w1[1], w3[1], El, x3, x3s, pairs, None, 0, a3, a3s, I, K, ge, gs, gc, ng, sp,
+                ge.numel(), limit, st.t)
+    native.call("tf_moe_gemv_split", w2[0], None, w2[1], None, El, a3, a3s, pairs, y, K, None, None, K, I, ge, gs, gc, ng, sp,
+                ge.numel(), 0.0, st.t)
+    st.check()
+    return y
+
+
+@pytest.mark.parametrize("limit", [0.0, 10.0])
+def test_rows_that_are_not_finite_stay_so(limit):
+    """An infinity or a NaN among a row's inputs, and (without a clamp) a SwiGLU product beyond f16: every output of that row is
+    NaN, those of the other rows keep their bits."""
+    K = I = 512
+    gen = torch.Generator(device=DEV).manual_seed(11)
+    x = torch.randn(9, K, device=DEV, generator=gen).half()
+    w1, w3, w2 = (E.quant_mxfp4_device(torch.randn(5, n, k, device=DEV, generator=gen) * 0.5) for n, k in ((I, K), (I, K), (K, I)))
+    groups = _groups([6, 3], 1)
+    clean = _both(x, w1, w3, w2, groups, limit)
+    assert bool(torch.isfinite(clean).all())
+    bad = x.clone()
+    bad[1, 40], bad[2, 77], bad[4, 500] = float("inf"), -float("inf"), float("nan")
+    spoilt = [1, 2, 4]
+    if limit == 0.0:
+        bad[7] *= 200.0                                      # products of 2e5 and more
+        spoilt.append(7)
+    y = _both(bad, w1, w3, w2, groups, limit)
+    kept = [r for r in range(9) if r not in spoilt]
+    assert bool(torch.isnan(y[spoilt]).all()) and torch.equal(y[kept], clean[kept])

@@ -100,6 +100,9 @@ __device__ __forceinline__ int mx_exponent(float amax) {
   const float m = frexpf(amax * (1.f / 448.f), &e2);       // value = m * 2^e2, m in [0.5, 1)
   return max(-127, min(127, (m == 0.5f) ? e2 - 1 : e2));
 }
+// e4m3 has a NaN and no infinity: one in a row, or a product beyond f16, goes on as NaN, and with it every sum over the row (as a
+// saturated 448 times the block's scale it came out as a plausible number)
+__device__ __forceinline__ float finite_or_nan(float x) { return fmaf(x, 0.f, x); }
 __device__ __forceinline__ uint8_t to_e4m3(float x) { return (uint8_t)__nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3); }
 
 // DUAL 1: w1 and w3 tiles + SwiGLU; 0: two adjacent tiles of one matrix
@@ -298,15 +301,15 @@ moe_split_kernel(const __grid_constant__ CUtensorMap mapW1, const __grid_constan
         const float o3 = (__uint_as_float(a3[3 * r]) + __uint_as_float(a3[3 * r + 1])) + __uint_as_float(a3[3 * r + 2]);
         if (DUAL) {
           float gate = o1, up = o3;
-          if (p.limit > 0.f) {
-            gate = fminf(gate, p.limit);
-            up = fminf(fmaxf(up, -p.limit), p.limit);
+          if (p.limit > 0.f) {                 // (comparisons, not fminf: a NaN is not clamped away)
+            gate = gate > p.limit ? p.limit : gate;
+            up = up > p.limit ? p.limit : up < -p.limit ? -p.limit : up;
           }
-          float rest = __half2float(__float2half(gate / (1.f + __expf(-gate)) * up));
+          float rest = finite_or_nan(__half2float(__float2half(gate / (1.f + __expf(-gate)) * up)));
           // the warp's 32 features are one scale group of the second GEMV's input
 #pragma unroll
           for (int i = 0; i < kPieces; ++i) {
-            const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(rest))));
+            const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, rest == rest ? __float_as_uint(fabsf(rest)) : 0u));
             const int ex = mx_exponent(amax);
             const uint8_t q = to_e4m3(rest * exp2f((float)-ex));
             const long row = kPieces * (long)(st.start + st.c0 + r) + i;
@@ -416,15 +419,15 @@ __global__ void __launch_bounds__(128) split_rows_kernel(const __half* __restric
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 f = __half22float2(h[e]);
-      v[8 * j + 2 * e] = f.x;
-      v[8 * j + 2 * e + 1] = f.y;
+      v[8 * j + 2 * e] = finite_or_nan(f.x);
+      v[8 * j + 2 * e + 1] = finite_or_nan(f.y);
     }
   }
 #pragma unroll 1
   for (int piece = 0; piece < kPieces; ++piece) {
     float amax = 0.f;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) amax = fmaxf(amax, fabsf(v[j]));
+    for (int j = 0; j < 32; ++j) amax = fmaxf(amax, fabsf(v[j]));          // (of the numbers: fmaxf passes a NaN by)
     const int ex = mx_exponent(amax);
     const float inv = exp2f((float)-ex), scale = exp2f((float)ex);
     uint32_t o[8];
