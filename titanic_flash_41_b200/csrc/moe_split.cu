@@ -2,22 +2,24 @@
 //
 // The experts are MXFP4 (packed e2m1, one UE8M0 scale per 32 inputs).  Where the activations stay f16, the register-fed kernel
 // of smallm_gemm.cu unpacks every nibble on the CUDA cores and runs at half of the HBM rate.  An f16 number is the sum of
-// three e4m3 numbers with block scales of their own (4 significant bits each, and the sign of a remainder is one more:
-// the eleven bits of an f16 and some), so three rows of `tcgen05.mma kind::mxf8f6f4.block_scale` replace one f16 row:
+// six e4m3 numbers with block scales of their own, so six rows of `tcgen05.mma kind::mxf8f6f4.block_scale` replace one f16 row:
 //
-//   x = p0 + p1 + p2      p_i: e4m3, UE8M0 scale per 32 inputs of the remainder x - p0 .. - p_{i-1}
+//   x = p0 + p1 + .. + p5      p_i: e4m3, UE8M0 scale per 32 inputs of the remainder x - p0 .. - p_{i-1}
 //
-// Elements near their block's maximum are represented exactly; what is left of the others is below 2^-27 of the maximum.  Products
-// of e2m1 and e4m3 are exact and sums are fp32, the three sums are added in fp32.  Error against fp64 sums of the same
+// Each piece takes four significant bits of an element near the maximum of what its block still holds, and all bits above 2^-9 of
+// its scale of the others; the maximum falls by 16 or more from piece to piece.  Three pieces hold the eleven bits of every
+// element above 2^-14 of its block's maximum, six those of any finite f16 numbers in one block (the largest is 2^40 times the
+// smallest; with three, four, five pieces up to 2^-27, 2^-32, 2^-37 of the maximum were left).  Products of e2m1 and e4m3 are exact and
+// sums are fp32; the pieces' sums are added in fp32, the smallest first.  Error against fp64 sums of the same
 // f16 inputs, 5,120 normal inputs: 3.8e-8 (f16 x f16 mma.sync form: 2.3e-7); with magnitudes spread over e^(2 normal):
 // 7e-7 (1.7e-6).
 //
-// An accumulator has 16 columns: five rows of an expert (three columns each).  An expert with more rows takes another pass over
+// An accumulator has 16 columns: two rows of an expert (six columns each).  An expert with more rows takes another pass over
 // its weights, out of L2; decode blocks give an expert one or two.
 //
-//   split_rows_kernel  the activations of every (row, expert) pair, in the order of the groups, as three rows
+//   split_rows_kernel  the activations of every (row, expert) pair, in the order of the groups, as six rows
 //   moe_split_kernel   persistent CTAs, one per SM; work item = (expert, 128 features of w1 and of w3) or
-//                      (expert, 256 features of w2); FC1 writes FC2's input (clamped SwiGLU, rounded to f16, three pieces)
+//                      (expert, 256 features of w2); FC1 writes FC2's input (clamped SwiGLU, rounded to f16, six pieces)
 //     warp 0    TMA producer of the tiles, warp 1 MMA issuer, warps 2-5 scale movers and epilogue, warp 6 TMA producer of the
 //               scales (512 inputs at a time: row-major as stored, 16 bytes a row)
 // The structure of a CTA is that of moe_mx.cu; here K may end inside 512 inputs, and rows of scales may be 8 bytes off the
@@ -39,7 +41,7 @@ namespace {
 constexpr int kThreads = 7 * 32;
 constexpr int kTile = 128;          // features of a matrix tile
 constexpr int kCols = 16;           // accumulator columns of a matrix
-constexpr int kPieces = 3, kItemRows = kCols / kPieces;
+constexpr int kPieces = 6, kItemRows = kCols / kPieces;
 constexpr int kBK = 128;            // inputs per stage
 constexpr int kStages = 6;
 constexpr int kStageBytes = 2 * kTile * 128 + kCols * 128;
@@ -57,7 +59,7 @@ struct SplitParams {
   const int* n_groups;
   const int* sorted_pairs;
   void* out;                        // plain form: f32 rows by pair
-  uint8_t* q_out;                   // fused form: pieces [3 pairs][N] and their scales [3 pairs][q_pitch]
+  uint8_t* q_out;                   // fused form: pieces [6 pairs][N] and their scales [6 pairs][q_pitch]
   uint8_t* q_scale;
   int q_pitch, ldo, N, K, off_grain;       // off_grain: rows of weight scales 8 bytes off the 16-byte grain
   float limit;
@@ -160,7 +162,7 @@ moe_split_kernel(const __grid_constant__ CUtensorMap mapW1, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   tf_pdl_sync();
   const int items = *p.n_groups * tiles_n;
-  // One step of a role: five rows of one expert against one item's features
+  // One step of a role: two rows of one expert against one item's features
   struct Step {
     int item, g, n0, start, count, c0;       // group, first feature, first pair and pairs of the group, first pair of the step
   };
@@ -297,8 +299,12 @@ moe_split_kernel(const __grid_constant__ CUtensorMap mapW1, const __grid_constan
 #pragma unroll
       for (int r = 0; r < kItemRows; ++r) {
         if (r >= rows) break;
-        const float o1 = (__uint_as_float(a1[3 * r]) + __uint_as_float(a1[3 * r + 1])) + __uint_as_float(a1[3 * r + 2]);
-        const float o3 = (__uint_as_float(a3[3 * r]) + __uint_as_float(a3[3 * r + 1])) + __uint_as_float(a3[3 * r + 2]);
+        float o1 = __uint_as_float(a1[kPieces * r + kPieces - 1]), o3 = __uint_as_float(a3[kPieces * r + kPieces - 1]);
+#pragma unroll
+        for (int i = kPieces - 2; i >= 0; --i) {
+          o1 += __uint_as_float(a1[kPieces * r + i]);
+          o3 += __uint_as_float(a3[kPieces * r + i]);
+        }
         if (DUAL) {
           float gate = o1, up = o3;
           if (p.limit > 0.f) {                 // (comparisons, not fminf: a NaN is not clamped away)
@@ -403,7 +409,7 @@ moe_split_kernel(const __grid_constant__ CUtensorMap mapW1, const __grid_constan
   }
 }
 
-// x [rows, K] f16 -> pieces of the rows of the sorted pairs: q [3 pairs][K], s [3 pairs][pitch].  One thread per (pair, 32 inputs).
+// x [rows, K] f16 -> pieces of the rows of the sorted pairs: q [6 pairs][K], s [6 pairs][pitch].  One thread per (pair, 32 inputs).
 __global__ void __launch_bounds__(128) split_rows_kernel(const __half* __restrict__ x, int ldx, const int* __restrict__ sorted_pairs,
                                                          const int* __restrict__ n_local, int topk, uint8_t* __restrict__ q,
                                                          uint8_t* __restrict__ s, int pitch, int pairs, int K) {
@@ -467,10 +473,13 @@ inline bool make_map_fp4(CUtensorMap* map, const void* base, uint64_t rows, uint
 
 }  // namespace
 
+// Rows of a split buffer for one f16 row
+TF_API int tf_moe_split_pieces() { return kPieces; }
+
 // Bytes between the scale rows of a split buffer of K inputs (K / 32, rounded up to whole 16 bytes)
 TF_API int tf_moe_split_pitch(int K) { return (K / 32 + 15) / 16 * 16; }
 
-// x [rows, K] f16 (16-byte aligned rows) -> q [3 * pairs, K] e4m3, s [3 * pairs, tf_moe_split_pitch(K)] UE8M0: three pieces of the
+// x [rows, K] f16 (16-byte aligned rows) -> q [6 * pairs, K] e4m3, s [6 * pairs, tf_moe_split_pitch(K)] UE8M0: the six pieces of the
 // row of every sorted pair (rows sorted_pairs[i] / topk, i < *n_local <= pairs).
 TF_API int tf_moe_split_rows(const void* x, int ldx, const int* sorted_pairs, const int* n_local, int topk, int pairs, void* q,
                              void* s, int K, cudaStream_t st) {
@@ -482,8 +491,8 @@ TF_API int tf_moe_split_rows(const void* x, int ldx, const int* sorted_pairs, co
 }
 
 // Routed experts over the groups of tf_route_group with split f16 rows (x, sx: tf_moe_split_rows or the fused form's outputs,
-// 3 * pairs rows in sorted order).  With w3: clamped SwiGLU of w1 / w3, rounded to f16, as pieces q_out [3 * pairs, N] and
-// q_scale [3 * pairs, tf_moe_split_pitch(N)], in sorted order; N a multiple of 128.  Without: f32 out rows by pair; N of 256.
+// 6 * pairs rows in sorted order).  With w3: clamped SwiGLU of w1 / w3, rounded to f16, as pieces q_out [6 * pairs, N] and
+// q_scale [6 * pairs, tf_moe_split_pitch(N)], in sorted order; N a multiple of 128.  Without: f32 out rows by pair; N of 256.
 // w [experts, N, K / 2] packed e2m1, s [experts, N, K / 32] UE8M0; K a multiple of 256.
 TF_API int tf_moe_gemv_split(const void* w1, const void* w3, const void* s1, const void* s3, int experts, const void* x,
                              const void* sx, int pairs, void* out, int ldo, void* q_out, void* q_scale, int N, int K,

@@ -700,10 +700,11 @@ class Engine:
             b.update(x8=torch.zeros(T, d, **u8), x8s=torch.zeros(T, d // 32, **u8),
                      a8=torch.zeros(npairs, cfg.moe_inter, **u8), a8s=torch.zeros(npairs, cfg.moe_inter // 32, **u8))
         elif self._moe_split_ok(T):
-            # f16 expert inputs as three MXFP8 rows each, in the order of the groups
+            # f16 expert inputs as rows of MXFP8 pieces, in the order of the groups
             u8, pitch = dict(dtype=torch.uint8, device=dev), native.lib().tf_moe_split_pitch
-            b.update(x3=torch.zeros(3 * npairs, d, **u8), x3s=torch.zeros(3 * npairs, pitch(d), **u8),
-                     a3=torch.zeros(3 * npairs, cfg.moe_inter, **u8), a3s=torch.zeros(3 * npairs, pitch(cfg.moe_inter), **u8))
+            rows = native.lib().tf_moe_split_pieces() * npairs
+            b.update(xp=torch.zeros(rows, d, **u8), xps=torch.zeros(rows, pitch(d), **u8),
+                     ap=torch.zeros(rows, cfg.moe_inter, **u8), aps=torch.zeros(rows, pitch(cfg.moe_inter), **u8))
         m = cfg.hc_mult
         if m > 1:
             # the residual stream is m copies per row; b["x"] is their flat [T, m*d] view
@@ -1162,13 +1163,13 @@ class Engine:
                 native.call("tf_moe_gemv_mx", L.ew2, None, L.es2, None, self.El, b["a8"], b["a8s"], npairs,
                             b["y_pair"], d, None, None, d, I, 1, b["g_expert"], b["g_start"], b["g_count"],
                             b["n_groups"], b["sorted_pairs"], slots, 0.0, 0, 0, T, self.status.t)
-            elif "x3" in b:
-                # MXFP4 weights x f16 activations, every row as the sum of three MXFP8 rows
+            elif "xp" in b:
+                # MXFP4 weights x f16 activations, every row as the sum of its MXFP8 pieces
                 groups = (b["g_expert"], b["g_start"], b["g_count"], b["n_groups"], b["sorted_pairs"], slots)
-                native.call("tf_moe_split_rows", b["h16"], d, b["sorted_pairs"], b["n_local"], cfg.topk, npairs, b["x3"], b["x3s"], d)
-                native.call("tf_moe_gemv_split", L.ew1, L.ew3, L.es1, L.es3, self.El, b["x3"], b["x3s"], npairs, None, 0,
-                            b["a3"], b["a3s"], I, d, *groups, cfg.swiglu_limit, self.status.t)
-                native.call("tf_moe_gemv_split", L.ew2, None, L.es2, None, self.El, b["a3"], b["a3s"], npairs, b["y_pair"], d,
+                native.call("tf_moe_split_rows", b["h16"], d, b["sorted_pairs"], b["n_local"], cfg.topk, npairs, b["xp"], b["xps"], d)
+                native.call("tf_moe_gemv_split", L.ew1, L.ew3, L.es1, L.es3, self.El, b["xp"], b["xps"], npairs, None, 0,
+                            b["ap"], b["aps"], I, d, *groups, cfg.swiglu_limit, self.status.t)
+                native.call("tf_moe_gemv_split", L.ew2, None, L.es2, None, self.El, b["ap"], b["aps"], npairs, b["y_pair"], d,
                             None, None, d, I, *groups, 0.0, self.status.t)
             else:
                 self._moe_small_f16(L, T, b, slots)
