@@ -114,7 +114,7 @@ def test_block_scaled_expert_path_matches_register_path_and_oracle():
     assert eng._moe_mx_ok(4) and "x8" in eng._bufs(4)
     old = E.Engine.from_weights(cfg, EngineConfig(reference_matmul=True, regions=2, max_context=512, prefill_widths=(128,),
                                                   moe_block_scaled=False), W)
-    assert "x8" not in old._bufs(4)
+    assert "x8" not in old._bufs(4) and "xp" not in old._bufs(4)             # the register-fed form
     ref = oracle.OracleModel(cfg, rt)
     g = torch.Generator().manual_seed(1)
     prompt = torch.randint(0, cfg.vocab, (77,), generator=g)
@@ -152,7 +152,7 @@ def test_block_scaled_expert_path_matches_register_path_and_oracle():
     new24 = E.Engine.from_weights(cfg24, ecfg, W24)
     old24 = E.Engine.from_weights(cfg24, EngineConfig(reference_matmul=True, regions=2, max_context=512,
                                                       prefill_widths=(128,), moe_block_scaled=False), W24)
-    assert "x8" in new24._bufs(24) and "x8" not in old24._bufs(24)
+    assert "x8" in new24._bufs(24) and "x8" not in old24._bufs(24) and "xp" not in old24._bufs(24)
     toks = torch.randint(0, cfg.vocab, (24,), generator=g).tolist()
     outs = []
     for e in (new24, old24):
@@ -161,6 +161,23 @@ def test_block_scaled_expert_path_matches_register_path_and_oracle():
         e.status.check()
     d24 = _row_err(outs[0], outs[1])
     assert d24.max() < 0.12 and d24.median() < 0.06, d24
+
+
+def test_f16_experts_in_pieces_follow_the_switch_and_match_the_register_form():
+    """Widths off the MXFP8 form (256 inputs): f16 activations in pieces where block-scaled MMAs are wanted, the register-fed
+    kernel where they are not.  Both multiply the same f16 numbers: the logits differ by the order of fp32 sums and the f16
+    rounding between the two GEMVs (2^-11 of a SwiGLU product), far below the 0.1 of the quantised oracle."""
+    cfg = small_config(topk=8)                               # every expert: nothing discrete flips
+    W = oracle.init_weights(cfg, 0)
+    outs = []
+    for on in (True, False):
+        eng = E.Engine.from_weights(cfg, EngineConfig(reference_matmul=True, regions=2, max_context=512, prefill_widths=(128,),
+                                                      moe_block_scaled=on), W)
+        assert "x8" not in eng._bufs(2) and ("xp" in eng._bufs(2)) == on
+        eng.forward(E.StepPlan.build([(0, 0, list(range(7, 47)))], logits="last"))
+        outs.append(eng.forward(E.StepPlan.build([(0, 40, [5, 6])])).cpu())
+        eng.status.check()
+    assert _row_err(outs[0], outs[1]).max() < 0.01, _row_err(outs[0], outs[1])
 
 
 def test_index_scoring_in_row_tiles_is_bitwise_the_same():

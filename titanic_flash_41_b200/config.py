@@ -346,7 +346,7 @@ class EngineConfig(_JsonMixin):
     sp_chunk_rows: int = 0                 # rows of one sequence-parallel prefill chunk over ALL ranks (0: the single-rank chunk); the window ring holds a whole chunk
     index_score_bytes: int = 2 << 30       # most bytes of one fp32 index-score matrix: prefill rows are scored and selected in row tiles beyond it (long contexts)
     prefill_mx: bool = True                # prefill GEMMs on the block-scaled tensor-core form (MXFP8 activations)
-    moe_block_scaled: bool = True     # decode rows <= 16: routed experts on block-scaled tcgen05 MMAs (MXFP8 activations)
+    moe_block_scaled: bool = True     # decode rows <= 32: routed experts on block-scaled tcgen05 MMAs (MXFP8 activations; f16 ones in MXFP8 pieces where a width is not a multiple of 512); off: the register-fed f16 kernel
     seed: int = 0
 
 

@@ -1188,12 +1188,14 @@ class Engine:
                 and cfg.hidden % 512 == 0 and cfg.moe_inter % 512 == 0)
 
     def _moe_split_ok(self, T: int) -> bool:
-        """Split form of the f16 activations (``csrc/moe_split.cu``): MXFP4 experts, widths in whole 256-input pieces."""
+        """Split form of the f16 activations (``csrc/moe_split.cu``): MXFP4 experts, widths in whole 256-input pieces; like the
+        MXFP8 form only where block-scaled MMAs are wanted at all."""
         cfg = self.cfg
-        return T <= self.SMALL_M and cfg.expert_quant == "mxfp4" and cfg.hidden % 256 == 0 and cfg.moe_inter % 256 == 0
+        return (self.ecfg.moe_block_scaled and T <= self.SMALL_M and cfg.expert_quant == "mxfp4"
+                and cfg.hidden % 256 == 0 and cfg.moe_inter % 256 == 0)
 
     def _moe_small_f16(self, L: LayerWeights, T: int, b: dict, slots: int) -> None:
-        """Register-fed form (f16 activations, nibbles unpacked on the CUDA cores): widths the
+        """Register-fed form (f16 activations, nibbles unpacked on the CUDA cores): ``moe_block_scaled`` off, and widths the
         tensor-core forms do not tile."""
         cfg = self.cfg
         d, I = cfg.hidden, cfg.moe_inter
