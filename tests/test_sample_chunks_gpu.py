@@ -234,3 +234,57 @@ def test_row_statistics_of_crowded_and_spread_rows(V):
         native.call("tf_rowstats_per_session", lg, V, V, S, temp, topp, 1, want, scratch, st.t)
         st.check()
         assert torch.equal(got, want), (p, [i for i in range(S) if not torch.equal(got[i], want[i])])
+
+def _scan(x):
+    """Inclusive prefix sums of 32 numbers by doubling steps, the order of the device's."""
+    x = list(x)
+    for o in (1, 2, 4, 8, 16):
+        x = [v + (x[i - o] if i >= o else 0.0) for i, v in enumerate(x)]
+    return x
+
+
+def _boundary(level):
+    """Tokens of equal weight in the first chunk (one to nine a lane) and a draw u such that u * total is exactly the mass in
+    front of a warp (level 0) or lane (1), and less than the sum up to that one's end with its own mass taken away again."""
+    import numpy as np
+    rng = np.random.default_rng(level)
+    for _ in range(20000):
+        count = np.zeros((32, 32), dtype=int)
+        count[:6] = rng.integers(1, 10, (6, 32))
+        w = 1.0 / int(count.sum())
+        lane = np.array([[sum([w] * c) for c in row] for row in count])
+        wm = []
+        for row in lane:
+            x = list(row)
+            for o in (16, 8, 4, 2, 1):
+                x = [x[i] + x[i ^ o] for i in range(32)]
+            wm.append(x[0])
+        t = list(wm)
+        for o in (16, 8, 4, 2, 1):
+            t = [t[i] + t[i ^ o] for i in range(32)]
+        own = wm if level == 0 else lane[0]
+        upto = _scan(own)
+        for i in range(1, 6):
+            draw = upto[i - 1]
+            if not upto[i] - own[i] > draw:
+                continue
+            u = draw / t[0]
+            for v in (u, np.nextafter(u, 0.0), np.nextafter(u, 1.0)):
+                if v * t[0] == draw:
+                    return count, float(v), (i, 0) if level == 0 else (0, i)
+    raise AssertionError("no such draw found")
+
+
+@pytest.mark.parametrize("level", [0, 1])
+def test_a_draw_on_the_edge_of_a_warp_or_lane_takes_what_follows_the_edge(level):
+    count, u, (warp, lane) = _boundary(level)
+    V = 129280
+    lg = torch.full((1, 1, V), -float("inf"), device=DEV)
+    for w in range(32):
+        for l in range(32):
+            for j in range(int(count[w, l])):
+                lg[0, 0, w * 32 + l + 1024 * j] = 0.0
+    one = torch.ones(1, device=DEV)
+    f = Flow(V, 1, 0, 1)
+    tok = int(f.run(lg, None, None, torch.tensor([[u, u]], dtype=torch.float64, device=DEV), one, one)[4])
+    assert (tok % 1024 // 32, tok % 32) == (warp, lane)

@@ -523,36 +523,35 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
       }
       return x;
     };
-    if (warp == 0) {
-      const double mass_w = wm[lane], upto = prefix(mass_w), draw = s_draw;
-      const unsigned int over = __ballot_sync(0xffffffffu, upto > draw), some = __ballot_sync(0xffffffffu, mass_w > 0.0);
-      int w = over ? __ffs(over) - 1 : 31;
-      // rounding can leave the draw past the last positive warp: step back to one that has mass
+    // Among 32 masses the one whose end is the first past the draw; where rounding leaves the draw past all of them, or on one
+    // without mass, the last before it that has mass.  A mass begins where the one before it ends: its own sum taken away from its
+    // end again is off by an ulp, and a draw between the two would belong to neither.
+    auto pick = [&](double mass, double draw, double* begin) {
+      const double upto = prefix(mass), end_before = __shfl_up_sync(0xffffffffu, upto, 1);
+      *begin = lane ? end_before : 0.0;
+      const unsigned int over = __ballot_sync(0xffffffffu, upto > draw), some = __ballot_sync(0xffffffffu, mass > 0.0);
+      const int w = over ? __ffs(over) - 1 : 31;
       const unsigned int up_to_w = some & (0xffffffffu >> (31 - w));
-      w = up_to_w ? 31 - __clz(up_to_w) : 0;
-      const double before = __shfl_sync(0xffffffffu, upto - mass_w, w);
-      if (lane == 0) {
+      return up_to_w ? 31 - __clz(up_to_w) : some ? __ffs(some) - 1 : 0;
+    };
+    if (warp == 0) {
+      double begin;
+      const double draw = s_draw;
+      const int w = pick(wm[lane], draw, &begin);
+      if (lane == w) {
         s_warp = w;
-        s_draw = draw - before;
+        s_draw = draw - begin;
       }
     }
     __syncthreads();
     if (warp == s_warp) {
-      // inclusive scan of the lane masses in lane order
-      const double incl = prefix(my_mass);
-      const double excl = incl - my_mass, draw = s_draw;
-      const bool hit = my_mass > 0.0 && excl <= draw && draw < incl;
-      unsigned int hits = __ballot_sync(0xffffffffu, hit);
-      if (!hits) {
-        // rounding left the draw past the last positive lane: take that lane
-        const unsigned int pos = __ballot_sync(0xffffffffu, my_mass > 0.0);
-        hits = pos ? (1u << (31 - __clz(pos))) : 1u;
-      }
-      const int winner = __ffs(hits) - 1;
+      double begin;
+      const double draw = s_draw;
+      const int winner = pick(my_mass, draw, &begin);
       // the winner's elements (at most sixteen), one a lane, in its order
       const int k_own = (warp * 32 + winner) + lane * kThreads;
       const double val = k_own < n ? residual(k_own) : 0.0;
-      const double rest = __shfl_sync(0xffffffffu, draw - excl, winner);
+      const double rest = __shfl_sync(0xffffffffu, draw - begin, winner);
       const unsigned int past = __ballot_sync(0xffffffffu, prefix(val) > rest && val > 0.0), with = __ballot_sync(0xffffffffu, val > 0.0);
       const int el = past ? __ffs(past) - 1 : 31 - __clz(with);            // (none past the draw: the last that has mass)
       if (lane == winner) {
