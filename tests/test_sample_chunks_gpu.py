@@ -252,7 +252,7 @@ def _boundary(level):
         count = np.zeros((32, 32), dtype=int)
         count[:6] = rng.integers(1, 10, (6, 32))
         w = 1.0 / int(count.sum())
-        lane = np.array([[sum([w] * c) for c in row] for row in count])
+        lane = np.cumsum(np.concatenate([[0.0], np.full(9, w)]))[count]          # one addition after another (sum() compensates)
         wm = []
         for row in lane:
             x = list(row)
