@@ -288,19 +288,3 @@ def test_a_draw_on_the_edge_of_a_warp_or_lane_takes_what_follows_the_edge(level)
     f = Flow(V, 1, 0, 1)
     tok = int(f.run(lg, None, None, torch.tensor([[u, u]], dtype=torch.float64, device=DEV), one, one)[4])
     assert (tok % 1024 // 32, tok % 32) == (warp, lane)
-
-def test_infinite_temperature_draws_from_the_uniform_law():
-    """Every token weighs the same, the places behind a chunk's last token weigh nothing: statistics as the full-row kernel has them."""
-    V, rows = 129280, 2
-    lg = (torch.randn(rows, V, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)) * 3).contiguous()
-    st, sb = native.StatusWord(DEV), native.lib().tf_rowstat_bytes()
-    for top_p in (0.4, 1.0):
-        want = torch.zeros(rows, sb, dtype=torch.uint8, device=DEV)
-        scr = torch.zeros(native.lib().tf_rowstats_scratch_bytes(rows), dtype=torch.uint8, device=DEV)
-        native.call("tf_rowstats", lg, V, V, rows, float("inf"), top_p, want, scr, st.t)
-        u = torch.tensor([[0.25, 0.25], [0.75, 0.75]], dtype=torch.float64, device=DEV)
-        _, _, got, _, tok = Flow(V, rows, 0, 1).run(lg.view(rows, 1, V), None, None, u, torch.full((rows,), float("inf"), device=DEV),
-                                                   torch.full((rows,), top_p, device=DEV))
-        assert torch.equal(got, want)
-        if top_p == 1.0:                                       # chunk 2 of 8 and chunk 6
-            assert [t // (V // 8) for t in tok.tolist()] == [2, 6]

@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
       for (int k = threadIdx.x; k < padded; k += kThreads) {
         const float v = tbuf[k];
         const int bin = (int)(fkey(v) >> 24), cls = class_of(bin);
-        const float e = k < n ? expf((v - stat.m) * inv_t) : 0.f;         // (at an infinite temperature -inf * 0 is NaN)
+        const float e = expf((v - stat.m) * inv_t);
         const unsigned long long mass = (unsigned long long)((double)e * kFix);
         if (!has_d) dbuf[k] = e;                         // (step 4 reads the weights back where no draft row is staged)
         if (cls >= (pos && bin < 128 ? 4 : 0) && cls < 8) priv[cls * 32] += mass;
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) sample_chunks_kernel(const ChunkP
       for (int k = threadIdx.x; k < padded; k += kThreads) {
         const float v = tbuf[k];
         const uint32_t key = fkey(v);
-        if ((key & mask) != prefix || k >= n) continue;
+        if ((key & mask) != prefix) continue;
         const int bin = (key >> shift) & 255;
         if (bin != cur) {
           if (cur >= 0) atomicAdd(&copy[cur], run);
