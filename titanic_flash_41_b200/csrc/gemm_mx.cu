@@ -36,8 +36,8 @@
 //   warp 0       TMA producer of the operands (its 128 features, its half of the tile's rows); warp 14 of the scales.
 //                One thread that issued all of a k block's copies took 720 - 770 cycles for it, more than the MMAs.
 //   warp 1       owns the tensor memory; in the first CTA of the pair one thread issues the MMAs of both
-//   warps 2-5    scale movers: shared memory -> tensor memory, one per 32-lane quadrant.  Their arrival at the
-//                first CTA's barrier also says that this CTA's operands have landed.
+//   warps 2-5    scale movers: shared memory -> tensor memory, one per 32-lane quadrant; they arrive at the first CTA's
+//                barrier.  The operand tiles of both CTAs complete on the first CTA's barrier by themselves.
 //   warps 6-13   epilogue: tensor memory -> registers -> bf16 / f32; a lane is a feature, a register a row, so a
 //                warp stores 64 (128) contiguous bytes of one row
 // Stages and accumulators follow the tile: as many stages as 227 KB hold (6 at 256 rows, 9 at 32), two accumulators
@@ -49,7 +49,7 @@
 // copies in flight land, frees its tensor memory and returns.
 //
 // The same kernel without scales (MX = 0) multiplies bf16 x bf16 (64 k a block, the vision tower and the router logits of
-// gemm_tc.cu): warp 2 only passes on that its CTA's operands have landed, and two accumulators always fit.
+// gemm_tc.cu): no scale movers, and two accumulators always fit.
 // 8192^3: 1.59 PFLOP/s (1.35 by the one-SM form of gemm_tc.cu).
 //
 // Reference behaviour: block-scaled dense and expert GEMMs of the prefill path
@@ -128,14 +128,49 @@ __device__ __forceinline__ uint32_t pair_rank() {
 __device__ __forceinline__ void pair_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrival at the barrier at the same offset of the pair's first CTA.  What it announces is tensor memory (ordered by the
-// tcgen05 fences around it) and tiles that TMA has written (complete before the warp got here); no plain store has to be
-// visible across the CTAs, so it has the default scope: with .release.cluster here and .acquire.cluster at the wait every
-// k block paid two memory barriers, about 2,000 cycles.
-__device__ __forceinline__ void arrive_first(uint32_t bar) {
+// address of the barrier at the same offset of the pair's first CTA
+__device__ __forceinline__ uint32_t of_first(uint32_t bar) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(bar));
+  return r;
+}
+// A tile of this CTA whose bytes complete on a barrier of the pair's first CTA: the operands of both CTAs announce themselves to
+// the thread that issues the MMAs of both, with no thread of the second CTA in between.
+__device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t first_bar) {
   asm volatile(
-      "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar)
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(first_bar)
       : "memory");
+}
+// Arrival at a barrier of the pair's first CTA, and the wait for it.  All that they order is tensor memory (scale columns
+// written, accumulators read), between the tcgen05 fences on both sides: relaxed, at cluster scope.  With .release.cluster and
+// .acquire.cluster every k block paid two memory barriers, about 2,000 cycles.
+__device__ __forceinline__ void arrive_first(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(of_first(bar)) : "memory");
+}
+__device__ __forceinline__ bool pair_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// bounded like tc::mbar_wait
+__device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (pair_try(bar, parity)) return true;
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (pair_try(bar, parity)) return true;
+    if (*abort_flag) return false;
+    if (clock64() - t0 > 2000000000LL) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
 }
 // one arrival at this barrier of BOTH CTAs when every MMA issued so far by this thread has completed
 __device__ __forceinline__ void commit_pair(uint32_t bar) {
@@ -187,14 +222,17 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   const int stages = p.stages, stage_bytes = p.stage_bytes;
   const uint32_t sfs0 = base + stages * stage_bytes;       // ring of row-major scales
   const uint32_t bar0 = sfs0 + (p.sf_kind ? kSfSlots * kSfSlotBytes : 0);
-  auto full = [&](int s) { return bar0 + 8u * s; };
+  auto full = [&](int s) { return bar0 + 8u * s; };                             // of the first CTA: operands of both
   auto empty = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
-  auto sf_full = [&](int s) { return bar0 + 8u * (2 * kMaxStages + s); };        // of the first CTA
-  auto tfull = [&](int b) { return bar0 + 8u * (3 * kMaxStages + b); };
-  auto tempty = [&](int b) { return bar0 + 8u * (3 * kMaxStages + 2 + b); };     // of the first CTA
-  auto sfs_full = [&](int b) { return bar0 + 8u * (3 * kMaxStages + 4 + b); };
-  auto sfs_empty = [&](int b) { return bar0 + 8u * (3 * kMaxStages + 4 + kSfSlots + b); };
-  uint8_t* tail = aligned + (bar0 - base) + 8 * (3 * kMaxStages + 4 + 2 * kSfSlots);
+  auto sc_full = [&](int s) { return bar0 + 8u * (2 * kMaxStages + s); };        // this CTA's scales in shared memory
+  auto sf_full = [&](int s) { return bar0 + 8u * (3 * kMaxStages + s); };        // of the first CTA: those of both in tensor memory
+  auto tfull = [&](int b) { return bar0 + 8u * (4 * kMaxStages + b); };
+  auto tempty = [&](int b) { return bar0 + 8u * (4 * kMaxStages + 2 + b); };     // of the first CTA
+  auto sfs_full = [&](int b) { return bar0 + 8u * (4 * kMaxStages + 4 + b); };
+  auto sfs_empty = [&](int b) { return bar0 + 8u * (4 * kMaxStages + 4 + kSfSlots + b); };
+  constexpr int kBars = 4 * kMaxStages + 4 + 2 * kSfSlots;
+  static_assert(8 * kBars + 8 <= kTailBytes, "");
+  uint8_t* tail = aligned + (bar0 - base) + 8 * kBars;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 4);
 
@@ -205,9 +243,10 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
-      tc::mbar_init(full(s), MX ? 2 : 1);
+      tc::mbar_init(full(s), 1);
       tc::mbar_init(empty(s), 1);
-      tc::mbar_init(sf_full(s), MX ? 8 : 2);
+      tc::mbar_init(sc_full(s), 1);
+      tc::mbar_init(sf_full(s), 8);
     }
     for (int b = 0; b < 2; ++b) {
       tc::mbar_init(tfull(b), 1);
@@ -270,6 +309,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       tc::prefetch_tmap(&mapX);
       tc::prefetch_tmap(&mapW);
       const int wbytes = p.b_fp4 ? 128 * 64 : 128 * 128, box_bytes = p.box_rows * 128;
+      const uint32_t first_full = of_first(full(0));
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -277,14 +317,16 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
         const MxTile t = tile_of(item);
         const CUtensorMap* mw = t.mat ? &mapW2 : &mapW;
         const int half = t.n >> 1, xrow = t.row0 + rank * half, loads = (half + p.box_rows - 1) / p.box_rows;
-        const uint32_t tx = wbytes + loads * box_bytes;
+        const uint32_t tx = 2 * (wbytes + loads * box_bytes);             // both CTAs' (parts of a box out of range count too)
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!(ok = tc::mbar_wait(empty(s), ph ^ 1, abort_flag))) break;
-          tc::mbar_expect_tx(full(s), tx);
-          const uint32_t sa = base + s * stage_bytes, sx = sa + 128 * 128;
-          tc::tma_load_2d(sa, mw, kb * BKE, t.wrow, full(s));
-          tc::tma_load_2d(sx, &mapX, kb * BKE, xrow, full(s));
-          for (int i = 1; i < loads; ++i) tc::tma_load_2d(sx + i * box_bytes, &mapX, kb * BKE, xrow + i * p.box_rows, full(s));
+          // (the second CTA's bytes may come before the first has set its count: the phase cannot end before that arrival,
+          // nor can it be an older one, whose MMAs have freed this stage)
+          if (rank == 0) tc::mbar_expect_tx(full(s), tx);
+          const uint32_t sa = base + s * stage_bytes, sx = sa + 128 * 128, bar = first_full + 8u * s;
+          tma_load_pair(sa, mw, kb * BKE, t.wrow, bar);
+          tma_load_pair(sx, &mapX, kb * BKE, xrow, bar);
+          for (int i = 1; i < loads; ++i) tma_load_pair(sx + i * box_bytes, &mapX, kb * BKE, xrow + i * p.box_rows, bar);
           if (++s == stages) { s = 0; ph ^= 1; }
         }
       }
@@ -327,9 +369,9 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
           }
           if (!(ok = tc::mbar_wait(empty(s), ph ^ 1, abort_flag))) break;
           const uint32_t sc = base + (s + 1) * stage_bytes - 2048;
-          tc::mbar_expect_tx(full(s), xbytes + (p.sf_kind ? 0 : kSfwBytes));
-          tc::bulk_g2s(sc + kSfwBytes, sfx, xbytes, full(s));
-          if (!p.sf_kind) tc::bulk_g2s(sc, sfw, kSfwBytes, full(s));
+          tc::mbar_expect_tx(sc_full(s), xbytes + (p.sf_kind ? 0 : kSfwBytes));
+          tc::bulk_g2s(sc + kSfwBytes, sfx, xbytes, sc_full(s));
+          if (!p.sf_kind) tc::bulk_g2s(sc, sfw, kSfwBytes, sc_full(s));
           sfx += (long)p.sfa_units * 128;
           sfw += (long)p.sfb_units * 128;
           if (++s == stages) { s = 0; ph ^= 1; }
@@ -349,10 +391,9 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       for (int item = first; item < items && ok; item += step) {
         const uint32_t n = (uint32_t)tile_of(item).n, id = MX ? idesc_mx(p.b_fp4 ? 5u : 0u, n) : tc::instr_desc(1, 1, BF, n);
         const uint32_t td = tmem_base + ab * p.tile_n;
-        if (!(ok = tc::mbar_wait(tempty(ab), aph ^ 1, abort_flag))) break;
+        if (!(ok = pair_wait(tempty(ab), aph ^ 1, abort_flag))) break;
         for (int kb = 0; kb < kblocks; ++kb) {
-          // all eight movers: operands and scales of both CTAs are in place
-          if (!(ok = tc::mbar_wait(sf_full(s), ph, abort_flag))) break;
+          if (MX && !(ok = pair_wait(sf_full(s), ph, abort_flag))) break;
           if (!(ok = tc::mbar_wait(full(s), ph, abort_flag))) break;
           tc::tc_fence_after();
           const uint32_t sa = base + s * stage_bytes;
@@ -371,21 +412,10 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       }
     }
   } else if (!MX && warp < 6) {
-    // ------------------------------------------------------------------ this CTA's operands have landed: passed on
-    if (warp == 2 && tc::elect_one()) {
-      int s = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int item = first; item < items && ok; item += step)
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (!(ok = tc::mbar_wait(full(s), ph, abort_flag))) break;
-          arrive_first(sf_full(s));
-          if (++s == stages) { s = 0; ph ^= 1; }
-        }
-    }
+    // ------------------------------------------------------------------ (no scales to move)
   } else if (warp < 6) {
     // ------------------------------------------------------------------ scale movers
-    // When full(s) completes for lap r of the ring, the MMAs that read scale columns s in lap r - 1 are
+    // When sc_full(s) completes for lap r of the ring, the MMAs that read scale columns s in lap r - 1 are
     // done (the producer refilled the stage only after their commit): the columns are free.
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     int s = 0, b = 0;
@@ -412,7 +442,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
           if (lane == 0) tc::mbar_arrive(sfs_empty(b));
           if (++b == kSfSlots) { b = 0; bph ^= 1; }
         }
-        if (!(ok = tc::mbar_wait(full(s), ph, abort_flag))) break;
+        if (!(ok = tc::mbar_wait(sc_full(s), ph, abort_flag))) break;
         const uint8_t* sf = aligned + s * stage_bytes + stage_bytes - 2048;
         uint32_t vw[4], vx[8];
         if (p.sf_kind) {
@@ -504,6 +534,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   tc::tc_fence_before();
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) tf_report(p.status, TF_TIMEOUT, MX ? 140 : 141, blockIdx.x, p.b_fp4);
+  __syncwarp();
   pair_sync();                                 // nobody leaves while the other CTA may still arrive at its barriers
   if (warp == 1) {
     tc::tc_fence_after();
