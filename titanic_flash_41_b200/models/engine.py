@@ -1189,10 +1189,18 @@ class Engine:
 
     def _moe_split_ok(self, T: int) -> bool:
         """Split form of the f16 activations (``csrc/moe_split.cu``): MXFP4 experts, widths in whole 256-input pieces; like the
-        MXFP8 form only where block-scaled MMAs are wanted at all."""
+        MXFP8 form only where block-scaled MMAs are wanted at all.
+
+        Against the register-fed form (us of both GEMVs, 5,120 x 2,304, 48 experts): one or two rows an expert 171 - 175 and 327, three
+        or four 273 and 330, five 374 and 331, eight 478 and 335: every two rows walk the weights again, so two rows an
+        expert on average is the line.  It starts later, with one launch more: 23.6 and 15.4 us for eight experts of 512 x 512; both
+        meet at about 40 MB of experts' weights (16 experts of 2,048 x 768: 31.7 and 31.8; two of 5,120 x 2,304: 38 and 40)."""
         cfg = self.cfg
+        pairs = T * cfg.topk
+        weights = 1.5 * cfg.hidden * cfg.moe_inter * min(self.El, pairs / self.world)       # bytes of the experts met, at most
         return (self.ecfg.moe_block_scaled and T <= self.SMALL_M and cfg.expert_quant == "mxfp4"
-                and cfg.hidden % 256 == 0 and cfg.moe_inter % 256 == 0)
+                and cfg.hidden % 256 == 0 and cfg.moe_inter % 256 == 0
+                and pairs <= 2 * cfg.n_experts and weights >= 40e6)
 
     def _moe_small_f16(self, L: LayerWeights, T: int, b: dict, slots: int) -> None:
         """Register-fed form (f16 activations, nibbles unpacked on the CUDA cores): ``moe_block_scaled`` off, and widths the
