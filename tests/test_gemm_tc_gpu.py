@@ -112,9 +112,10 @@ def _rs_case(M, N, K):
         assert _rel(out, a.float() @ b.float().t()) < 5e-3
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 128, 1088), (33, 384, 2048), (257, 128, 1088), (1300, 1152, 1152), (2049, 256, 1088)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 1088), (33, 384, 2048), (257, 128, 1088), (1300, 1152, 1152), (2049, 256, 1088),
+                                   (1, 128, 2112), (33, 384, 3072), (257, 128, 2112), (1300, 1152, 2112), (2049, 256, 2112), (2600, 1152, 128)])
 def test_bf16_by_pairs_of_sms(M, N, K):
-    """Rows and feature blocks that end inside a pair's tile (one CTA's 128 features or fewer rows than a tile), both output
+    """Both sides of the line between the one-SM and the pair form (K 2,048 at no more tiles than SMs; 189 tiles).  Rows and feature blocks that end inside a pair's tile (one CTA's 128 features or fewer rows than a tile), both output
     types, rows beyond M and columns beyond N untouched: exact products, fp32 sums (2e-5; bf16 rounding 4e-3)."""
     gen = torch.Generator(device="cuda").manual_seed(M + N)
     a, b = (torch.randn(r, K, device="cuda", generator=gen).bfloat16() for r in (M, N))

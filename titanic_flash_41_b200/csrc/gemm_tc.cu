@@ -537,10 +537,12 @@ TF_API int tf_gemm_tc(int kind, const void* A, long lda, const void* B, long ldb
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   // bf16 matrices by pairs of SMs: 8192^3 812 -> 691 us (1.59 PFLOP/s), 8580 x 8192 x 1024 137 -> 99, 16384 x 256 x 4096 64 -> 44.
-  // A short K over no more 128 x 128 tiles than SMs stays here: setting a pair up costs more than it saves
-  // (1521 x 1024 x 1024 13.2 us here, 15.2 by pairs; x 640 12.3 and 14.3; at K 4096 both 24.6), and so do the forms that the
-  // pair kernel does not have (experts, reduce-scatter, all-gather).
-  const bool small = K <= 1024 && (long)((M + BM - 1) / BM) * (N / 128) <= g_sms;
+  // A short K over no more 128 x 128 tiles than SMs stays here: setting a pair up costs more than it saves.  One-SM and pair
+  // form, us back to back: 1521 x 1024 x 512 8.4 and 10.4, x 1024 10.4 and 12.0, x 1536 12.4 and 12.4, x 2048 14.5 and 14.5, x 3072
+  // 16.7 and 16.5, x 4096 20.6 and 19.2; 400 x 4096 x 1024 10.5 and 12.4, x 2048 14.5 and 14.5, x 3072 18.6 and 17.0; 33 x 128 x
+  // 1024 8.3 and 10.4, x 2048 10.4 and 12.4, x 4096 16.4 and 16.5.  So do the forms that the pair kernel does not have (experts, reduce-scatter,
+  // all-gather).
+  const bool small = K <= 2048 && (long)((M + BM - 1) / BM) * (N / 128) <= g_sms;
   if (kind == 0 && experts <= 0 && !g_rs.peers && !g_ag.peers && g_force_bn == 0 && !small)
     return tf_gemm_pair_bf16(A, lda, B, ldb, C, ldc, out_kind, M, N, K, status, stream);
   CUtensorMap ma, mb;
