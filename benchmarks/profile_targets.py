@@ -5,6 +5,9 @@ under a GB on the device).  Each target prints the CUDA-event time of its launch
     python benchmarks/profile_targets.py sampler       # chunked sampler: verification of 4 x (3 + 1) rows, vocabulary 129,280
     python benchmarks/profile_targets.py attention     # sparse attention: 2,048 prefill rows, 64 heads x 128, 128 window + 2,048 selected keys
     python benchmarks/profile_targets.py index         # index scores + exact top-2048 of 2,048 prefill rows over 32,768 keys, 8 heads x 128
+    python benchmarks/profile_targets.py gemm          # pair GEMM: 64 MXFP4 experts of 5 rows, 2 x 2,048 x 4,096, and 4,001 x 9,984 x 4,096 dense
+    python benchmarks/profile_targets.py split         # f16 decode experts in pieces: 4 rows x 6 experts of 5,120 x 2,304
+    python benchmarks/profile_targets.py copies        # residual copies of a prefill: 4,001 rows of 4 x 5,120
     python benchmarks/profile_targets.py prep          # attention prep of 2,048 prefill rows (RoPE, FP8 window rows, pooling, FP4 entries, index keys)
 """
 import math
@@ -129,6 +132,55 @@ def index():
     print(f"top-{k} select of {T} rows x {C} scores: {us:.0f} us per launch")
 
 
+def gemm():
+    from titanic_flash_41_b200.ops import mx
+    st, i32 = native.StatusWord(DEV), lambda n: torch.zeros(n, dtype=torch.int32, device=DEV)
+    u8 = lambda *s: torch.randint(0, 100, s, dtype=torch.uint8, device=DEV)
+    scales = lambda *s: torch.full(s, 120, dtype=torch.uint8, device=DEV)
+    El, rows, N, K = 64, 5, 2048, 4096
+    n, tile_max = El * rows, mx.expert_tile_rows(El * rows, El)
+    cap, room = -(-(n + El * 31) // 32) * 32, n // tile_max + El
+    te, r0, tr, nt, dst = i32(room), i32(room), i32(room), i32(1), i32(n)
+    native.call("tf_moe_plan_tiles", torch.arange(El, device=DEV).repeat_interleave(rows).int(), n, 0, El, i32(El), i32(El + 1), i32(El), te, r0, tr,
+                tile_max, room, nt, i32(1), dst)
+    a, sa, w, s = u8(cap, K), scales(K // 128, cap // 32, 128), [u8(El, N, K // 2) for _ in range(2)], [scales(El, N, K // 32) for _ in range(2)]
+    c = torch.zeros(cap, 2 * N, device=DEV, dtype=torch.bfloat16)
+    us = timed(lambda: mx.gemm_experts(a, sa, w[0], w[1], s[0], s[1], El * N, c, cap, N, K, (te, r0, tr, nt, tile_max, room), st.t))
+    print(f"{El} experts x {rows} rows, two of {N} x {K}: {us:.1f} us, {2 * El * N * K * (0.5 + 1 / 32) / us / 1e6:.2f} TB/s of weights")
+    M, N = 4001, 9984
+    a, sa, b, sb = u8(M, K), scales(K // 128, 128, 128), u8(N, K), scales(K // 128, 320, 128)
+    c = torch.zeros(M, N, device=DEV, dtype=torch.bfloat16)
+    us = timed(lambda: mx.gemm(a, sa, b, sb, c, M, N, K, st.t))
+    st.check()
+    print(f"dense {M} x {N} x {K}: {us:.1f} us, {2 * M * N * K / us / 1e6:.0f} TFLOP/s")
+
+
+def split():
+    K, I, El, T, topk = 5120, 2304, 24, 4, 6
+    pairs, lib, st = T * topk, native.lib(), native.StatusWord(DEV)
+    i32, u8 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV), lambda *s: torch.randint(118, 122, s, dtype=torch.uint8, device=DEV)
+    w1, w3, w2, s1, s3, s2 = (u8(El, *s) for s in ((I, K // 2), (I, K // 2), (K, I // 2), (I, K // 32), (I, K // 32), (K, I // 32)))
+    x, sp, y = torch.randn(T, K, device=DEV).half(), torch.arange(pairs, dtype=torch.int32, device=DEV), torch.zeros(pairs, K, device=DEV)
+    rows = lib.tf_moe_split_pieces() * pairs
+    xp, xs, ap, aps = u8(rows, K), u8(rows, lib.tf_moe_split_pitch(K)), u8(rows, I), u8(rows, lib.tf_moe_split_pitch(I))
+    groups, nl = (i32(list(range(El))), i32(list(range(El))), i32([1] * El), i32([El]), sp, El), i32([pairs])
+    parts = [timed(f) for f in (
+        lambda: native.call("tf_moe_split_rows", x, K, sp, nl, topk, pairs, xp, xs, K),
+        lambda: native.call("tf_moe_gemv_split", w1, w3, s1, s3, El, xp, xs, pairs, None, 0, ap, aps, I, K, *groups, 10.0, st.t),
+        lambda: native.call("tf_moe_gemv_split", w2, None, s2, None, El, ap, aps, pairs, y, K, None, None, K, I, *groups, 0.0, st.t))]
+    st.check()
+    print(f"f16 experts in pieces, {pairs} of one row, {K} x {I}: split {parts[0]:.1f} us, FC1 {parts[1]:.1f}, FC2 {parts[2]:.1f}")
+
+
+def copies():
+    from titanic_flash_41_b200.ops.mhc import HcBoundary
+    T, H, d = 4001, 4, 5120
+    x = torch.randn(T, H, d, device=DEV).bfloat16()
+    fn, nw = torch.randn(H * (2 + H), H * d, device=DEV) * 0.05, torch.ones(d, device=DEV, dtype=torch.bfloat16)
+    hb = HcBoundary(fn, torch.zeros(H * (2 + H), device=DEV), torch.ones(3, device=DEV), H, d)
+    print(f"residual copies, {T} rows of {H} x {d}: {timed(lambda: hb.prepare(x, nw)):.1f} us")
+
+
 def prep():
     T, Hl, Dh, Di, Hi, ratio, rope = 2048, 64, 128, 128, 8, 4, 64
     ring, maxC = 16384 + 256, 32768 + 8
@@ -166,7 +218,8 @@ def prep():
 
 
 if __name__ == "__main__":
-    targets = {"allreduce": allreduce, "sampler": sampler, "attention": attention, "index": index, "prep": prep}
+    targets = {"allreduce": allreduce, "sampler": sampler, "attention": attention, "index": index, "prep": prep,
+               "gemm": gemm, "split": split, "copies": copies}
     if len(sys.argv) != 2 or sys.argv[1] not in targets:
         sys.exit("usage: python benchmarks/profile_targets.py {" + " | ".join(sorted(targets)) + "}")
     targets[sys.argv[1]]()

@@ -17,25 +17,25 @@
 // and chunk on one unit were 1,024 cycles, as long as the chunk's MMAs).  P holds zeros for the keys of the other copy, so
 // lanes 0..63 of O are the sums over half of the keys, lanes 64.. over the other half; the row's end adds them.
 //
-// One Q, one S (and P over it) and one O, two key tiles, 104 KB of shared memory and 256 tensor-memory columns: two CTAs
+// One Q, one S (and P over it) and one O, two key tiles, 108 KB of shared memory and 256 tensor-memory columns: two CTAs
 // share an SM, and the chains of one row fill the waits of the other.  P as a tensor-memory operand takes a quarter of the
 // MMAs' shared-memory reads away.
 // 2,048 rows of 2,176 keys: 305 us; two softmax warps, one thread per key row, the row's end in the softmax warps: 346 (the MMAs
 // alone: 130).  Inside a long prefill the clock follows the power limit (1.5 - 1.65 of 1.97 GHz) and the gain is smaller: four
-// launches of 16,384 rows 8.4 -> 7.3 ms.  What bounds it now is the issue of 136 M warp instructions (a third of them the gather's
-// conversion) at 40 % of the slots, with scoreboard waits between.
+// launches of 16,384 rows 8.4 -> 7.3 ms.  What bounds it now is the issue of 146 M warp instructions (a third of them the gather's
+// conversion) at half of the slots, with scoreboard waits between; the tensor pipe is active half of the time.
 //
-//   warps 0-3   gather: four threads per key of the chunk fetch its FP8 window row or FP4 compressed row (the next
+//   warps 0-7   gather: four threads per key of the chunk fetch its FP8 window row or FP4 compressed row (the next
 //               chunk's bytes are requested when this one has been converted; ids are decoded a chunk after
 //               they are loaded) and write it as a row of the key tile; two tiles in flight.  Behind the first chunks
 //               of a row they finish the row before: the halves exchange dims through shared memory (each finishes
 //               64 of the 128), sink, inverse rotation of the tail, f16 / bf16 output
-//   warps 4-7   softmax, one (head, half of the keys) per thread, its 64 scores in registers: base-2 online softmax
+//   warps 8-11  softmax, one (head, half of the keys) per thread, its 64 scores in registers: base-2 online softmax
 //               with a stale reference maximum (O is rescaled only when a score exceeds it by 2^8); they also write
 //               the next row's Q while the last PV runs
-//               One thread of warp 4 issues the MMAs: PV of chunk c and, once that is done, QK of chunk c + 1 (it
-//               overwrites S and P).  Eight warps a CTA leave 128 registers a thread; a ninth for the MMAs left 96 and
-//               the gather's prefetched rows in local memory.
+//               One thread of warp 8 issues the MMAs: PV of chunk c and, once that is done, QK of chunk c + 1 (it
+//               overwrites S and P).  The kernel is launched with 80 registers a thread; the gather gives up 16 (64), the
+//               softmax takes 32 (112) for its scores and probabilities.
 // Every mbarrier wait is bounded; on a time-out the CTA raises its abort flag, reports TF_TIMEOUT,
 // frees its tensor memory and returns.
 //

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kItThreads, 1) index_score_tc_kernel(ScorePara
   auto k_full = [&](int s) { return bar0 + 8u * s; };             // key tile written     (4 warps)
   auto k_empty = [&](int s) { return bar0 + 16u + 8u * s; };      // its MMAs are done    (commit)
   auto s_ready = [&](int s) { return bar0 + 32u + 8u * s; };      // accumulator ready    (commit)
-  auto s_free = [&](int s) { return bar0 + 48u + 8u * s; };       // accumulator read     (4 warps)
+  auto s_free = [&](int s) { return bar0 + 48u + 8u * s; };       // accumulator read     (8 warps)
   auto q_ready = [&](int s) { return bar0 + 64u + 8u * s; };      // Q tile written       (4 warps)
   auto q_free = [&](int s) { return bar0 + 80u + 8u * s; };       // the item's MMAs done (commit)
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tail + 96);

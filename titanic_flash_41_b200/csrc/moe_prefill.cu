@@ -2,8 +2,8 @@
 //   * row-wise FP8 quantisation with one fp32 scale per 128 (activations entering an FP8 GEMM)
 //   * clamped SwiGLU (+ optional FP8 quantisation) over a [rows, 2I] GEMM output
 //   * routed-expert bookkeeping without a host round trip: histogram of (token, slot) pairs per
-//     local expert, 128-row-padded segment offsets, per-M-tile expert table, destination row of
-//     every pair
+//     local expert, segment offsets padded to whole 128-row tiles or (block-scaled form) to whole 32
+//     rows, table of the tiles' experts, first rows and rows, destination row of every pair
 //   * gather + quantise token rows into the expert-sorted, padded activation matrix
 //   * MXFP4 (e2m1 + UE8M0/32) expert weights re-expressed as FP8 with one power-of-two scale per
 //     128x128 block, the operand format of the block-scaled tcgen05 GEMM
