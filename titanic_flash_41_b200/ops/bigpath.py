@@ -122,7 +122,6 @@ class BigPath:
         st = eng.status.t
         if eng.ecfg.prefill_mx and d % 256 == 0 and I % 256 == 0:
             # block-scaled form: the packed e2m1 weights and their UE8M0 scales are read as stored
-            self._mx_layer = L
             tile_max = mx.expert_tile_rows(npairs, El * eng.world)
             cap = -(-(npairs + El * 31) // 32) * 32
             max_tiles = npairs // tile_max + El
@@ -140,6 +139,7 @@ class BigPath:
             native.call("tf_swiglu_pairs_mx_units", y1, 2 * I, aq, sfq, cap // 32, pair_dst, npairs, I, cfg.swiglu_limit)
             y2 = self._get("y2", (cap, d), torch.bfloat16)
             mx.gemm_experts(aq, sfq, L.ew2, None, L.es2, None, El * d, y2, cap, d, I, tiles, st)
+            self._mx_layer = L
             self._moe_tail(eng, L, T, b, y2, pair_dst, with_shared, out)
             return
         cap = npairs + El * 127

@@ -3,6 +3,11 @@ scales in the kernel's unit layout, and the calls that fill them.
 
 Unit layout: 128 bytes hold the scales of 32 consecutive rows x 128 inputs, byte
 ``(row % 32) * 4 + (k // 32) % 4``; units are ordered ``[k // 128][row // 32]``.
+
+The engine's experts keep their scales row-major as stored (``gemm_experts``).  The grouped arguments of ``gemm``,
+``units_from_rowmajor`` and the row form of the SwiGLU quantiser (``tf_swiglu_rows_mx_units``) serve callers whose rows
+lie in whole 128-row tiles and whose weight scales are, or are to be, units: ``benchmarks/bench_gemm.py`` and the
+kernel tests, not the engine.
 """
 from __future__ import annotations
 
